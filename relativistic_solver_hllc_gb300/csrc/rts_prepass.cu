@@ -24,18 +24,13 @@
 
 #include "rts_internal.h"
 #include "rts_ptx.cuh"
+#include "rts_rows.cuh"
 
 using namespace rts_ptx;
+using rts_rows::pow2_scale;
+using rts_rows::pow2_scaled_to_f32;
 
 namespace {
-
-// 2^(13 - ilogb(m)), within FP32's normal range (rows or columns whose
-// largest value is below 2^-113 or above 2^139 keep the nearest scale).
-__device__ __forceinline__ float pow2_scale(double m)
-{
-    if (!(m > 0.0) || !isfinite(m)) return 1.0f;
-    return ldexpf(1.0f, max(-126, min(127, 13 - ilogb(m))));
-}
 
 // Block sum of one double per thread (blockDim.x a multiple of 32); every
 // thread receives the total.
@@ -63,7 +58,7 @@ __device__ double block_sum(double x, double* red)
 // time in coalesced 256-byte pieces -- the next piece while the current one
 // is added -- and turns them through shared memory.  One block that walked
 // the rows thread by thread (the former layout: a 32-byte sector per value,
-// one SM) took 1,173 us at M = 1000 against 239 us for the three launches.
+// one SM) took 1,173 us at M = 1000 against 64 us for the three launches.
 constexpr int WS_T = 32;
 
 // Row sums of f(W[j][k], k) over k in order for rows [32 b, 32 b + 32): lane
@@ -163,7 +158,7 @@ __global__ void __launch_bounds__(WS_T) w_stats_u_kernel(const double* __restric
 // (lane = out-direction) for the columns' maxima, then each takes every 8th
 // group of 32 in-directions, whose split parts are 128 contiguous bytes of a
 // lane's own row (256 for TF32).  A thread per out-direction over all
-// in-directions (the former layout) wrote 2 bytes at a time: 455 -> 42 us at
+// in-directions (the former layout) wrote 2 bytes at a time: 455 -> 16 us at
 // M = 1000.
 constexpr int SW_THREADS = 256, SW_WARPS = SW_THREADS / 32;
 __global__ void __launch_bounds__(SW_THREADS)
@@ -254,28 +249,6 @@ __global__ void rowscale_faces_kernel(const double* __restrict__ illum, int64_t 
     rs[npad + c] = 1.0f / s;
 }
 
-// x * 2^k rounded to the nearest FP32 (ties to even), from the bit pattern
-// on the integer pipe: GB300's FP64 pipe issues about two instructions per SM
-// per cycle against 128 for FP32 / integer, and would bound a pass that
-// scaled and converted every value there.  Where x * 2^k is in FP32's normal
-// range the 52-bit mantissa keeps its top 23 bits, rounded on the 29 below
-// (a carry into the exponent is the correctly rounded result, up to
-// infinity); zeros, FP64 subnormals, FP32 subnormal or overflowing results
-// and NaN take ldexp and the hardware conversion.  Either way one rounding
-// of the exact product.
-__device__ __forceinline__ float pow2_scaled_to_f32(double x, int k)
-{
-    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    const int e = (int)((u >> 52) & 0x7FF);
-    const int ef = e + k - 1023 + 127;  // biased FP32 exponent of x * 2^k
-    if (e == 0 || e == 0x7FF || ef < 1 || ef > 254) return __double2float_rn(ldexp(x, k));
-    const unsigned long long m = u & 0xFFFFFFFFFFFFFull;
-    unsigned int f = ((unsigned int)ef << 23) | (unsigned int)(m >> 29);
-    const unsigned int rem = (unsigned int)m & 0x1FFFFFFFu;
-    if (rem > 0x10000000u || (rem == 0x10000000u && (f & 1u))) ++f;
-    return __uint_as_float(f | ((unsigned int)(u >> 32) & 0x80000000u));
-}
-
 // Face sums of the face layout (FP64, the reference's order) into a
 // direction-major staging [M][N], and with cmax non-null the per-cell max
 // over the directions of |face sum| (FP64 bits: non-negative doubles order
@@ -324,19 +297,35 @@ __global__ void rowscale_from_max_kernel(const unsigned long long* __restrict__ 
     rs[npad + c] = 1.0f / s;
 }
 
-// Row scales from direction-major FP32 Ibar [groups][M][N]: thread per row.
-__global__ void rowscale_f32_kernel(const float* __restrict__ ibar, int64_t N, int M, int64_t rows,
-                                    const float* __restrict__ B, float* __restrict__ rs, int64_t rows_pad)
+// Row scales from direction-major FP32 Ibar [groups][M][N].  A block takes 32
+// rows, its 8 warps every 8th direction each (a thread per row left a
+// 15,000-row problem with one warp per SM in flight); the maximum of FP32
+// values is taken in FP32, which is exact and off the FP64 pipe: 260 -> 28 us at
+// 60,000 rows x 590.
+constexpr int RF32_WARPS = 8;
+__global__ void __launch_bounds__(32 * RF32_WARPS)
+rowscale_f32_kernel(const float* __restrict__ ibar, int64_t N, int M, int64_t rows, const float* __restrict__ B,
+                    float* __restrict__ rs, int64_t rows_pad)
 {
-    const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows_pad) return;
-    float s = 1.0f;
+    __shared__ float smax[RF32_WARPS][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t r = (int64_t)blockIdx.x * 32 + lane;  // rows_pad is a multiple of 128
+    float m = 0.0f;
     if (r < rows) {
         const int64_t g = r / N, c = r - g * N;
         const float* base = ibar + g * (int64_t)M * N + c;
-        double m = B ? fabs((double)B[r]) : 0.0;
-        for (int j = 0; j < M; ++j) m = fmax(m, fabs((double)base[(int64_t)j * N]));
-        s = pow2_scale(2.0 * m);
+#pragma unroll 8
+        for (int j = warp; j < M; j += RF32_WARPS) m = fmaxf(m, fabsf(__ldg(base + (int64_t)j * N)));
+    }
+    smax[warp][lane] = m;
+    __syncthreads();
+    if (warp != 0) return;
+#pragma unroll
+    for (int w = 1; w < RF32_WARPS; ++w) m = fmaxf(m, smax[w][lane]);
+    float s = 1.0f;
+    if (r < rows) {
+        if (B) m = fmaxf(m, fabsf(B[r]));
+        s = pow2_scale(2.0 * (double)m);
     }
     rs[r] = s;
     rs[rows_pad + r] = 1.0f / s;
@@ -354,7 +343,7 @@ struct FaceSum {
 };
 __device__ __forceinline__ float scaled_f32(FaceSum v, float s)
 {
-    return pow2_scaled_to_f32(v.x, (int)((__float_as_uint(s) >> 23) & 0xFF) - 127 - 2);
+    return pow2_scaled_to_f32(v.x, rts_rows::scale_log2(s) - 2);
 }
 
 // Transpose-and-split through shared memory.  Tile: 32 in-directions x 64
@@ -530,7 +519,23 @@ int rts_pp_rows_from_faces(rts_ctx* ctx, const double* illum, int64_t N, int64_t
                            int mode, float* rs, int64_t npad, uint16_t* A, cudaStream_t st, bool bound)
 {
     const bool fp16 = mode == 1;
-    if (fp16 || bound) {  // the scales; the unscaled formats keep them only as a bound of the rows
+    size_t smem = 0;
+    if (const int lg = rts_rows::cells_log2(kpad, &smem)) {
+        // one pass; the unscaled formats write the scales only as a bound of the rows
+        rts_rows::Args a;
+        a.illum = illum, a.N = N, a.ld = ld, a.M = M, a.kpad = kpad, a.pitch = rts_rows::pitch_of(kpad), a.lg = lg;
+        a.B = B, a.rs = fp16 || bound ? rs : nullptr, a.npad = npad, a.A = A;
+        auto* kernel = mode == 2   ? rts_rows::rows_from_faces_kernel<2>
+                       : mode == 1 ? rts_rows::rows_from_faces_kernel<1>
+                                   : rts_rows::rows_from_faces_kernel<0>;
+        RTS_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<(unsigned)(npad >> lg), rts_rows::THREADS, smem, st>>>(a);
+        RTS_CHECK_LAUNCH(ctx, "rows_from_faces_kernel");
+        ctx->launches++;
+        return RTS_OK;
+    }
+    // rows too long for shared memory (M > 14,000): a pass for the scales, a pass for the rows
+    if (fp16 || bound) {
         rowscale_faces_kernel<<<(unsigned)((npad + 127) / 128), 128, 0, st>>>(illum, N, ld, M, B, rs, npad);
         RTS_CHECK_LAUNCH(ctx, "rowscale_faces_kernel");
         ctx->launches++;
@@ -586,7 +591,7 @@ int rts_pp_rows_from_f32(rts_ctx* ctx, const float* ibar, int64_t N, int M, int6
 {
     const bool fp16 = mode == 1;
     if (fp16 || bound) {
-        rowscale_f32_kernel<<<(unsigned)((rows_pad + 127) / 128), 128, 0, st>>>(ibar, N, M, rows, B, rs, rows_pad);
+        rowscale_f32_kernel<<<(unsigned)(rows_pad / 32), 32 * RF32_WARPS, 0, st>>>(ibar, N, M, rows, B, rs, rows_pad);
         RTS_CHECK_LAUNCH(ctx, "rowscale_f32_kernel");
         ctx->launches++;
     }
