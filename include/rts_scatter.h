@@ -146,7 +146,12 @@ int rts_copy_illum(rts_ctx* ctx, int64_t size, const double* illum_host);
  * (4 bytes per cell and in-direction, 8 for RTS_PREC_TF32X3) and, where the
  * HBM budget and the device leave room, a staging of the FP64 face sums
  * (8 bytes per cell and direction) that speeds up their preparation; without
- * that room the rows are prepared directly, with the same results. */
+ * that room the rows are prepared directly, with the same results.
+ * RTS_PREC_FP64 computes with FP64's accuracy on either the FP64 CUDA cores
+ * or, for Thomson and smooth Henyey-Greenstein kernels on sm_10x, the tensor
+ * cores (exact products of FP16 digits, integer sums), which hold 12 bytes per
+ * direction pair and, during a call, up to 2 GB of scratch; without that room
+ * the CUDA cores run. */
 int rts_set_precision(rts_ctx* ctx, int precision);
 int rts_get_precision(const rts_ctx* ctx, int* precision);
 

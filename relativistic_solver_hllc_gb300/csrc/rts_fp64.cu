@@ -52,17 +52,34 @@ __device__ __forceinline__ void residual_max(unsigned long long* dst, double v)
 // width changes no result.  GB300's FP64 pipe retires about two FMAs per SM
 // per cycle, far below the shared-memory loads that feed them, so a narrow
 // tile costs about NB/4 of a full one.
-template <bool kUpdate, bool kResidual, int NB>
+//
+// kList: the tile's cells are entries [c0, n) of fx.list instead of
+// consecutive ones, and only the outputs marked in fx.mask are written.
+struct ListArgs {
+    const unsigned int* list;  // null: the identity (every cell)
+    const unsigned int* mask;  // [quarter tile][ld], a bit per column; null: every output
+    int64_t ld;
+    int bn, k_base;
+    __device__ bool marked(int64_t c, int k) const
+    {
+        if (!mask) return true;
+        const int kk = k - k_base, group = kk / (bn / 4);  // a word per quarter tile
+        return (mask[(int64_t)group * ld + c] >> (kk - group * (bn / 4))) & 1u;
+    }
+};
+
+template <bool kUpdate, bool kResidual, int NB, bool kList = false>
 __device__ __forceinline__ void scatter_tile(double (*sI)[F64_TC], double (*sW)[F64_TK],
                                              const double* __restrict__ illum, const double* __restrict__ W,
-                                             int64_t N, int M, int ldw, int k0, int k_end, double* __restrict__ S,
-                                             const double* __restrict__ B, double lambda,
-                                             unsigned long long* __restrict__ resid)
+                                             int64_t c0, int64_t n, int64_t N, int M, int ldw, int k0, int k_end,
+                                             double* __restrict__ S, const double* __restrict__ B, double lambda,
+                                             unsigned long long* __restrict__ resid, const ListArgs& fx = ListArgs())
 {
     constexpr int TK = 16 * NB;
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
-    const int64_t c0 = (int64_t)blockIdx.x * F64_TC;
+    // cell of list position p < n
+    auto cell = [&](int64_t p) { return kList && fx.list ? (int64_t)fx.list[p] : p; };
 
     double acc[NB][8];
 #pragma unroll
@@ -80,8 +97,8 @@ __device__ __forceinline__ void scatter_tile(double (*sI)[F64_TC], double (*sW)[
             const int j = j0 + jj;
             const int64_t c = c0 + cc;
             double v = 0.0;
-            if (j < M && c < N) {
-                const double2* src = reinterpret_cast<const double2*>(illum + ((int64_t)j * N + c) * 4);
+            if (j < M && c < n) {
+                const double2* src = reinterpret_cast<const double2*>(illum + ((int64_t)j * N + cell(c)) * 4);
                 const double2 a = __ldg(src), b = __ldg(src + 1);
                 double I = 0.0;  // faces 0..3 in order, then /4 (GET_FACE_TO_CELL)
                 I += a.x;
@@ -123,8 +140,9 @@ __device__ __forceinline__ void scatter_tile(double (*sI)[F64_TC], double (*sW)[
         if (k >= k_end) continue;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int64_t c = c0 + tx + 16 * i;
-            if (c >= N) continue;
+            if (c0 + tx + 16 * i >= n) continue;
+            const int64_t c = cell(c0 + tx + 16 * i);
+            if (kList && !fx.marked(c, k)) continue;
             double v = acc[m][i];
             if (kUpdate) v = (1.0 - lambda) * B[c] + lambda * v;
             double* dst = S + (int64_t)k * N + c;
@@ -140,7 +158,7 @@ __device__ __forceinline__ void scatter_tile(double (*sI)[F64_TC], double (*sW)[
 // tile of 16*nb_last (nb_last 1..4) for the rest.  The narrow tiles are last
 // in launch order, so they fill the final wave.
 template <bool kUpdate, bool kResidual>
-__global__ void __launch_bounds__(F64_THREADS)
+__global__ void __launch_bounds__(F64_THREADS, 2)
 scatter_fp64_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t N,
                     int M, int ldw, int k_begin, int k_end, int n_full, int nb_last, double* __restrict__ S,
                     const double* __restrict__ B, double lambda,
@@ -148,22 +166,46 @@ scatter_fp64_kernel(const double* __restrict__ illum, const double* __restrict__
 {
     __shared__ double sI[F64_KC][F64_TC];
     __shared__ double sW[F64_KC][F64_TK];
+    const int64_t c0 = (int64_t)blockIdx.x * F64_TC;
     const int k0 = k_begin + (int)blockIdx.y * F64_TK;
     const int nb = (int)blockIdx.y < n_full ? 4 : nb_last;
     switch (nb) {
     case 1:
-        scatter_tile<kUpdate, kResidual, 1>(sI, sW, illum, W, N, M, ldw, k0, k_end, S, B, lambda, resid);
+        scatter_tile<kUpdate, kResidual, 1>(sI, sW, illum, W, c0, N, N, M, ldw, k0, k_end, S, B, lambda, resid);
         break;
     case 2:
-        scatter_tile<kUpdate, kResidual, 2>(sI, sW, illum, W, N, M, ldw, k0, k_end, S, B, lambda, resid);
+        scatter_tile<kUpdate, kResidual, 2>(sI, sW, illum, W, c0, N, N, M, ldw, k0, k_end, S, B, lambda, resid);
         break;
     case 3:
-        scatter_tile<kUpdate, kResidual, 3>(sI, sW, illum, W, N, M, ldw, k0, k_end, S, B, lambda, resid);
+        scatter_tile<kUpdate, kResidual, 3>(sI, sW, illum, W, c0, N, N, M, ldw, k0, k_end, S, B, lambda, resid);
         break;
     default:
-        scatter_tile<kUpdate, kResidual, 4>(sI, sW, illum, W, N, M, ldw, k0, k_end, S, B, lambda, resid);
+        scatter_tile<kUpdate, kResidual, 4>(sI, sW, illum, W, c0, N, N, M, ldw, k0, k_end, S, B, lambda, resid);
         break;
     }
+}
+
+// The outputs that the tensor-core route left (rts_launch_scatter_list): a few
+// CTAs walk the tiles of the listed cells; count and list are the device's, so
+// nothing waits on the host.  Usually there are none and the launch costs its
+// latency.
+template <bool kUpdate, bool kResidual>
+__global__ void __launch_bounds__(F64_THREADS, 2)
+scatter_list_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t n, int64_t N, int M,
+                    int ldw, int k_begin, int k_end, double* __restrict__ S, const double* __restrict__ B,
+                    double lambda, unsigned long long* __restrict__ resid, ListArgs fx,
+                    const unsigned int* __restrict__ count)
+{
+    __shared__ double sI[F64_KC][F64_TC];
+    __shared__ double sW[F64_KC][F64_TK];
+    const bool whole = count[1] != 0;  // the contraction gave up: every output of the range
+    const int64_t cells = whole ? n : (int64_t)count[0];
+    if (whole) fx.list = fx.mask = nullptr;
+    const int gy = (k_end - k_begin + F64_TK - 1) / F64_TK;
+    const int64_t work = (cells + F64_TC - 1) / F64_TC * gy;
+    for (int64_t w = blockIdx.x; w < work; w += gridDim.x)
+        scatter_tile<kUpdate, kResidual, 4, true>(sI, sW, illum, W, w / gy * F64_TC, cells, N, M, ldw,
+                                                  k_begin + (int)(w % gy) * F64_TK, k_end, S, B, lambda, resid, fx);
 }
 
 // The y extent of scatter_fp64_kernel's grid over `width` out-directions.
@@ -502,6 +544,9 @@ int rts_launch_scatter_fp64(rts_ctx* ctx, int64_t k_begin, int64_t k_end, cudaSt
                             const double* B, double lambda, bool update, bool residual)
 {
     if (k_end <= k_begin) return RTS_OK;
+    bool taken = false;
+    const int rc = rts_sliced_scatter(ctx, 0, ctx->N, k_begin, k_end, st, B, lambda, update, residual, &taken);
+    if (rc != RTS_OK || taken) return rc;
     const int64_t gx = (ctx->N + F64_TC - 1) / F64_TC;
     const DirTiles dt = dir_tiles(k_end - k_begin);
     RTS_REQUIRE(ctx, gx < (1ll << 31) && dt.gy < 65536, RTS_ERR_UNSUPPORTED, "FP64 grid too large");
@@ -522,6 +567,25 @@ int rts_launch_scatter_fp64(rts_ctx* ctx, int64_t k_begin, int64_t k_end, cudaSt
             ctx->d_S, nullptr, 0.0, ctx->resid_target);
     rts_timing_end(ctx, st);
     RTS_CHECK_LAUNCH(ctx, "scatter_fp64_kernel");
+    ctx->launches++;
+    return RTS_OK;
+}
+
+int rts_launch_scatter_list(rts_ctx* ctx, int64_t c0, int64_t n, int64_t k_begin, int64_t k_end, int bn,
+                            int64_t mask_ld, const unsigned int* mask, const unsigned int* list,
+                            const unsigned int* count, cudaStream_t st, const double* B, double lambda, bool update,
+                            bool residual)
+{
+    const ListArgs fx{list, mask, mask_ld, bn, (int)k_begin};
+    const int64_t tiles = (n + F64_TC - 1) / F64_TC * ((k_end - k_begin + F64_TK - 1) / F64_TK);
+    const unsigned grid = (unsigned)(tiles < 2 * ctx->num_sms ? tiles : 2 * ctx->num_sms);
+    auto* kernel = update && residual ? scatter_list_kernel<true, true>
+                   : update           ? scatter_list_kernel<true, false>
+                                      : scatter_list_kernel<false, false>;
+    kernel<<<grid, F64_THREADS, 0, st>>>(ctx->d_illum + 4 * c0, ctx->d_W, n, ctx->N, (int)ctx->M, (int)ctx->local(),
+                                         (int)k_begin, (int)k_end, ctx->d_S + c0, update ? B + c0 : nullptr, lambda,
+                                         ctx->resid_target, fx, count);
+    RTS_CHECK_LAUNCH(ctx, "scatter_list_kernel");
     ctx->launches++;
     return RTS_OK;
 }

@@ -65,6 +65,11 @@ int make_map(rts_ctx* ctx, void* map, const void* base, int64_t rows, int64_t un
 
 }  // namespace
 
+int rts_group_make_map(rts_ctx* ctx, void* map, const void* base, int64_t rows, int64_t units, int box_rows)
+{
+    return make_map(ctx, map, base, rows, units, box_rows);
+}
+
 // ---------------------------------------------------------------------------
 // problem and batch objects
 // ---------------------------------------------------------------------------

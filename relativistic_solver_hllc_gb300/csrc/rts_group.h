@@ -12,6 +12,9 @@
 struct rts_ctx;
 struct rts_batch;
 
+// Tensor map of rows [rows][units] of 16-bit values in boxes of 64 x box_rows
+// with a 128-byte swizzle (map: a CUtensorMap).
+int rts_group_make_map(rts_ctx* ctx, void* map, const void* base, int64_t rows, int64_t units, int box_rows);
 // One resident problem: split operands, scales, source, albedo, output.
 struct GProb {
     int64_t id = 0;

@@ -101,6 +101,17 @@ struct rts_split_state {
     int eager_mode = -1;
 };
 
+// FP64 integrals on the tensor cores (rts_sliced.cu): W^T as FP16 digit rows,
+// built by the first call after a change of W.
+struct rts_sliced_state {
+    uint16_t* w = nullptr;    // [local][6*kpad]
+    int* colexp = nullptr;    // [local]
+    size_t w_bytes = 0, e_bytes = 0;
+    int64_t w_version = -1;   // ctx->w_version the rows were built from
+    cudaEvent_t ev_w = nullptr;                 // rows built
+    cudaEvent_t ev_use[RTS_STREAM_COUNT] = {};  // on each slot's stream: its last contraction queued
+};
+
 // Device state of the transport sweep (rts_sweep.cu): the mesh, the
 // per-direction structures of the local directions and the medium.  The unit
 // of work is an out-face of a cell (its 3 nodes); per local direction d:
@@ -199,6 +210,7 @@ struct rts_ctx {
     int64_t inputs_version = 0;       // bumped at every write of the device Illum, W or scattering array
     cudaEvent_t ev_sync[RTS_STREAM_COUNT] = {};   // rts_sync_stream deadlines
     rts_split_state split;
+    rts_sliced_state sliced;
     int split_flush = 0;         // hi*hi drain period in stages (0: default)
     int split_bias = 0;          // truncation correction: 0 conservation-based (relaxed steps), -1 none, >0 constant (1e-10 units)
     int tuning_epoch = 0;        // bumped when a setting that batch tables copy changes
@@ -235,6 +247,21 @@ void rts_pfree(rts_ctx* ctx, void* p, size_t bytes, cudaStream_t st);
 // Kernel launchers (defined in the .cu files).
 int rts_launch_scatter_fp64(rts_ctx* ctx, int64_t k_begin, int64_t k_end, cudaStream_t st,
                             const double* B, double lambda, bool update, bool residual);
+// The FP64 integral of cells [c_begin, c_end) and local out-directions
+// [k_begin, k_end) on the tensor cores (rts_sliced.cu).  *taken is false, and
+// nothing was queued, where the context's weights or size do not suit it or
+// there is no room for its scratch.
+int rts_sliced_scatter(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_begin, int64_t k_end, cudaStream_t st,
+                       const double* B, double lambda, bool update, bool residual, bool* taken);
+void rts_sliced_free(rts_ctx* ctx);
+// Its rows that the digits could not carry, by the FP64 kernel: cells
+// list[0..*count) of the range starting at c0, the outputs marked in mask
+// [quarter tile][mask_ld], a bit per column (tiles of bn columns).  With
+// count[1] set (a bounded wait of the contraction gave up) all n cells whole.
+int rts_launch_scatter_list(rts_ctx* ctx, int64_t c0, int64_t n, int64_t k_begin, int64_t k_end, int bn,
+                            int64_t mask_ld, const unsigned int* mask, const unsigned int* list,
+                            const unsigned int* count, cudaStream_t st, const double* B, double lambda, bool update,
+                            bool residual);
 int rts_launch_moments(rts_ctx* ctx, cudaStream_t st);
 int rts_launch_illum_params(rts_ctx* ctx, cudaStream_t st);
 int rts_launch_update(rts_ctx* ctx, int64_t k_begin, int64_t k_end, cudaStream_t st,
@@ -292,6 +319,10 @@ int rts_pp_face_sums(rts_ctx* ctx, const double* illum, int64_t N, int64_t ld, i
 int rts_pp_rows_from_sums(rts_ctx* ctx, int64_t N, int M, int kpad, const double* B, int mode, float* rs, int64_t npad,
                           uint16_t* A, const double* sums, const unsigned long long* cmax, cudaStream_t st,
                           bool bound = false);
+// FP64 rows as FP16 digits (rts_rows.cuh) of cells [0, N) of a device Illum:
+// rows A [N][6*kpad], row exponents, and the rows without digits on the list.
+int rts_pp_slice_rows(rts_ctx* ctx, const double* illum, int64_t N, int64_t ld, int M, int kpad, uint16_t* A, int* exps,
+                      unsigned int* flags, unsigned int* list, unsigned int* count, cudaStream_t st);
 int rts_pp_join_rows(rts_ctx* ctx, const uint16_t* A, int64_t N, int M, int64_t rows, int kpad, const float* rs_inv,
                      int mode, double* out, cudaStream_t st);
 int rts_pp_f32_to_f64(rts_ctx* ctx, const float* s, double* d, int64_t n, cudaStream_t st);

@@ -58,7 +58,7 @@ __device__ double block_sum(double x, double* red)
 // time in coalesced 256-byte pieces -- the next piece while the current one
 // is added -- and turns them through shared memory.  One block that walked
 // the rows thread by thread (the former layout: a 32-byte sector per value,
-// one SM) took 1,173 us at M = 1000 against 64 us for the three launches.
+// one SM) took 1,173 us at M = 1000 against 239 us for the three launches.
 constexpr int WS_T = 32;
 
 // Row sums of f(W[j][k], k) over k in order for rows [32 b, 32 b + 32): lane
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(WS_T) w_stats_u_kernel(const double* __restric
 // (lane = out-direction) for the columns' maxima, then each takes every 8th
 // group of 32 in-directions, whose split parts are 128 contiguous bytes of a
 // lane's own row (256 for TF32).  A thread per out-direction over all
-// in-directions (the former layout) wrote 2 bytes at a time: 455 -> 16 us at
+// in-directions (the former layout) wrote 2 bytes at a time: 455 -> 42 us at
 // M = 1000.
 constexpr int SW_THREADS = 256, SW_WARPS = SW_THREADS / 32;
 __global__ void __launch_bounds__(SW_THREADS)
@@ -522,7 +522,7 @@ int rts_pp_rows_from_faces(rts_ctx* ctx, const double* illum, int64_t N, int64_t
     size_t smem = 0;
     if (const int lg = rts_rows::cells_log2(kpad, &smem)) {
         // one pass; the unscaled formats write the scales only as a bound of the rows
-        rts_rows::Args a;
+        rts_rows::Args a{};
         a.illum = illum, a.N = N, a.ld = ld, a.M = M, a.kpad = kpad, a.pitch = rts_rows::pitch_of(kpad), a.lg = lg;
         a.B = B, a.rs = fp16 || bound ? rs : nullptr, a.npad = npad, a.A = A;
         auto* kernel = mode == 2   ? rts_rows::rows_from_faces_kernel<2>
@@ -543,6 +543,23 @@ int rts_pp_rows_from_faces(rts_ctx* ctx, const double* illum, int64_t N, int64_t
     dim3 grid((unsigned)((N + 63) / 64), (unsigned)(kpad / 32));
     split_faces_kernel<<<grid, 256, 0, st>>>(illum, N, ld, M, kpad, fp16 ? rs : nullptr, mode, A);
     RTS_CHECK_LAUNCH(ctx, "split_faces_kernel");
+    ctx->launches++;
+    return RTS_OK;
+}
+
+int rts_pp_slice_rows(rts_ctx* ctx, const double* illum, int64_t N, int64_t ld, int M, int kpad, uint16_t* A, int* exps,
+                      unsigned int* flags, unsigned int* list, unsigned int* count, cudaStream_t st)
+{
+    size_t smem = 0;
+    const int lg = rts_rows::cells_log2(kpad, &smem);
+    RTS_REQUIRE(ctx, lg > 0, RTS_ERR_UNSUPPORTED, "rows of %d directions do not fit shared memory", kpad);
+    rts_rows::Args a{};
+    a.illum = illum, a.N = N, a.ld = ld, a.M = M, a.kpad = kpad, a.pitch = rts_rows::pitch_of(kpad), a.lg = lg, a.A = A;
+    a.rows = rts_rows::RowList{exps, flags, list, count};
+    auto* kernel = rts_rows::rows_from_faces_kernel<3>;
+    RTS_CUDA_TRY(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<(unsigned)((N + (1 << lg) - 1) >> lg), rts_rows::THREADS, smem, st>>>(a);
+    RTS_CHECK_LAUNCH(ctx, "rows_from_faces_kernel");
     ctx->launches++;
     return RTS_OK;
 }

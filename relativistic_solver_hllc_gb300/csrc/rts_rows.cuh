@@ -72,6 +72,63 @@ inline int cells_log2(int kpad, size_t* smem)
     return 0;
 }
 
+// ---- FP64 rows as sums of FP16 digits (mode 3, rts_sliced.cu) ----
+//
+// x = m * 2^(e - 54), 0 <= m <= 2^54 an integer, is held as six digits,
+//   m = sum_i d_i 2^(9 (5 - i)),  d_0 in [0, 512], d_1..d_5 in [-256, 255],
+// each exact in FP16.  Adding 256 to every digit but the first makes them plain
+// bit fields, and 0x6400 + n is the FP16 number 1024 + n, so a digit costs a
+// shift, a mask and half of a packed subtraction.
+constexpr int SLICES = 6;
+constexpr int SLICE_BITS = 54;                 // x < 2^e is rounded to a multiple of 2^(e - 54)
+constexpr int ROW_BAD = 1 << 20;               // row exponents: a value negative or not finite, or e out of range
+constexpr int ROW_ZERO = (1 << 20) + 1;        // every value of the row is zero
+constexpr int ROW_EXP_MAX = 900;               // |e| of a row that takes the digits
+
+// m of x >= 0 at the row exponent e (x < 2^e), rounded half up.
+__device__ __forceinline__ unsigned long long slice_int(double x, int e)
+{
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+    const int ex = (int)(u >> 52);
+    const unsigned long long f = u & 0xFFFFFFFFFFFFFull;
+    const unsigned long long t = (ex ? (f | 0x10000000000000ull) : f) << 1;
+    const int sh = min(1022 + e - (ex ? ex : 1), 63);  // x / 2^(e - 54) = t / 2^sh, sh >= 0
+    return (t + ((1ull << sh) >> 1)) >> sh;
+}
+
+// The six digits of two values, packed as FP16 pairs (first in the low half).
+__device__ __forceinline__ void slice_digits(unsigned long long m0, unsigned long long m1, uint32_t (&d)[SLICES])
+{
+    // 256 for the digits 1..5
+    constexpr unsigned long long OFF = (1ull << 8) + (1ull << 17) + (1ull << 26) + (1ull << 35) + (1ull << 44);
+    const unsigned long long a = m0 + OFF, b = m1 + OFF;
+    const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
+    auto field = [](uint32_t x, uint32_t y, uint32_t sub) {
+        const uint32_t w = (x | (y << 16)) + 0x64006400u;
+        const __half2 h = __hsub2(*reinterpret_cast<const __half2*>(&w), *reinterpret_cast<const __half2*>(&sub));
+        return *reinterpret_cast<const uint32_t*>(&h);
+    };
+    constexpr uint32_t S0 = 0x64006400u, S256 = 0x65006500u;  // FP16 1024 and 1280 = 1024 + 256, twice
+    d[5] = field(al & 511u, bl & 511u, S256);
+    d[4] = field((al >> 9) & 511u, (bl >> 9) & 511u, S256);
+    d[3] = field((al >> 18) & 511u, (bl >> 18) & 511u, S256);
+    d[2] = field(__funnelshift_r(al, ah, 27) & 511u, __funnelshift_r(bl, bh, 27) & 511u, S256);
+    d[1] = field((ah >> 4) & 511u, (bh >> 4) & 511u, S256);
+    d[0] = field(ah >> 13, bh >> 13, S0);
+}
+
+// offset (in halves) of digit 0 of in-direction j in a sliced row: per 32
+// in-directions, the 32 values of each digit in turn (6 x 64 bytes)
+__host__ __device__ __forceinline__ int64_t ilv_slice(int64_t j) { return (j >> 5) * (32 * SLICES) + (j & 31); }
+
+// Rows that the digits cannot carry are collected for the FP64 kernel.
+struct RowList {
+    int* exps;            // [N] row exponents, ROW_BAD or ROW_ZERO
+    unsigned int* flags;  // [N] the row is on the list
+    unsigned int* list;   // [N]
+    unsigned int* count;
+};
+
 struct Args {
     const double* illum;  // cell 0 of the range; a direction's row holds ld cells
     int64_t N, ld;        // cells of the range
@@ -80,9 +137,11 @@ struct Args {
     float* rs;            // [2*npad] row scales and their inverses (or null)
     int64_t npad;
     uint16_t* A;          // rows
+    RowList rows;         // kMode 3
 };
 
-// kMode: 0 BF16, 1 FP16 (scaled), 2 TF32.
+// kMode: 0 BF16, 1 FP16 (scaled), 2 TF32, 3 FP64 as six FP16 digits (12 bytes
+// per cell-direction written).
 template <int kMode>
 __global__ void __launch_bounds__(THREADS, 3) rows_from_faces_kernel(const Args a)
 {
@@ -101,7 +160,8 @@ __global__ void __launch_bounds__(THREADS, 3) rows_from_faces_kernel(const Args 
         double* row = sums + cell * a.pitch;
         const double* src = a.illum + 4 * c;
         const int64_t dir = 4 * a.ld;
-        // NaN is skipped, as fmax does; non-negative doubles order as their bits
+        // NaN is skipped, as fmax does (kMode 3 keeps it and negative values:
+        // larger than any other); non-negative doubles order as their bits
         unsigned long long mx = 0;
         constexpr int U = 4;
         for (int j0 = t >> lg; j0 < a.kpad; j0 += U * jstep) {
@@ -126,8 +186,13 @@ __global__ void __launch_bounds__(THREADS, 3) rows_from_faces_kernel(const Args 
                 I += q[i].x;
                 I += q[i].y;
                 row[j] = I;
-                const unsigned long long ub = (unsigned long long)__double_as_longlong(I) & 0x7FFFFFFFFFFFFFFFull;
-                if (ub <= 0x7FF0000000000000ull && ub > mx) mx = ub;
+                unsigned long long ub = (unsigned long long)__double_as_longlong(I);
+                if (kMode == 3) {
+                    if (ub == 0x8000000000000000ull) ub = 0;  // -0; negative values lie above every other pattern
+                } else {
+                    ub &= 0x7FFFFFFFFFFFFFFFull;
+                }
+                if ((kMode == 3 || ub <= 0x7FF0000000000000ull) && ub > mx) mx = ub;
             }
         }
         for (int o = 16; o >= cells; o >>= 1) {
@@ -137,7 +202,19 @@ __global__ void __launch_bounds__(THREADS, 3) rows_from_faces_kernel(const Args 
         if ((t & 31) < cells) atomicMax(&cmax[cell], mx);
     }
     __syncthreads();
-    if (t < cells) {
+    if (kMode == 3 && t < cells) {
+        // the exponent of the largest sum: every sum of the row < 2^e
+        const unsigned long long mx = cmax[t];
+        const int ex = (int)(mx >> 52), e = ex - 1022;
+        const bool bad = mx != 0 && (ex == 0 || ex >= 0x7FF || e < -ROW_EXP_MAX || e > ROW_EXP_MAX);
+        klog[t] = mx == 0 ? ROW_ZERO : bad ? ROW_BAD : e;
+        if (c < a.N) {
+            a.rows.exps[c] = klog[t];
+            a.rows.flags[c] = bad ? 1u : 0u;
+            if (bad) a.rows.list[atomicAdd(a.rows.count, 1u)] = (unsigned int)c;
+        }
+    }
+    if (kMode != 3 && t < cells) {
         // the scale of 2 max(|mean|, |B|): max_j |sum / 4| = max_j |sum| / 4 exactly
         float s = 1.0f;
         if (a.rs && c < a.N) {
@@ -160,6 +237,15 @@ __global__ void __launch_bounds__(THREADS, 3) rows_from_faces_kernel(const Args 
         if (c0 + uc >= a.N || j >= a.kpad) continue;
         const double2 x = *reinterpret_cast<const double2*>(sums + uc * a.pitch + j);
         const int k = klog[uc];
+        if (kMode == 3) {
+            uint32_t d[SLICES];
+            const bool none = k >= ROW_BAD;  // zero digits
+            slice_digits(none ? 0 : slice_int(x.x, k), none ? 0 : slice_int(x.y, k), d);
+            uint16_t* row = a.A + (c0 + uc) * SLICES * (int64_t)a.kpad + ilv_slice(j);
+#pragma unroll
+            for (int i = 0; i < SLICES; ++i) *reinterpret_cast<uint32_t*>(row + 32 * i) = d[i];
+            continue;
+        }
         const float f0 = pow2_scaled_to_f32(x.x, k), f1 = pow2_scaled_to_f32(x.y, k);
         if (kMode == 2) {
             float* row = reinterpret_cast<float*>(a.A + (c0 + uc) * 4 * (int64_t)a.kpad) + rts_ptx::ilv_hi_tf32(j);
