@@ -475,16 +475,8 @@ int rts_scattering(rts_ctx* ctx, const double* illum_host, double* host_out)
         rts_inputs_changed(ctx);
         return rts_split_host_call(ctx, ctx->call_precision, src, nullptr, 1.0, dst);
     }
-    cudaStream_t st = ctx->streams[RTS_STREAM_SCATTERING_1];
-    RTS_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_illum, src, rts_bytes<double>(ctx->M * ctx->N * 4),
-                                      cudaMemcpyHostToDevice, st));
     rts_inputs_changed(ctx);
-    int rc = rts_launch_scatter_fp64(ctx, 0, ctx->local(), st, nullptr, 0.0, false, false);
-    if (rc != RTS_OK) return rc;
-    RTS_CUDA_TRY(ctx, cudaMemcpyAsync(dst, ctx->d_S, rts_bytes<double>(ctx->local() * ctx->N),
-                                      cudaMemcpyDeviceToHost, st));
-    RTS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    return RTS_OK;
+    return rts_fp64_host_call(ctx, src, nullptr, 1.0, dst);
 }
 
 int rts_scattering_update(rts_ctx* ctx, int precision, const double* illum_host,
@@ -501,21 +493,8 @@ int rts_scattering_update(rts_ctx* ctx, int precision, const double* illum_host,
         return rts_split_host_call(ctx, precision, illum_host, B_host, lambda, S_host);
     }
     RTS_REQUIRE(ctx, precision == RTS_PREC_FP64, RTS_ERR_INVALID_ARGUMENT, "unknown precision %d", precision);
-    cudaStream_t st = ctx->streams[RTS_STREAM_SCATTERING_1];
-    RTS_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_illum, illum_host,
-                                      rts_bytes<double>(ctx->M * ctx->N * 4),
-                                      cudaMemcpyHostToDevice, st));
     rts_inputs_changed(ctx);
-    const bool update = B_host != nullptr && lambda != 1.0;
-    if (update)
-        RTS_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_B, B_host, rts_bytes<double>(ctx->N),
-                                          cudaMemcpyHostToDevice, st));
-    int rc = rts_launch_scatter_fp64(ctx, 0, ctx->local(), st, ctx->d_B, lambda, update, false);
-    if (rc != RTS_OK) return rc;
-    RTS_CUDA_TRY(ctx, cudaMemcpyAsync(S_host, ctx->d_S, rts_bytes<double>(ctx->local() * ctx->N),
-                                      cudaMemcpyDeviceToHost, st));
-    RTS_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-    return RTS_OK;
+    return rts_fp64_host_call(ctx, illum_host, B_host, lambda, S_host);
 }
 
 int rts_read_scattering(rts_ctx* ctx, int64_t start, int64_t end, int stream, double* host_out)

@@ -159,7 +159,7 @@ __device__ __forceinline__ void scatter_tile(double (*sI)[F64_TC], double (*sW)[
 // in launch order, so they fill the final wave.
 template <bool kUpdate, bool kResidual>
 __global__ void __launch_bounds__(F64_THREADS, 2)
-scatter_fp64_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t N,
+scatter_fp64_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t n, int64_t N,
                     int M, int ldw, int k_begin, int k_end, int n_full, int nb_last, double* __restrict__ S,
                     const double* __restrict__ B, double lambda,
                     unsigned long long* __restrict__ resid)
@@ -171,16 +171,16 @@ scatter_fp64_kernel(const double* __restrict__ illum, const double* __restrict__
     const int nb = (int)blockIdx.y < n_full ? 4 : nb_last;
     switch (nb) {
     case 1:
-        scatter_tile<kUpdate, kResidual, 1>(sI, sW, illum, W, c0, N, N, M, ldw, k0, k_end, S, B, lambda, resid);
+        scatter_tile<kUpdate, kResidual, 1>(sI, sW, illum, W, c0, n, N, M, ldw, k0, k_end, S, B, lambda, resid);
         break;
     case 2:
-        scatter_tile<kUpdate, kResidual, 2>(sI, sW, illum, W, c0, N, N, M, ldw, k0, k_end, S, B, lambda, resid);
+        scatter_tile<kUpdate, kResidual, 2>(sI, sW, illum, W, c0, n, N, M, ldw, k0, k_end, S, B, lambda, resid);
         break;
     case 3:
-        scatter_tile<kUpdate, kResidual, 3>(sI, sW, illum, W, c0, N, N, M, ldw, k0, k_end, S, B, lambda, resid);
+        scatter_tile<kUpdate, kResidual, 3>(sI, sW, illum, W, c0, n, N, M, ldw, k0, k_end, S, B, lambda, resid);
         break;
     default:
-        scatter_tile<kUpdate, kResidual, 4>(sI, sW, illum, W, c0, N, N, M, ldw, k0, k_end, S, B, lambda, resid);
+        scatter_tile<kUpdate, kResidual, 4>(sI, sW, illum, W, c0, n, N, M, ldw, k0, k_end, S, B, lambda, resid);
         break;
     }
 }
@@ -543,28 +543,28 @@ int grid_stride_blocks(rts_ctx* ctx, int64_t n, int threads)
 int rts_launch_scatter_fp64(rts_ctx* ctx, int64_t k_begin, int64_t k_end, cudaStream_t st,
                             const double* B, double lambda, bool update, bool residual)
 {
-    if (k_end <= k_begin) return RTS_OK;
+    return rts_launch_scatter_fp64_cells(ctx, 0, ctx->N, k_begin, k_end, st, B, lambda, update, residual);
+}
+
+int rts_launch_scatter_fp64_cells(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_begin, int64_t k_end,
+                                  cudaStream_t st, const double* B, double lambda, bool update, bool residual)
+{
+    if (k_end <= k_begin || c_end <= c_begin) return RTS_OK;
     bool taken = false;
-    const int rc = rts_sliced_scatter(ctx, 0, ctx->N, k_begin, k_end, st, B, lambda, update, residual, &taken);
+    const int rc = rts_sliced_scatter(ctx, c_begin, c_end, k_begin, k_end, st, B, lambda, update, residual, &taken);
     if (rc != RTS_OK || taken) return rc;
-    const int64_t gx = (ctx->N + F64_TC - 1) / F64_TC;
+    const int64_t n = c_end - c_begin, gx = (n + F64_TC - 1) / F64_TC;
     const DirTiles dt = dir_tiles(k_end - k_begin);
     RTS_REQUIRE(ctx, gx < (1ll << 31) && dt.gy < 65536, RTS_ERR_UNSUPPORTED, "FP64 grid too large");
     dim3 grid((unsigned)gx, (unsigned)dt.gy);
-    const int ldw = (int)ctx->local();
+    auto* kernel = update && residual ? scatter_fp64_kernel<true, true>
+                   : update           ? scatter_fp64_kernel<true, false>
+                                      : scatter_fp64_kernel<false, false>;
     rts_timing_begin(ctx, st);
-    if (update && residual)
-        scatter_fp64_kernel<true, true><<<grid, F64_THREADS, 0, st>>>(
-            ctx->d_illum, ctx->d_W, ctx->N, (int)ctx->M, ldw, (int)k_begin, (int)k_end, dt.n_full, dt.nb_last,
-            ctx->d_S, B, lambda, ctx->resid_target);
-    else if (update)
-        scatter_fp64_kernel<true, false><<<grid, F64_THREADS, 0, st>>>(
-            ctx->d_illum, ctx->d_W, ctx->N, (int)ctx->M, ldw, (int)k_begin, (int)k_end, dt.n_full, dt.nb_last,
-            ctx->d_S, B, lambda, ctx->resid_target);
-    else
-        scatter_fp64_kernel<false, false><<<grid, F64_THREADS, 0, st>>>(
-            ctx->d_illum, ctx->d_W, ctx->N, (int)ctx->M, ldw, (int)k_begin, (int)k_end, dt.n_full, dt.nb_last,
-            ctx->d_S, nullptr, 0.0, ctx->resid_target);
+    kernel<<<grid, F64_THREADS, 0, st>>>(ctx->d_illum + 4 * c_begin, ctx->d_W, n, ctx->N, (int)ctx->M,
+                                         (int)ctx->local(), (int)k_begin, (int)k_end, dt.n_full, dt.nb_last,
+                                         ctx->d_S + c_begin, update ? B + c_begin : nullptr, lambda,
+                                         ctx->resid_target);
     rts_timing_end(ctx, st);
     RTS_CHECK_LAUNCH(ctx, "scatter_fp64_kernel");
     ctx->launches++;
@@ -745,7 +745,7 @@ extern "C" int rts_scattering_noalloc(const double* d_illum, const double* d_xyz
     if (cudaGetLastError() != cudaSuccess) return RTS_ERR_CUDA;  // nothing was pending: this launch's error
     const DirTiles dt = dir_tiles(M);
     dim3 grid((unsigned)gx, (unsigned)dt.gy);
-    scatter_fp64_kernel<false, false><<<grid, F64_THREADS, 0, st>>>(d_illum, W, N, (int)M, (int)M, 0, (int)M,
+    scatter_fp64_kernel<false, false><<<grid, F64_THREADS, 0, st>>>(d_illum, W, N, N, (int)M, (int)M, 0, (int)M,
                                                                      dt.n_full, dt.nb_last, d_scattering, nullptr,
                                                                      0.0, nullptr);
     if (cudaGetLastError() != cudaSuccess) return RTS_ERR_CUDA;

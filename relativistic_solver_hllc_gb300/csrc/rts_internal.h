@@ -247,6 +247,9 @@ void rts_pfree(rts_ctx* ctx, void* p, size_t bytes, cudaStream_t st);
 // Kernel launchers (defined in the .cu files).
 int rts_launch_scatter_fp64(rts_ctx* ctx, int64_t k_begin, int64_t k_end, cudaStream_t st,
                             const double* B, double lambda, bool update, bool residual);
+// ... of cells [c_begin, c_end) only.
+int rts_launch_scatter_fp64_cells(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_begin, int64_t k_end,
+                                  cudaStream_t st, const double* B, double lambda, bool update, bool residual);
 // The FP64 integral of cells [c_begin, c_end) and local out-directions
 // [k_begin, k_end) on the tensor cores (rts_sliced.cu).  *taken is false, and
 // nothing was queued, where the context's weights or size do not suit it or
@@ -363,6 +366,8 @@ int rts_split_step(rts_ctx* ctx, bool relax, cudaStream_t st);
 // the source update when B != nullptr; local out-directions [0, local).
 int rts_split_host_call(rts_ctx* ctx, int precision, const double* illum_host, const double* B_host, double lambda,
                         double* S_host);
+// The same in FP64 (rts_scattering and rts_scattering_update).
+int rts_fp64_host_call(rts_ctx* ctx, const double* illum_host, const double* B_host, double lambda, double* S_host);
 // One evaluation from the device Illum (faces) into the FP64 device S for
 // every local out-direction, no host copies (the sweep's source iteration).
 int rts_split_device_call(rts_ctx* ctx, int precision, cudaStream_t st);
