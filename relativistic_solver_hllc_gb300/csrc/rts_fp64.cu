@@ -261,42 +261,50 @@ weights_kernel(const double* __restrict__ xyz, const double* __restrict__ area, 
     }
 }
 
-// Normalises the columns of W: each divided by its sum, taken in in-direction
-// order (a serial FP64 chain per column, so that the weights do not depend on
-// the launch).  A cluster of 8 CTAs owns 32 columns: a warp of every CTA runs
-// the chain (latency bound; the next 16 rows are loaded while the current ones
-// are added), the cluster's barrier holds the divisions back until all 8 have
-// read the columns, and the divisions -- FP64-pipe bound -- spread over the
-// 8 CTAs' rows.
-constexpr int WN_CTAS = 8, WN_THREADS = 256;
+// Normalises the columns of W: each divided by its sum.  A cluster of 8 CTAs
+// owns 32 columns; a warp adds every 64th row of them (lane = column), the
+// partial sums meet in the warps' and CTAs' order through shared and cluster
+// memory, and each CTA divides its own rows -- FP64-pipe bound, like the sums
+// spread over 8 SMs (a serial chain per column took 127 us at M = 1202, this
+// 40; 61 -> 17 at M = 590).
+constexpr int WN_CTAS = 8, WN_THREADS = 256, WN_ROWS = WN_CTAS * WN_THREADS / 32;
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 __global__ void __cluster_dims__(1, WN_CTAS, 1) __launch_bounds__(WN_THREADS)
 weights_normalise_kernel(double* __restrict__ W, int M, int loc)
 {
-    __shared__ double colsum[32];
+    __shared__ double part[WN_THREADS / 32][32], ctasum[32], colsum[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int kl = blockIdx.x * 32 + lane;
+    const int kl = blockIdx.x * 32 + lane, j0 = blockIdx.y * (WN_THREADS / 32) + warp;
+    double sum = 0.0;
+    if (kl < loc)
+#pragma unroll 4
+        for (int j = j0; j < M; j += WN_ROWS) sum += W[(int64_t)j * loc + kl];
+    part[warp][lane] = sum;
+    __syncthreads();
     if (warp == 0) {
-        const double* col = W + min(kl, loc - 1);
-        constexpr int U = 16;
-        double cur[U], nxt[U], sum = 0.0;
-#pragma unroll
-        for (int i = 0; i < U; ++i) cur[i] = i < M ? col[(int64_t)i * loc] : 0.0;
-        for (int j0 = 0; j0 < M; j0 += U) {
-#pragma unroll
-            for (int i = 0; i < U; ++i) nxt[i] = j0 + U + i < M ? col[(int64_t)(j0 + U + i) * loc] : 0.0;
-#pragma unroll
-            for (int i = 0; i < U; ++i) sum += cur[i];  // + 0.0 past M
-#pragma unroll
-            for (int i = 0; i < U; ++i) cur[i] = nxt[i];
+        for (int w = 1; w < WN_THREADS / 32; ++w) sum += part[w][lane];
+        ctasum[lane] = sum;
+    }
+    cluster_sync();
+    if (warp == 0) {
+        const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&ctasum[lane]);
+        sum = 0.0;
+        for (uint32_t r = 0; r < (uint32_t)WN_CTAS; ++r) {
+            uint32_t addr;
+            double x;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(mine), "r"(r));
+            asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(x) : "r"(addr) : "memory");
+            sum += x;
         }
         colsum[lane] = sum;
     }
-    __syncthreads();
-    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    cluster_sync();  // no CTA leaves while another reads its sums; colsum is visible
     if (kl >= loc) return;
-    const double sum = colsum[lane];
-    for (int j = blockIdx.y * (WN_THREADS / 32) + warp; j < M; j += WN_CTAS * (WN_THREADS / 32))
-        W[(int64_t)j * loc + kl] /= sum;
+    sum = colsum[lane];
+    for (int j = j0; j < M; j += WN_ROWS) W[(int64_t)j * loc + kl] /= sum;
 }
 
 constexpr int MOM_THREADS = 128;

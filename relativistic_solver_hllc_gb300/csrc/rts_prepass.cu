@@ -32,17 +32,29 @@ using rts_rows::pow2_scaled_to_f32;
 
 namespace {
 
-// Block sum of one double per thread (blockDim.x a multiple of 32); every
-// thread receives the total.
+__device__ __forceinline__ double warp_sum(double x)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// Block sum of one double per thread (blockDim.x == 1024); every thread
+// receives the total.  One warp adds the warps' sums: an FP64 addition of a
+// whole block takes the SM's pipe 512 cycles.
 __device__ double block_sum(double x, double* red)
 {
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    x = warp_sum(x);
     __syncthreads();  // red may still be read from a previous call
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
     __syncthreads();
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    return t;
+    if (threadIdx.x < 32) {
+        x = warp_sum(red[threadIdx.x]);
+        __syncwarp();
+        red[threadIdx.x] = x;
+    }
+    __syncthreads();
+    return red[0];
 }
 
 // Statistics of W [Min][ldw] FP64 (column k = out-direction, Mout == Min) for
@@ -52,69 +64,44 @@ __device__ double block_sum(double x, double* red)
 //   v[kpad+1] c, the FP32 value of the mean of the v_j; v[kpad+2] D, the sum
 //   of d_j = v_j - c; v[kpad+3] 1 / c;
 // and u [Min] FP64, u_i = sum_j W[i][j] d_j: the extra row of W^T whose
-// output is sum_j d_j (W^T x)_j.  v64 [Min] FP64 scratch.  The row sums are
-// serial FP64 chains (their values do not depend on the launch), so the time
-// is one chain's latency; a warp takes 32 rows, reads them 32 columns at a
-// time in coalesced 256-byte pieces -- the next piece while the current one
-// is added -- and turns them through shared memory.  One block that walked
-// the rows thread by thread (the former layout: a 32-byte sector per value,
-// one SM) took 1,173 us at M = 1000 against 239 us for the three launches.
-constexpr int WS_T = 32;
-
-// Row sums of f(W[j][k], k) over k in order for rows [32 b, 32 b + 32): lane
-// l of the block's one warp returns row 32 b + l's.  Add(k, w) is called for
-// every k in order on the owner's lane.
-template <class Add>
-__device__ __forceinline__ void row_chain(const double* __restrict__ W, int rows, int cols, int ldw, Add add)
-{
-    __shared__ double tile[WS_T][WS_T + 1];
-    const int lane = threadIdx.x, j0 = blockIdx.x * WS_T;
-    double nxt[WS_T];
-    auto load = [&](int k0) {
-        const int k = k0 + lane;
-#pragma unroll
-        for (int r = 0; r < WS_T; ++r)
-            nxt[r] = (j0 + r < rows && k < cols) ? __ldg(W + (int64_t)(j0 + r) * ldw + k) : 0.0;
-    };
-    load(0);
-    for (int k0 = 0; k0 < cols; k0 += WS_T) {
-#pragma unroll
-        for (int r = 0; r < WS_T; ++r) tile[r][lane] = nxt[r];
-        __syncwarp();
-        if (k0 + WS_T < cols) load(k0 + WS_T);
-        const int n = min(WS_T, cols - k0);
-        if (n == WS_T) {
-#pragma unroll
-            for (int i = 0; i < WS_T; ++i) add(k0 + i, tile[lane][i]);
-        } else {
-            for (int i = 0; i < n; ++i) add(k0 + i, tile[lane][i]);
-        }
-        __syncwarp();
-    }
-}
+// output is sum_j d_j (W^T x)_j.  v64 [Min] FP64 scratch.  A warp takes a row
+// (coalesced reads, lane sums added in a fixed tree), so the two passes over W
+// run at the FP64 pipe's rate over the whole device: serial chains over the
+// columns, 32 rows a warp, took 278 us at M = 1202 and 159 at M = 590, this 37
+// and 30; a block that walked all rows thread by thread (a 32-byte sector per
+// value, one SM) 1,173 us at M = 1000.
+constexpr int WS_WARPS = 8;
 
 // v, v64 and (in u, until w_stats_u_kernel writes it) the rows' sums of |W|.
-__global__ void __launch_bounds__(WS_T) w_stats_rows_kernel(const double* __restrict__ W, int Min, int Mout, int ldw,
-                                                            int kpad, float* __restrict__ v, double* __restrict__ v64,
-                                                            double* __restrict__ u)
+__global__ void __launch_bounds__(32 * WS_WARPS)
+w_stats_rows_kernel(const double* __restrict__ W, int Min, int Mout, int ldw, int kpad, float* __restrict__ v,
+                    double* __restrict__ v64, double* __restrict__ u)
 {
-    const int j = blockIdx.x * WS_T + threadIdx.x;
+    const int lane = threadIdx.x & 31, j = blockIdx.x * WS_WARPS + (threadIdx.x >> 5);
+    if (j >= kpad) return;
     double s = 0.0, a = 0.0;
-    row_chain(W, Min, Mout, ldw, [&](int, double w) {
-        s += w;
-        a += fabs(w);
-    });
     if (j < Min) {
-        v64[j] = s;
-        u[j] = a;
+#pragma unroll 4
+        for (int k = lane; k < Mout; k += 32) {
+            const double w = __ldg(W + (int64_t)j * ldw + k);
+            s += w;
+            a += fabs(w);
+        }
     }
-    if (j < kpad) v[j] = j < Min ? (float)s : 0.0f;
+    s = warp_sum(s);
+    a = warp_sum(a);
+    if (lane == 0) {
+        v[j] = j < Min ? (float)s : 0.0f;
+        if (j < Min) {
+            v64[j] = s;
+            u[j] = a;
+        }
+    }
 }
 
-// The sums over the rows, one block.
+// The sums over the rows, one block; v64 becomes the d_j.
 __global__ void __launch_bounds__(1024) w_stats_reduce_kernel(int Min, int kpad, float* __restrict__ v,
-                                                              const double* __restrict__ v64,
-                                                              const double* __restrict__ u)
+                                                              double* __restrict__ v64, const double* __restrict__ u)
 {
     __shared__ double red[32];
     double a = 0.0, sv = 0.0;
@@ -126,7 +113,11 @@ __global__ void __launch_bounds__(1024) w_stats_reduce_kernel(int Min, int kpad,
     sv = block_sum(sv, red);
     const float c = Min > 0 ? (float)(sv / Min) : 0.0f;
     double ds = 0.0;
-    for (int i = threadIdx.x; i < Min; i += blockDim.x) ds += v64[i] - (double)c;
+    for (int i = threadIdx.x; i < Min; i += blockDim.x) {
+        const double d = v64[i] - (double)c;
+        v64[i] = d;
+        ds += d;
+    }
     ds = block_sum(ds, red);
     if (threadIdx.x == 0) {
         float q = 0.0f;
@@ -141,31 +132,34 @@ __global__ void __launch_bounds__(1024) w_stats_reduce_kernel(int Min, int kpad,
     }
 }
 
-__global__ void __launch_bounds__(WS_T) w_stats_u_kernel(const double* __restrict__ W, int Min, int Mout, int ldw,
-                                                         int kpad, const float* __restrict__ v,
-                                                         const double* __restrict__ v64, double* __restrict__ u)
+__global__ void __launch_bounds__(32 * WS_WARPS)
+w_stats_u_kernel(const double* __restrict__ W, int Min, int Mout, int ldw, const double* __restrict__ d64,
+                 double* __restrict__ u)
 {
-    const int i = blockIdx.x * WS_T + threadIdx.x;
-    const double c = (double)v[kpad + 1];
+    const int lane = threadIdx.x & 31, i = blockIdx.x * WS_WARPS + (threadIdx.x >> 5);
+    if (i >= Min) return;
     double s = 0.0;
-    row_chain(W, Min, Mout, ldw, [&](int j, double w) { s += w * (__ldg(v64 + j) - c); });
-    if (i < Min) u[i] = s;
+#pragma unroll 4
+    for (int j = lane; j < Mout; j += 32) s += __ldg(W + (int64_t)i * ldw + j) * __ldg(d64 + j);
+    s = warp_sum(s);
+    if (lane == 0) u[i] = s;
 }
 
 // W [Min][ldw] FP64 (column k = out-direction) -> Wc [mpad][2*kpad] split
 // W^T rows; with `extra`, row Mout holds extra [Min] (the correction's row).
 // A block takes 32 out-directions: its warps read 256-byte pieces of W's rows
-// (lane = out-direction) for the columns' maxima, then each takes every 8th
-// group of 32 in-directions, whose split parts are 128 contiguous bytes of a
-// lane's own row (256 for TF32).  A thread per out-direction over all
-// in-directions (the former layout) wrote 2 bytes at a time: 455 -> 42 us at
-// M = 1000.
+// (lane = out-direction) for the columns' maxima, then each takes some of the
+// groups of 32 in-directions, whose split parts are 128 contiguous bytes of a
+// lane's own row (256 for TF32).  The split is exact arithmetic on the bits, on
+// the integer pipe.  M = 590: 16 us; 31 with FP64 operations and one block per
+// 32 columns; 219 with a thread per out-direction, writing 2 bytes at a time.
 constexpr int SW_THREADS = 256, SW_WARPS = SW_THREADS / 32;
+constexpr int SW_Y = 4;  // blocks per 32 out-directions: each takes the maxima, and a quarter of the groups
 __global__ void __launch_bounds__(SW_THREADS)
 split_w_kernel(const double* __restrict__ W, int Min, int Mout, int ldw, int kpad, int mpad, int mode,
                uint16_t* __restrict__ Wc, float* __restrict__ cs, const double* __restrict__ extra)
 {
-    __shared__ double smax[SW_WARPS][32];
+    __shared__ unsigned long long smax[SW_WARPS][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int k = blockIdx.x * 32 + lane;
     // element j of this row: column k of W, or the extra row; zero past both
@@ -175,22 +169,29 @@ split_w_kernel(const double* __restrict__ W, int Min, int Mout, int ldw, int kpa
     const int64_t step = ex ? 1 : ldw;
     float s = 1.0f;
     if (mode == 1) {
-        double m = 0.0;
+        // |W| orders as its bits; NaN is skipped
+        unsigned long long m = 0;
         if (real)
-            for (int j = warp; j < Min; j += SW_WARPS) m = fmax(m, fabs(col[j * step]));
+#pragma unroll 8
+            for (int j = warp; j < Min; j += SW_WARPS) {
+                const unsigned long long w =
+                    (unsigned long long)__double_as_longlong(col[j * step]) & 0x7FFFFFFFFFFFFFFFull;
+                if (w <= 0x7FF0000000000000ull && w > m) m = w;
+            }
         smax[warp][lane] = m;
         __syncthreads();
 #pragma unroll
-        for (int w = 0; w < SW_WARPS; ++w) m = fmax(m, smax[w][lane]);
-        if (real) s = pow2_scale(m);
+        for (int w = 0; w < SW_WARPS; ++w) m = smax[w][lane] > m ? smax[w][lane] : m;
+        if (real) s = pow2_scale(__longlong_as_double((long long)m));
     }
     if (k >= mpad) return;
-    if (warp == 0) {
+    if (warp == 0 && blockIdx.y == 0) {
         cs[k] = s;
         cs[mpad + k] = 1.0f / s;
     }
+    const int ks = rts_rows::scale_log2(s);
     uint16_t* row = Wc + (int64_t)k * (mode == 2 ? 4 : 2) * kpad;
-    for (int j0 = warp * 32; j0 < kpad; j0 += SW_WARPS * 32) {
+    for (int j0 = (blockIdx.y * SW_WARPS + warp) * 32; j0 < kpad; j0 += SW_Y * SW_WARPS * 32) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) {  // 8 in-directions at a time
             double x[8];
@@ -202,7 +203,7 @@ split_w_kernel(const double* __restrict__ W, int Min, int Mout, int ldw, int kpa
             if (mode == 2) {
                 float hi[8], lo[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) split_tf32((float)x[i], hi[i], lo[i]);
+                for (int i = 0; i < 8; ++i) split_tf32(pow2_scaled_to_f32(x[i], 0), hi[i], lo[i]);
                 float4* d = reinterpret_cast<float4*>(reinterpret_cast<float*>(row) + ilv_hi_tf32(j0 + 8 * q));
                 d[0] = make_float4(hi[0], hi[1], hi[2], hi[3]);
                 d[1] = make_float4(hi[4], hi[5], hi[6], hi[7]);
@@ -211,7 +212,7 @@ split_w_kernel(const double* __restrict__ W, int Min, int Mout, int ldw, int kpa
             } else {
                 uint16_t hi[8], lo[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) split_any(mode == 1, (float)(x[i] * (double)s), hi[i], lo[i]);
+                for (int i = 0; i < 8; ++i) split_any(mode == 1, pow2_scaled_to_f32(x[i], ks), hi[i], lo[i]);
                 uint4* d = reinterpret_cast<uint4*>(row + ilv_hi(j0 + 8 * q));
                 d[0] = make_uint4(pack2(hi[0], hi[1]), pack2(hi[2], hi[3]), pack2(hi[4], hi[5]), pack2(hi[6], hi[7]));
                 d[4] = make_uint4(pack2(lo[0], lo[1]), pack2(lo[2], lo[3]), pack2(lo[4], lo[5]), pack2(lo[6], lo[7]));
@@ -497,10 +498,10 @@ int blocks_for(rts_ctx* ctx, int64_t n, int threads)
 int rts_pp_w_stats(rts_ctx* ctx, const double* W, int Min, int Mout, int ldw, int kpad, float* v, double* v64,
                    double* u, cudaStream_t st)
 {
-    const unsigned blocks = (unsigned)((kpad + WS_T - 1) / WS_T);
-    w_stats_rows_kernel<<<blocks, WS_T, 0, st>>>(W, Min, Mout, ldw, kpad, v, v64, u);
+    const unsigned blocks = (unsigned)((kpad + WS_WARPS - 1) / WS_WARPS);
+    w_stats_rows_kernel<<<blocks, 32 * WS_WARPS, 0, st>>>(W, Min, Mout, ldw, kpad, v, v64, u);
     w_stats_reduce_kernel<<<1, 1024, 0, st>>>(Min, kpad, v, v64, u);
-    w_stats_u_kernel<<<blocks, WS_T, 0, st>>>(W, Min, Mout, ldw, kpad, v, v64, u);
+    w_stats_u_kernel<<<blocks, 32 * WS_WARPS, 0, st>>>(W, Min, Mout, ldw, v64, u);
     RTS_CHECK_LAUNCH(ctx, "w_stats kernels");
     ctx->launches += 3;
     return RTS_OK;
@@ -509,7 +510,8 @@ int rts_pp_w_stats(rts_ctx* ctx, const double* W, int Min, int Mout, int ldw, in
 int rts_pp_split_w(rts_ctx* ctx, const double* W, int Min, int Mout, int ldw, int kpad, int mpad, int mode,
                    uint16_t* Wc, float* cs, cudaStream_t st, const double* extra)
 {
-    split_w_kernel<<<(mpad + 31) / 32, SW_THREADS, 0, st>>>(W, Min, Mout, ldw, kpad, mpad, mode, Wc, cs, extra);
+    split_w_kernel<<<dim3((unsigned)((mpad + 31) / 32), SW_Y), SW_THREADS, 0, st>>>(W, Min, Mout, ldw, kpad, mpad, mode,
+                                                                                   Wc, cs, extra);
     RTS_CHECK_LAUNCH(ctx, "split_w_kernel");
     ctx->launches++;
     return RTS_OK;
