@@ -185,6 +185,83 @@ scatter_fp64_kernel(const double* __restrict__ illum, const double* __restrict__
     }
 }
 
+// Tiles of 32 cells x 32 out-directions for problems whose 128 x 64 tiles would
+// leave SMs idle: 2,000 x 64 makes 16 of those, each a serial loop of loads,
+// barriers and FMAs (152 us), and 126 of these (23 us).  A chunk's operands are
+// loaded while the previous one is multiplied, one barrier a chunk.  Every output
+// is the same FMA chain as in the larger tiles.
+constexpr int S64_T = 32, S64_KC = 16, S64_THREADS = 256;
+template <bool kUpdate>
+__global__ void __launch_bounds__(S64_THREADS)
+scatter_fp64_small_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t n, int64_t N, int M,
+                          int ldw, int k_begin, int k_end, double* __restrict__ S, const double* __restrict__ B,
+                          double lambda, unsigned long long* __restrict__ resid)
+{
+    __shared__ double sI[2][S64_KC][S64_T], sW[2][S64_KC][S64_T];
+    constexpr int PER = S64_KC * S64_T / S64_THREADS;  // pairs of a chunk per thread: 2
+    const int tx = threadIdx.x & (S64_T - 1), ty = threadIdx.x / S64_T;
+    const int64_t c = (int64_t)blockIdx.x * S64_T + tx;
+    const int k0 = k_begin + (int)blockIdx.y * S64_T;
+    double2 p[PER], q[PER];
+    double w[PER];
+    auto load = [&](int j0) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int j = j0 + ty + (S64_THREADS / S64_T) * i;
+            p[i] = q[i] = make_double2(0.0, 0.0);
+            if (j < M && c < n) {
+                const double2* src = reinterpret_cast<const double2*>(illum + ((int64_t)j * N + c) * 4);
+                p[i] = __ldg(src);
+                q[i] = __ldg(src + 1);
+            }
+            w[i] = (j < M && k0 + tx < k_end) ? __ldg(W + (int64_t)j * ldw + k0 + tx) : 0.0;
+        }
+    };
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    load(0);
+    int b = 0;
+    for (int j0 = 0; j0 < M; j0 += S64_KC, b ^= 1) {
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int jj = ty + (S64_THREADS / S64_T) * i;
+            double I = 0.0;  // faces 0..3 in order, then /4 (GET_FACE_TO_CELL)
+            I += p[i].x;
+            I += p[i].y;
+            I += q[i].x;
+            I += q[i].y;
+            sI[b][jj][tx] = I / 4;
+            sW[b][jj][tx] = w[i];
+        }
+        __syncthreads();
+        if (j0 + S64_KC < M) load(j0 + S64_KC);
+        const int nj = min(S64_KC, M - j0);
+        if (nj == S64_KC) {
+#pragma unroll
+            for (int jj = 0; jj < S64_KC; ++jj)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) acc[m] = fma(sW[b][jj][ty + 8 * m], sI[b][jj][tx], acc[m]);
+        } else {
+            for (int jj = 0; jj < nj; ++jj)
+#pragma unroll
+                for (int m = 0; m < 4; ++m) acc[m] = fma(sW[b][jj][ty + 8 * m], sI[b][jj][tx], acc[m]);
+        }
+    }
+    double rmax = 0.0;
+    if (c < n) {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const int k = k0 + ty + 8 * m;
+            if (k >= k_end) continue;
+            double v = acc[m];
+            if (kUpdate) v = (1.0 - lambda) * B[c] + lambda * v;
+            double* dst = S + (int64_t)k * N + c;
+            if (resid) rmax = fmax(rmax, fabs(v - *dst));
+            *dst = v;
+        }
+    }
+    if (resid) residual_max(resid, rmax);
+}
+
 // The outputs that the tensor-core route left (rts_launch_scatter_list): a few
 // CTAs walk the tiles of the listed cells; count and list are the device's, so
 // nothing waits on the host.  Usually there are none and the launch costs its
@@ -220,6 +297,14 @@ inline DirTiles dir_tiles(int64_t width)
     t.nb_last = rem ? (rem + 15) / 16 : 4;
     t.gy = t.n_full + (rem ? 1 : 0);
     return t;
+}
+
+// Which of the two kernels: the larger tiles need four a SM (two resident at a
+// time, two waves) to keep the FP64 pipe busy to the end.
+inline bool small_tiles(int64_t gx, const DirTiles& dt, int num_sms) { return gx * dt.gy < 4 * num_sms; }
+inline dim3 small_grid(int64_t n, int64_t width)
+{
+    return dim3((unsigned)((n + S64_T - 1) / S64_T), (unsigned)((width + S64_T - 1) / S64_T));
 }
 
 __device__ __forceinline__ double gamma_thomson(double ax, double ay, double az, double bx,
@@ -265,8 +350,8 @@ weights_kernel(const double* __restrict__ xyz, const double* __restrict__ area, 
 // owns 32 columns; a warp adds every 64th row of them (lane = column), the
 // partial sums meet in the warps' and CTAs' order through shared and cluster
 // memory, and each CTA divides its own rows -- FP64-pipe bound, like the sums
-// spread over 8 SMs (a serial chain per column took 127 us at M = 1202, this
-// 40; 61 -> 17 at M = 590).
+// spread over 8 SMs (a serial chain per column took 127 us at M = 1202 and 61 at
+// M = 590, this 40 and 17).
 constexpr int WN_CTAS = 8, WN_THREADS = 256, WN_ROWS = WN_CTAS * WN_THREADS / 32;
 __device__ __forceinline__ void cluster_sync()
 {
@@ -565,6 +650,17 @@ int rts_launch_scatter_fp64_cells(rts_ctx* ctx, int64_t c_begin, int64_t c_end, 
     const DirTiles dt = dir_tiles(k_end - k_begin);
     RTS_REQUIRE(ctx, gx < (1ll << 31) && dt.gy < 65536, RTS_ERR_UNSUPPORTED, "FP64 grid too large");
     dim3 grid((unsigned)gx, (unsigned)dt.gy);
+    if (small_tiles(gx, dt, ctx->num_sms)) {
+        auto* kernel = update ? scatter_fp64_small_kernel<true> : scatter_fp64_small_kernel<false>;
+        rts_timing_begin(ctx, st);
+        kernel<<<small_grid(n, k_end - k_begin), S64_THREADS, 0, st>>>(
+            ctx->d_illum + 4 * c_begin, ctx->d_W, n, ctx->N, (int)ctx->M, (int)ctx->local(), (int)k_begin, (int)k_end,
+            ctx->d_S + c_begin, update ? B + c_begin : nullptr, lambda, residual ? ctx->resid_target : nullptr);
+        rts_timing_end(ctx, st);
+        RTS_CHECK_LAUNCH(ctx, "scatter_fp64_small_kernel");
+        ctx->launches++;
+        return RTS_OK;
+    }
     auto* kernel = update && residual ? scatter_fp64_kernel<true, true>
                    : update           ? scatter_fp64_kernel<true, false>
                                       : scatter_fp64_kernel<false, false>;
@@ -746,12 +842,22 @@ extern "C" int rts_scattering_noalloc(const double* d_illum, const double* d_xyz
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     double* W = noalloc_scratch(device, st);
     if (!W) return RTS_ERR_CUDA;
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        cudaGetLastError();
+        return RTS_ERR_CUDA;
+    }
     // W is rewritten in full (all M x M entries) by every call: nothing in the
     // scratch has to start at zero, and calls that overlap on the GPU race.
     weights_kernel<<<weights_grid((int)M, (int)M), WE_K * WE_J, 0, st>>>(d_xyz, d_area, (int)M, 0, (int)M, full_area,
                                                                          RTS_PHASE_THOMSON, 0.0, W);
     if (cudaGetLastError() != cudaSuccess) return RTS_ERR_CUDA;  // nothing was pending: this launch's error
     const DirTiles dt = dir_tiles(M);
+    if (small_tiles(gx, dt, sms)) {
+        scatter_fp64_small_kernel<false><<<small_grid(N, M), S64_THREADS, 0, st>>>(
+            d_illum, W, N, N, (int)M, (int)M, 0, (int)M, d_scattering, nullptr, 0.0, nullptr);
+        return cudaGetLastError() != cudaSuccess ? RTS_ERR_CUDA : RTS_OK;
+    }
     dim3 grid((unsigned)gx, (unsigned)dt.gy);
     scatter_fp64_kernel<false, false><<<grid, F64_THREADS, 0, st>>>(d_illum, W, N, N, (int)M, (int)M, 0, (int)M,
                                                                      dt.n_full, dt.nb_last, d_scattering, nullptr,

@@ -25,12 +25,13 @@
 // 2^(e_c + e_k) in all (rms), against about sqrt(M) 2^-55 of S for the FP64 FMA
 // chain of scatter_fp64_kernel (measured against 113-bit sums, lognormal
 // intensities: 1.0e-16 against 8.6e-16 rms at M = 1000, 7.5e-17 against
-// 3.8e-16 at M = 200, 7.6e-17 against 2.1e-16 at M = 64).  An output below half of 2^(e_c + e_k) (a row
-// dominated by a few directions far above the rest) could be further off than
-// the chain: it is left to that kernel, as are rows with negative values,
-// infinities, NaN or exponents out of range -- the outputs are marked here and
-// rts_launch_scatter_list computes them from the Illum.  So every output is at
-// least as accurate as the chain's, for any input.
+// 3.8e-16 at M = 200, 7.6e-17 against 2.1e-16 at M = 64).  An output below half
+// of 2^(e_c + e_k) (a row dominated by a few directions far above the rest)
+// could be further off than the chain: it is left to that kernel, as are rows
+// with negative values, infinities, NaN or exponents out of range -- the
+// outputs are marked here and rts_launch_scatter_list computes them from the
+// Illum.  So every output is at least as accurate as the chain's, for any
+// input.
 //
 // Kernel: persistent CTAs (one per SM) on tiles of 128 cells x up to 128
 // out-directions.  Warp 0 brings the digits of 32 in-directions of both
@@ -561,16 +562,20 @@ constexpr int64_t S_ROWS_BYTES = (int64_t)1 << 31;
 // of cells and out-directions of a context takes the same route and rows
 // covered by two calls agree bit for bit.
 //
-// The size limit: the digit rows, the contraction and the list pass cost about
-// 37 us at the smallest sizes (5,000 x 64, 6,000 x 48) where
-// scatter_fp64_kernel took 161 and 98.
+// The size limit.  The digit rows, the contraction and the list pass take about
+// 22 us + 0.14 us M at the smallest sizes, whatever the cells; the 32 x 32 tiles
+// of scatter_fp64_small_kernel 0.31 us M in one wave of tiles, then by the
+// products.  Digits against tiles: 2,000 x 64 31 and 27 us, 1,000 x 100 44 and
+// 39, 1,200 x 128 49 and 47; 3,000 x 64 33 and 47, 2,000 x 100 45 and 70; and
+// where M is large even for few cells: 300 x 200 55 and 70, 100 x 302 64 and
+// 100, 40 x 1,000 156 and 313.
 static bool sliced_fits(const rts_ctx* ctx)
 {
     if (ctx->cc_major != 10) return false;
     const int64_t N = ctx->N, M = ctx->M;
     size_t smem = 0;
     if (M < 48 || N >= ((int64_t)1 << 31) || rts_rows::cells_log2((int)kpad_of(ctx), &smem) == 0) return false;
-    if ((double)N * (double)M * (double)ctx->local() < 1.0e7) return false;
+    if (M < 160 && (double)N * (double)M * (double)ctx->local() < 1.0e7) return false;
     double peak;
     if (ctx->phase == RTS_PHASE_THOMSON)
         peak = 1.5;
