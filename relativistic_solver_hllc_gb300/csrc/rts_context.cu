@@ -39,6 +39,11 @@ int rts_dmalloc(rts_ctx* ctx, void** p, size_t bytes, const char* what)
                         "%s: %zu bytes would exceed the HBM budget (%lld of %lld bytes in use)",
                         what, bytes, (long long)ctx->used_bytes, (long long)ctx->budget_bytes);
     cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->pool) {  // what the scratch pool holds unused goes back first
+        cudaGetLastError();
+        cudaMemPoolTrimTo(ctx->pool, 0);
+        e = cudaMalloc(p, bytes);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
