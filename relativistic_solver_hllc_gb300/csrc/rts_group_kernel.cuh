@@ -719,12 +719,14 @@ __global__ void group_energy_kernel(const GroupProblem* __restrict__ probs, int 
 
 // x as FP64, from the bits on the integer pipe (the conversion instruction
 // runs on the FP64 pipe, at two per SM per cycle); zeros, subnormals and
-// non-finite values take the instruction.
+// non-finite values take the instruction, out of line: predicated into the
+// loop it would hold the FP64 pipe without doing anything.
+__device__ __noinline__ double f32_to_f64_cvt(float x) { return (double)x; }
 __device__ __forceinline__ double f32_to_f64_bits(float x)
 {
     const uint32_t u = __float_as_uint(x);
     const uint32_t e = u & 0x7F800000u;
-    if (e == 0u || e == 0x7F800000u) return (double)x;
+    if (e == 0u || e == 0x7F800000u) return f32_to_f64_cvt(x);
     return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(u << 29));
 }
 
