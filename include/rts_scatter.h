@@ -627,10 +627,10 @@ int rts_illum_solve(rts_ctx* ctx, int precision, int max_iter, double accuracy, 
 #define RTS_TUNE_SERVE_BUDGET 4
 #define RTS_TUNE_SERVE_SLACK 5
 /*   RTS_TUNE_SWEEP_CACHE: 1 (default) the first rts_sweep after a change of
- *   the medium or of the structures stores every node's attenuation factor
- *   exp(-k s) (8 bytes per node record, allocated then; within budget), and
- *   the sweeps after it read the factor instead of evaluating it -- the same
- *   numbers, without the exponential; 0 every sweep evaluates them (and the
+ *   the medium or of the structures stores every out-face's attenuation
+ *   factors (32 bytes per out-face, its three node records; allocated then;
+ *   within budget), and the sweeps after it read them instead of evaluating
+ *   the exponentials -- the same numbers; 0 every sweep evaluates them (and the
  *   factors are not allocated).  A sweep that cannot allocate the factors
  *   evaluates them. */
 #define RTS_TUNE_SWEEP_CACHE 6
@@ -689,8 +689,8 @@ int rts_autotune_load(rts_ctx* ctx, const char* path);
  * or record CUDA events against the library's streams). */
 int rts_stream_handle(rts_ctx* ctx, int stream, void** handle);
 
-/* Self-check of the sweep's FP64 exponential (a table-driven method for
- * arguments in [-700, 0]) against CUDA's exp at n points of that range:
+/* Self-check of the sweep's exponential (a table-driven method for arguments
+ * in [-700, -1e-3]) against CUDA's exp at n points of that range:
  * *max_ulp receives the largest difference in units in the last place. */
 int rts_sweep_exp_check(rts_ctx* ctx, int64_t n, double* max_ulp);
 

@@ -116,7 +116,8 @@ struct rts_sliced_state {
 // per-direction structures of the local directions and the medium.  The unit
 // of work is an out-face of a cell (its 3 nodes); per local direction d:
 //   items[d]  out-faces in dependency order: cell << 8 | face << 6 | the
-//             in-faces of its 3 nodes (2 bits each)
+//             in-faces of its 3 nodes (2 bits each); behind them, with
+//             copy_words, a word per item on the neighbour's copy of its face
 //   recs[d]   3 node distances per item (the LocX0 records' s, same order)
 //   steps[d]  item offsets of the dependency steps (nsteps[d] + 1 entries)
 //   bnd[d]    boundary in-faces, cell * 4 + face (nbnd[d] of them)
@@ -128,6 +129,7 @@ struct rts_sweep_state {
     int32_t* d_pairs = nullptr;      // [N][4]
     double* d_normals = nullptr;     // [N][4][3]
     double* d_nodes = nullptr;       // [N][4][3][3] (MakeArrayX)
+    bool copy_words = true;          // behind every direction's items (false: no room for some)
     uint32_t** d_items = nullptr;    // device pointer tables [D]
     double** d_recs = nullptr;
     int32_t** d_steps = nullptr;
@@ -144,10 +146,10 @@ struct rts_sweep_state {
     std::vector<char> have;          // direction d built or imported
     double** d_att = nullptr;        // device pointer table [D] of the attenuation factors
     std::vector<double*> h_att;
-    double* att_blk = nullptr;       // one factor per node record (exp(-k s), or a negative mark)
+    double* att_blk = nullptr;       // per item its nodes' exp(-k s) / 3 (or negative marks) and the source's weight
     size_t att_bytes = 0;
     bool att_valid = false;          // stored by a sweep since the last change of medium or structures
-    double* d_med = nullptr;         // [N][4] k, beta, Q, 1/k (k = alpha + beta, or alpha)
+    double* d_med = nullptr;         // [N][4] beta, Q, k, 1/k (k = alpha + beta, or alpha)
     rts_medium md{};
     double bc[4] = {0.0, 0.0, 1.0, 0.0};
     bool has_medium = false;

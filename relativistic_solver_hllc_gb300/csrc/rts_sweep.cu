@@ -35,12 +35,8 @@ void rts_sweep_nodes_host(int64_t N, const double* vert, double* nodes);
 
 namespace {
 
-// 128 threads and at most 72 registers: 7 CTAs per SM, so one wave of 152 x 7
-// CTAs holds 1000 directions (the sweep is bound by the FP64 pipe; a second
-// partial wave cost 11 %).
-constexpr int SWEEP_THREADS = 128;
 constexpr double SWEEP_EPS = 1e-10;  // `eps`, global_value.h:13
-constexpr int kExpTable = 256;       // entries 2^(j/256) of the sweep's exponential (exp_neg)
+constexpr int kExpTable = 256;       // entries of the sweep's exponential (exp_fixed)
 
 __host__ __device__ inline void face_verts(int f, int& a, int& b, int& c)
 {
@@ -131,19 +127,41 @@ __device__ inline bool hits_face(const double* __restrict__ F, const double* A, 
     return (r1 < 0 && r2 < 0 && r3 < 0) || (r1 > 0 && r2 > 0 && r3 > 0);
 }
 
+// The word beside an item: the neighbour's copy of its face (its index in a
+// direction's Illum, below 2^26), and in the top bits
+//   kNoCopy     a boundary face, nothing to copy to;
+//   kBoundCell  the cell has a boundary face;
+//   kSharedOut  the face is an out-face of the neighbour too (the direction lies
+//               in its plane), so another item writes the same two values.
+constexpr uint32_t kNoCopy = 0x80000000u, kBoundCell = 0x40000000u, kSharedOut = 0x20000000u;
+constexpr uint32_t kCopyIndex = 0x03FFFFFFu;
+
+// pairs: all cells'; states: the direction's in-face flags (null: every face
+// counts as shared, which is slower and always right).
+__host__ __device__ inline uint32_t copy_word(const int32_t* pairs, const uint8_t* states, uint32_t w)
+{
+    const int32_t* p = pairs + 4 * (int64_t)(w >> 8);
+    const int32_t nb = p[(w >> 6) & 3u];
+    uint32_t x = (p[0] | p[1] | p[2] | p[3]) < 0 ? kBoundCell : 0u;
+    if (nb < 0) return x | kNoCopy;
+    if (!states || !((states[nb >> 2] >> (nb & 3)) & 1)) x |= kSharedOut;
+    return x | (uint32_t)nb;
+}
+
 struct X0Args {
     const double* vert;      // [N][4][3]
     const double* frames;    // [N][4][kFrame]
     const double* nodes;     // [N][4][3][3]
+    const int32_t* pairs;    // [N][4]
     const double* dirs;      // [D][3]
     const uint8_t* states;   // [D][N] in-face flags
     uint32_t* const* items;  // [D]
     double* const* recs;     // [D]
-    double* const* att;      // [D] attenuation factors, parallel to recs (stored or read by the cached forms)
     int32_t* const* steps;   // [D]
     const int32_t* nsteps;   // [D]
     int64_t N;
     int64_t d0;              // first direction of this launch (grid y covers at most 65535)
+    bool words;              // the items are followed by their copy words
     int* flag;               // set when a node finds no in-face
 };
 
@@ -188,6 +206,7 @@ __global__ void __launch_bounds__(256) sweep_x0_kernel(X0Args a)
             w |= (uint32_t)found << (2 * m);
         }
         items[i] = w;
+        if (a.words) items[n + i] = copy_word(a.pairs, a.states + d * a.N, w);
     }
 }
 
@@ -196,82 +215,94 @@ __global__ void __launch_bounds__(256) sweep_x0_kernel(X0Args a)
 struct SweepArgs {
     uint32_t* const* items;  // [D]
     double* const* recs;     // [D]
-    double* const* att;      // [D] attenuation factors, parallel to recs (stored or read by the cached forms)
+    double* const* att;      // [D] 4 factors per item (stored or read by the cached forms)
     int32_t* const* steps;   // [D]
     uint32_t* const* bnd;    // [D]
     const int32_t* nsteps;   // [D]
     const int32_t* nbnd;     // [D]
     const int32_t* pairs;    // [N][4]
     const double* nodes;     // [N][4][3][3] (read only with a ball)
-    const double* med;       // [N][4] k, beta, Q, 1/k
+    const double* med;       // [N][4] beta, Q, k, 1/k
     const double* S;         // [D][N]
     double* illum;           // [D][N][4], rows of the local directions
     int64_t N;
+    bool words;              // copy words behind the items
     rts_medium md;
     double bc[4];
-    double exp2tab[kExpTable];  // 2^(j/256)
+    uint64_t exptab[kExpTable];  // 2^(-j/256) / 3, times 2^65
     double ball[4];          // medium table entry of the ball's coefficients
     unsigned long long* norm;
 };
 
-// exp(x) for -700 <= x <= 0 by Tang's table-driven method (P. T. P. Tang,
-// "Table-driven implementation of the exponential function in IEEE
-// floating-point arithmetic", ACM TOMS 15(2), 1989): x = (256 m + j) ln2/256
-// + r with |r| <= ln2/512, exp(x) = 2^m 2^(j/256) (1 + p(r)), 2^(j/256) from
-// a 256-entry table and 2^m added to the exponent field.  p(r) = r + r^2 h(r)
-// with h the quadratic fitted to (exp(r) - 1 - r) / r^2 on that interval by
-// weighted least squares at Chebyshev nodes (relative error of 1 + p below
-// 5.1e-18, against 1.1e-16 for one ulp).  9 FP64 operations against the
-// general exp's range checks and longer polynomial; within 1.03 ulp of the
-// exact value over the range (checked against CUDA's exp by
-// rts_sweep_exp_check).
-constexpr double kExpInvL = 369.3299304675746;            // 256 / ln 2
-constexpr double kExpLHi = 0.0027076061740622863;         // ln 2 / 256, leading part
-constexpr double kExpLLo = 9.058776616587108e-20;         // ln 2 / 256 - kExpLHi
-constexpr double kExpShift = 6755399441055744.0;          // 1.5 * 2^52: rounds to an integer
-constexpr double kExpH0 = 0.49999999999999795, kExpH1 = 0.16666668003070842, kExpH2 = 0.04166667023041113;
+// exp(-x) for x in [1e-3, 700] in 64-bit fixed point.  GB300 retires two FP64
+// operations per SM and cycle against 64 or more 32-bit integer ones, so the
+// dozen 32 x 32 multiplies and the shifts and adds below cost a fraction of
+// Tang's FP64 form (P. T. P. Tang, "Table-driven implementation of the
+// exponential function in IEEE floating-point arithmetic", ACM TOMS 15(2),
+// 1989), whose reduction they keep: x = (256 k + j) ln2/256 + u with |u| <=
+// ln2/512, exp(-x) = 2^-k 2^(-j/256) exp(-u), 2^(-j/256) from a 256-entry table
+// and exp(-u) = 1 - u + u^2/2 - u^3/6 + u^4/24 - u^5/120 (the next term is below
+// 2^-60), each power with as many bits as its size asks for.  Within 0.65 units
+// in the last place of the exact value over the range (0.5 is the rounding's).
+//
+// `tab` holds 2^(-j/256) times a factor, times 2^65 as integers in [2^62, 2^64);
+// the result carries the factor.
+constexpr uint64_t kExpC = 0xB8AA3B295C17F0BBull;  // 256 / ln 2 = (kExpC + kExpC2 / 2^32) / 2^55
+constexpr uint32_t kExpC2 = 0xBE87FED0u;
+constexpr uint64_t kLn2 = 0xB17217F7D1CF79ACull;   // ln 2 * 2^64
 
-__device__ __forceinline__ double exp_neg(double x, const double* __restrict__ tab)
+__device__ __forceinline__ double exp_fixed(double x, const uint64_t* __restrict__ tab)
 {
-    const double t = fma(x, kExpInvL, kExpShift);
-    const int n = __double2loint(t);
-    const double N = t - kExpShift;
-    double r = fma(-N, kExpLHi, x);
-    r = fma(-N, kExpLLo, r);
-    const double h = fma(r, fma(r, kExpH2, kExpH1), kExpH0);
-    const double p = fma(r * r, h, r);
-    const double T = tab[n & (kExpTable - 1)];
-    const double y = fma(T, p, T);
-    return __longlong_as_double(__double_as_longlong(y) + ((long long)(n >> 8) << 52));
+    const uint64_t bits = (uint64_t)__double_as_longlong(x);
+    const int E = (int)(bits >> 52) - 1023;  // -10..9
+    const uint64_t m = ((bits & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull) << 11;  // x = m 2^(E - 63)
+    // x 256 / ln 2 = (hi + lo / 2^64) 2^(E - 54)
+    uint64_t hi = __umul64hi(m, kExpC), lo = m * kExpC;
+    const uint64_t corr = (uint64_t)(uint32_t)(m >> 32) * kExpC2;
+    lo += corr;
+    hi += lo < corr ? 1 : 0;
+    const int a = 10 + E;  // 0..19 bits of hi above the fraction
+    const uint64_t frac = a ? (hi << a) | (lo >> (64 - a)) : hi;
+    const int n = (a ? (int)(hi >> (64 - a)) : 0) + (int)(frac >> 63);  // rounded to nearest
+    const int64_t F = (int64_t)frac;                                     // the signed rest, times 2^64
+    // u = F / 2^64 * ln2 / 256, times 2^72
+    const int64_t A = (int64_t)(__umul64hi((uint64_t)F, kLn2) - (F < 0 ? kLn2 : 0));
+    const int ah = (int)(A >> 32);
+    const int64_t B = (int64_t)ah * ah + (((int64_t)ah * (int64_t)(uint32_t)A) >> 31);  // u^2 2^80
+    const int b32 = (int)(B >> 32);                                                      // u^2 2^48
+    const int d3 = __mulhi(__mulhi(ah, b32), 715827882);   // u^3 / 6, times 2^56
+    const int q4 = __mulhi(__mulhi(b32, b32), 178956970);  // u^4 / 24, times 2^64
+    const int f5 = __mulhi(d3, b32) / 20;                  // u^5 / 120, times 2^72
+    const int64_t V = (B >> 9) - A - ((int64_t)d3 << 16) + ((int64_t)q4 << 8) - f5;  // exp(-u) - 1, times 2^72
+    const uint64_t G = tab[n & (kExpTable - 1)];
+    const int64_t GV = (int64_t)(__umul64hi(G, (uint64_t)V) - (V < 0 ? G : 0));
+    const uint64_t R = G + (uint64_t)(GV >> 8);
+    const int lz = (int)(R >> 63) ^ 1;  // 2^62 < R < 2^64
+    const uint64_t r = ((R << lz) + 0x400ull) >> 11;
+    // r 2^(11 - lz) 2^-65 2^-(n / 256); r's leading bit adds to the exponent field
+    return __longlong_as_double((int64_t)(r + ((uint64_t)(1023 + 52 + 11 - lz - 65 - (n >> 8) - 1) << 52)));
 }
 
 // Per-cell terms of GetCurIllum (solve_module/illum/Illum_async.cpp:259-470):
 // scattering form k = alpha + beta, R = Q + S' beta; absorption form
-// k = alpha, R = Q; ks = k * s_scale, Rk = R / k.  The medium table keeps k,
-// beta (0 in the absorption form), Q and 1 / k per cell, so that neither an
-// item nor a node adds or divides for them.
+// k = alpha, R = Q; ks = k * s_scale, Rk = R / k.  The medium table keeps beta
+// (0 in the absorption form), Q, k and 1 / k per cell, so that neither an item
+// nor a node adds or divides for them.
 struct CellTerms {
     double k, ks, R, Rk;
 };
 
-__device__ inline CellTerms cell_terms(const rts_medium& md, bool unit_i, bool unit_s, double k, double betta,
-                                       double Q, double inv_k, double S)
+__device__ inline double cell_source(const rts_medium& md, bool unit_i, double betta, double Q, double S)
 {
-    CellTerms t;
-    t.k = k;
-    t.R = Q + (unit_i ? S : S * md.i_scale) * betta;
-    t.ks = unit_s ? k : k * md.s_scale;
-    t.Rk = t.R * inv_k;
-    return t;
+    return Q + (unit_i ? S : S * md.i_scale) * betta;
 }
-
-// the table entry (k, beta, Q, 1/k) of coefficients alpha, beta, Q
+// the table entry (beta, Q, k, 1/k) of coefficients alpha, beta, Q
 __host__ __device__ inline void medium_entry(int mode, double alpha, double betta, double Q, double* e)
 {
     const double k = mode == RTS_MEDIUM_ABSORPTION ? alpha : alpha + betta;
-    e[0] = k;
-    e[1] = mode == RTS_MEDIUM_ABSORPTION ? 0.0 : betta;
-    e[2] = Q;
+    e[0] = mode == RTS_MEDIUM_ABSORPTION ? 0.0 : betta;
+    e[1] = Q;
+    e[2] = k;
     e[3] = k != 0.0 ? 1.0 / k : 0.0;  // k = 0: those nodes take the reference's expression
 }
 
@@ -311,11 +342,11 @@ constexpr int kFastXHi = 0x4085E000;  // high word of 700
 // next ones.
 constexpr double kAttRef = -1.0;
 
-__device__ inline double node_att(const CellTerms& t, double s, const double* __restrict__ tab)
+__device__ inline double node_att(double ks, double s, const uint64_t* __restrict__ tab)
 {
-    const double x = t.ks * s;
+    const double x = ks * s;
     const int hx = __double2hiint(x);
-    return (hx >= kFastXLo && hx <= kFastXHi) ? exp_neg(-x, tab) * (1.0 / 3.0) : kAttRef;
+    return (hx >= kFastXLo && hx <= kFastXHi) ? exp_fixed(x, tab) : kAttRef;
 }
 
 // A third of the node value from its factor e3 = e / 3 (s is read only on
@@ -336,27 +367,51 @@ __device__ inline double node_third(const rts_medium& md, bool unit_i, const Cel
     return unit_i ? I : I / md.i_scale;
 }
 
-// ReCalcIllum's term |old - cur| / cur for one face (Illum_async.cpp:488-493),
-// folded into the running max.  The division runs only when the term can
-// raise the max; NaN terms (0 / 0) drop out as in the reference.  (A screen
-// of the terms on the exponent fields with integer operations, meant to spare
-// the multiply and compare, measured 4-7 % slower: as compiled it added FP64
-// operations instead of removing them.)
-__device__ inline void norm_term(double old, double cur, double& loc)
-{
-    const double d = fabs(old - cur);
-    if (d > loc * cur) {
-        const double b = d / cur;
-        if (b > loc) loc = b;
+// ReCalcIllum's max of |old - cur| / cur over the faces (Illum_async.cpp:
+// 488-493); NaN terms (0 / 0) drop out as in the reference.  A face whose term
+// cannot raise the max is told from the high words alone.  As integers these
+// step by 2^-20 of their octave's base 2^e: for cur = m 2^e and high words dh
+// < 2^20 apart |old - cur| is below (dh + 1) 2^(e-20), or twice that where old
+// lies in the next octave, so the term is below the max while dh + 1 <= max m 2^20; and
+// for 0 <= old < cur it is at most 1.  The FP64 operations run only where a lane
+// needs them.
+struct NormMax {
+    double loc = -1.0;
+    unsigned int skip = 0;  // floor(loc 2^20), at most 2^21
+    __device__ __forceinline__ bool below(double old, double cur) const
+    {
+        const int ho = __double2hiint(old), hc = __double2hiint(cur);
+        const unsigned int lo = (unsigned int)min(ho, hc), dh = (unsigned int)max(ho, hc) - lo;
+        const unsigned int m = ((unsigned int)hc & 0xFFFFFu) | 0x100000u;  // m 2^20
+        const unsigned int lim = __umulhi(skip << 6, m << 6);              // max m 2^20, rounded down
+        const unsigned int d = (ho >> 20) > (hc >> 20) ? 2 * dh + 1 : dh;
+        return hc >= 0x00100000 &&
+               ((dh < 1u << 20 && d < lim) || ((unsigned int)ho < (unsigned int)hc && skip >= 1u << 20));
     }
-}
+    // the terms of a face's own value and of the neighbour's copy
+    __device__ __forceinline__ void term(double old, double cur, bool copy, double old_n)
+    {
+        if (below(old, cur) && (!copy || below(old_n, cur))) return;
+#pragma unroll 1
+        for (int j = copy ? 0 : 1; j < 2; ++j) {
+            const double d = fabs((j ? old : old_n) - cur);
+            if (d > loc * cur) {
+                const double b = d / cur;
+                if (b > loc) {
+                    loc = b;
+                    skip = b >= 2.0 ? 1u << 21 : (unsigned int)(b * 1048576.0);
+                }
+            }
+        }
+    }
+};
 
-__device__ __forceinline__ void prefetch_l1(const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // L2 eviction priorities of the sweep's loads.  Every direction reads the
-// cells' neighbour table and medium entries (48 B per cell, 32 MB at 663,552
-// cells: they fit in L2), while the items and attenuation factors (4 B and
-// 24 B per item) are read once per sweep.  Loads of the shared tables are
+// cells' medium entries (beta, Q: 16 B of 32 B per cell, 21 MB at 663,552 cells:
+// they fit in L2), while the items, copy words and attenuation factors (4, 4 and
+// 32 B per item) are read once per sweep.  Loads of the shared tables are
 // marked evict-last and the streams evict-first, so the streams do not push
 // the tables out of L2 (cache hints only: the values are the same).
 __device__ __forceinline__ uint64_t l2_policy_last()
@@ -385,12 +440,6 @@ __device__ __forceinline__ double2 ld_hint(const double2* q, uint64_t pol)
     asm volatile("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(q), "l"(pol));
     return v;
 }
-__device__ __forceinline__ double ld_hint(const double* q, uint64_t pol)
-{
-    double v;
-    asm volatile("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(q), "l"(pol));
-    return v;
-}
 __device__ __forceinline__ uint32_t ld_hint(const uint32_t* q, uint64_t pol)
 {
     uint32_t v;
@@ -398,13 +447,57 @@ __device__ __forceinline__ uint32_t ld_hint(const uint32_t* q, uint64_t pol)
     return v;
 }
 
-__device__ inline double pick(int g, double v0, double v1, double v2, double v3)
+
+// What an item reads that nothing it depends on writes during a sweep (what its
+// face and the neighbour's copy hold is changed by the item itself).
+struct ItemData {
+    uint32_t w, cp; // item and copy word
+    double2 bq;     // beta, Q
+    double2 ki;     // k, 1 / k (kAtt 0, 1)
+    double S;
+    double2 fa, fb; // kAtt 2: the factors e_0, e_1, e_2 (thirds) and q; else the node distances (fb.y unused)
+    double old, old_n;
+};
+
+// Position in a direction's items: item idx of step lev, which ends at end.
+struct ItemIter {
+    int idx, lev, end;
+    // a thread takes every T-th item of a step, and goes on to the next step that has one for it
+    __device__ __forceinline__ void settle(const int32_t* steps, int ns)
+    {
+        while (idx >= end && lev + 1 < ns) {
+            idx = end + (int)threadIdx.x;
+            ++lev;
+            end = steps[lev + 1];
+        }
+    }
+    __device__ __forceinline__ bool valid() const { return idx < end; }
+};
+
+constexpr int kStepCache = 1024;  // step offsets kept in shared memory
+
+// The face mean node by node, for the items whose nodes may clamp or take the
+// reference's expression, and for media with a ball or a scale (out of line:
+// rare, or bound by its divisions anyway).  e3: the factors, negative where the
+// reference's expression applies.
+__device__ __noinline__ double mean_by_nodes(const SweepArgs& a, uint32_t w, bool unit_i, double betta, double Q,
+                                             double Sc, const double* sr, double e0, double e1, double e2, double v0,
+                                             double v1, double v2, bool in0, bool in1, bool in2)
 {
-    return g == 0 ? v0 : g == 1 ? v1 : g == 2 ? v2 : v3;
-}
-__device__ inline int pick(int g, int v0, int v1, int v2, int v3)
-{
-    return g == 0 ? v0 : g == 1 ? v1 : g == 2 ? v2 : v3;
+    const bool unit_s = a.md.s_scale == 1.0;
+    const double* me = a.med + 4 * (int64_t)(w >> 8);
+    const double k = me[2], ik = me[3];
+    double mean = 0.0;
+    for (int m = 0; m < 3; ++m) {
+        const bool in = m == 0 ? in0 : m == 1 ? in1 : in2;
+        CellTerms t;
+        t.k = in ? a.ball[2] : k;
+        t.R = cell_source(a.md, unit_i, in ? a.ball[0] : betta, in ? a.ball[1] : Q, Sc);
+        t.ks = unit_s ? t.k : t.k * a.md.s_scale;
+        t.Rk = t.R * (in ? a.ball[3] : ik);
+        mean += node_third(a.md, unit_i, t, m == 0 ? e0 : m == 1 ? e1 : e2, sr + m, m == 0 ? v0 : m == 1 ? v1 : v2);
+    }
+    return mean;
 }
 
 // One CTA per local direction.  First the boundary in-faces take their
@@ -414,162 +507,240 @@ __device__ inline int pick(int g, int v0, int v1, int v2, int v3)
 // (visible after the barrier); it writes its mean to the face and to the
 // neighbour's copy.  Every face is written once per sweep, so each writer
 // takes ReCalcIllum's term against the old value.
+//
+// A step is a chain: barrier, in-face means, five dependent FP64 operations,
+// store.  Everything else an item needs is known before the step starts, so it
+// is loaded one item ahead, across steps: the item words two, the factors'
+// lines into L2 four, the neighbour's copy into L2 two.  What bounds it: latency
+// (half of the stalls wait for the in-face means, a third of the issue slots are
+// used) and then the FP64 pipe, two operations per SM and cycle, of which an
+// item now takes five (the norm and the exponential are integer work); DRAM is
+// far from its rate.  T threads, kCtas of them per SM with their registers.
+// Reading the factors, 82,944 cells x 400 directions (192 threads, 3 CTAs per
+// SM): 1.83 ms, 4.49 with node-by-node means, 24-byte factors, FP64 norm and
+// loads where they are used; storing them 3.0, from 8.22 with FP64 exponentials;
+// 6,000 x 48 (256 threads, one CTA per SM): 0.16 from 0.39 and 0.20 from 0.61.
 // kAtt: 0 evaluates every node's attenuation factor, 1 also stores it,
-// 2 reads the stored factors (no exponential).  kUnitI: i_scale == 1 (no
-// scaling of the source and the node values, and the one-step face mean).
-template <int kAtt, bool kUnitI>
-__global__ void __launch_bounds__(SWEEP_THREADS, 7) sweep_kernel(SweepArgs a)
+// 2 reads the stored factors (no exponential).  kPlain: i_scale == 1 and no
+// ball (the one-step face mean).
+template <int kAtt, bool kPlain, int T, int kCtas>
+__global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__ SweepArgs a)
 {
     const int64_t d = blockIdx.x;
     const int64_t N = a.N;
-    const uint32_t* items = a.items[d];
-    const double* recs = a.recs[d];
-    const int32_t* steps = a.steps[d];
+    const uint32_t* __restrict__ items = a.items[d];
+    const double* __restrict__ recs = a.recs[d];
     const int ns = a.nsteps[d];
-    const double* Sd = a.S + d * N;
+    const double* __restrict__ Sd = a.S + d * N;
     double* Il = a.illum + d * N * 4;
-    const bool ball = a.md.radius > 0;
-    constexpr bool unit_i = kUnitI;
-    const bool unit_s = a.md.s_scale == 1.0;
-    double* att = kAtt ? a.att[d] : nullptr;
-    __shared__ double tab[kAtt == 2 ? 1 : kExpTable];
-    if (kAtt != 2) {
-        for (int i = threadIdx.x; i < kExpTable; i += SWEEP_THREADS) tab[i] = a.exp2tab[i];
-        __syncthreads();
+    const bool unit_i = kPlain || a.md.i_scale == 1.0;
+    const bool ball = !kPlain && a.md.radius > 0;
+    double2* att = kAtt ? reinterpret_cast<double2*>(a.att[d]) : nullptr;
+    __shared__ uint64_t tab[kAtt == 2 ? 1 : kExpTable];
+    __shared__ int32_t sstep[kStepCache];
+    const int32_t* steps = a.steps[d];
+    if (kAtt != 2)
+        for (int i = threadIdx.x; i < kExpTable; i += T) tab[i] = a.exptab[i];
+    if (ns < kStepCache) {
+        for (int i = threadIdx.x; i <= ns; i += T) sstep[i] = steps[i];
+        steps = sstep;
     }
-    double loc = -1.0;
+    NormMax norm;
     {
         const uint32_t* bnd = a.bnd[d];
         const int nb = a.nbnd[d];
-        for (int i = threadIdx.x; i < nb; i += SWEEP_THREADS) {
+        for (int i = threadIdx.x; i < nb; i += T) {
             const uint32_t id = bnd[i];
             const double I0 = a.bc[-a.pairs[id] - 1];
             const double mean = (I0 + I0 + I0) * (1.0 / 3.0);
-            norm_term(Il[id], mean, loc);
+            norm.term(Il[id], mean, false, 0.0);
             Il[id] = mean;
         }
     }
+    __syncthreads();
     const uint64_t keep = l2_policy_last(), stream = l2_policy_first();
+    const int n_items = ns > 0 ? steps[ns] : 0;
+    // cells are below 2^24 and items below 2^26, so 32-bit indexes reach everything
+    auto load = [&](uint32_t w, uint32_t cp, uint32_t i, ItemData& x) {
+        const uint32_t c = w >> 8;
+        x.w = w;
+        x.cp = cp;
+        x.bq = ld_hint(reinterpret_cast<const double2*>(a.med) + 2 * c, keep);
+        x.S = Sd[c];
+        x.old = Il[4 * c + ((w >> 6) & 3u)];
+        x.old_n = (int)cp >= 0 ? Il[cp & kCopyIndex] : 0.0;
+        if (kAtt == 2) {
+            x.fa = ld_hint(att + 2 * i, stream);
+            x.fb = ld_hint(att + 2 * i + 1, stream);
+        } else {
+            x.ki = ld_hint(reinterpret_cast<const double2*>(a.med) + 2 * c + 1, keep);
+            x.fa.x = recs[3 * (size_t)i];
+            x.fa.y = recs[3 * (size_t)i + 1];
+            x.fb.x = recs[3 * (size_t)i + 2];
+        }
+    };
+    ItemIter it;  // the item whose words are fetched next
+    it.lev = 0;
+    it.idx = ns > 0 ? steps[0] + (int)threadIdx.x : 0;
+    it.end = ns > 0 ? steps[1] : 0;
+    it.settle(steps, ns);
+    // the current item (i, lev; data in cur) and the next one's words
+    int i = it.idx, lev = it.lev;
+    bool have = it.valid();
+    ItemData cur;
+    uint32_t w1 = 0, cp1 = 0;
+    auto load_words = [&](int idx, uint32_t& w, uint32_t& cp) {
+        w = ld_hint(items + idx, stream);
+        cp = a.words ? ld_hint(items + n_items + idx, stream) : copy_word(a.pairs, nullptr, w);
+    };
+    if (have) {
+        load_words(i, w1, cp1);
+        load(w1, cp1, (uint32_t)i, cur);
+        it.idx += T;
+        it.settle(steps, ns);
+        if (it.valid()) load_words(it.idx, w1, cp1);
+    }
     for (int L = 0; L < ns; ++L) {
-        const int i1 = steps[L + 1];
-        // the next item's word is loaded one iteration ahead and its cell's
-        // rows prefetched into L1, so that the dependent loads of the next
-        // iteration find them (the chain word -> cell -> rows otherwise
-        // waits on memory twice per item)
-        int i = steps[L] + threadIdx.x;
-        uint32_t w_next = i < i1 ? ld_hint(items + i, stream) : 0u;
-        for (; i < i1; i += SWEEP_THREADS) {
-            const uint32_t w = w_next;
-            if (i + SWEEP_THREADS < i1) {
-                w_next = ld_hint(items + i + SWEEP_THREADS, stream);
-                const int64_t cn = w_next >> 8;
-                prefetch_l1(Il + 4 * cn);
-                prefetch_l1(a.pairs + 4 * cn);
-                prefetch_l1(a.med + 4 * cn);
-                prefetch_l1(Sd + cn);
+        while (have && lev == L) {
+            const double* row = Il + 4 * (cur.w >> 8);
+            double v0 = row[cur.w & 3u], v1 = row[(cur.w >> 2) & 3u], v2 = row[(cur.w >> 4) & 3u];
+            // the next item's data and the words of the one after it
+            ItemData nxt;
+            const bool more = it.valid();
+            const int i1 = it.idx, lev1 = it.lev;
+            if (more) {
+                load(w1, cp1, (uint32_t)i1, nxt);
+                it.idx += T;
+                it.settle(steps, ns);
+                if (it.valid()) load_words(it.idx, w1, cp1);
+                if (kAtt == 2 && i + 4 * T < n_items) prefetch_l2(att + 2 * (uint32_t)(i + 4 * T));
             }
-            const int64_t c = w >> 8;
-            const int f = (int)((w >> 6) & 3u);
-            const double2 f01 = *reinterpret_cast<const double2*>(Il + 4 * c);
-            const double2 f23 = *reinterpret_cast<const double2*>(Il + 4 * c + 2);
-            const int4 pr = ld_hint(reinterpret_cast<const int4*>(a.pairs + 4 * c), keep);
-            const double2 m01 = ld_hint(reinterpret_cast<const double2*>(a.med + 4 * c), keep);
-            const double2 m23 = ld_hint(reinterpret_cast<const double2*>(a.med + 4 * c + 2), keep);
-            const double Sc = Sd[c];
-            const CellTerms cell = cell_terms(a.md, unit_i, unit_s, m01.x, m01.y, m23.x, m23.y, Sc);
-            const double* sr = recs + 3 * (int64_t)i;
-            double I0[3], e3[3];
-            bool inb[3] = {false, false, false};
-#pragma unroll
-            for (int m = 0; m < 3; ++m) {
-                const int g = (int)((w >> (2 * m)) & 3u);
-                const int nbg = pick(g, pr.x, pr.y, pr.z, pr.w);
-                // CalculateIllumeOnInnerFace (Illum_async.cpp:172-199)
-                I0[m] = nbg < 0 ? a.bc[-nbg - 1] : pick(g, f01.x, f01.y, f23.x, f23.y);
-                if (ball) {  // class 0: other coefficients inside the ball
-                    const double* x = a.nodes + 36 * c + 9 * f + 3 * m;
-                    const double d0 = x[0] - a.md.ball[0], d1 = x[1] - a.md.ball[1], d2 = x[2] - a.md.ball[2];
-                    inb[m] = sqrt(d0 * d0 + d1 * d1 + d2 * d2) < a.md.radius;
+            const double R = cell_source(a.md, unit_i, cur.bq.x, cur.bq.y, cur.S);
+            double e0, e1, e2, q;
+            bool in0 = false, in1 = false, in2 = false;
+            if (ball) {  // class 0: other coefficients inside the ball
+                const double* x = a.nodes + 36 * (int64_t)(cur.w >> 8) + 9 * ((cur.w >> 6) & 3u);
+                auto inside = [&](const double* y) {
+                    const double d0 = y[0] - a.md.ball[0], d1 = y[1] - a.md.ball[1], d2 = y[2] - a.md.ball[2];
+                    return sqrt(d0 * d0 + d1 * d1 + d2 * d2) < a.md.radius;
+                };
+                in0 = inside(x), in1 = inside(x + 3), in2 = inside(x + 6);
+            }
+            if (kAtt == 2) {
+                e0 = cur.fa.x, e1 = cur.fa.y, e2 = cur.fb.x, q = cur.fb.y;
+            } else {
+                const double ks = a.md.s_scale == 1.0 ? cur.ki.x : cur.ki.x * a.md.s_scale;
+                const double kb = a.md.s_scale == 1.0 ? a.ball[2] : a.ball[2] * a.md.s_scale;
+                e0 = node_att(in0 ? kb : ks, cur.fa.x, tab);
+                e1 = node_att(in1 ? kb : ks, cur.fa.y, tab);
+                e2 = node_att(in2 ? kb : ks, cur.fb.x, tab);
+                // the source's weight in the face mean, (1 - sum_m e_m / 3) / k
+                q = (1.0 - ((e0 + e1) + e2)) * cur.ki.y;
+                if (kAtt == 1) {
+                    att[2 * (uint32_t)i] = make_double2(e0, e1);
+                    att[2 * (uint32_t)i + 1] = make_double2(e2, q);
                 }
-                if (kAtt == 2) {
-                    e3[m] = ld_hint(att + 3 * (int64_t)i + m, stream);
-                } else {
-                    const CellTerms t =
-                        inb[m] ? cell_terms(a.md, unit_i, unit_s, a.ball[0], a.ball[1], a.ball[2], a.ball[3], Sc)
-                               : cell;
-                    e3[m] = node_att(t, sr[m], tab);
-                    if (kAtt == 1) att[3 * (int64_t)i + m] = e3[m];
-                }
+            }
+            if (cur.cp & kSharedOut) {
+                // what an earlier step's item may have written
+                cur.old = row[(cur.w >> 6) & 3u];
+                cur.old_n = Il[cur.cp & kCopyIndex];
+            }
+            if (cur.cp & kBoundCell) {
+                // boundary in-faces give their value itself (CalculateIllumeOnInnerFace,
+                // Illum_async.cpp:172-199)
+                const int32_t* pr = a.pairs + 4 * (cur.w >> 8);
+                auto bound = [&](uint32_t g, double v) {
+                    const int nbg = pr[g & 3u];
+                    return nbg < 0 ? a.bc[-nbg - 1] : v;
+                };
+                v0 = bound(cur.w, v0), v1 = bound(cur.w >> 2, v1), v2 = bound(cur.w >> 4, v2);
             }
             // The face mean (I_0 + I_1 + I_2) / 3.  Where no node can clamp
-            // (R/k >= 0, every I0 >= 0 and every factor on the fast form: each
-            // node value R/k + e (I0 - R/k) is then >= 0, all sign bits tested
-            // at once) it is R/k + sum_m e_m/3 (I0_m - R/k): 3 subtractions and
-            // 3 FMAs instead of 6 operations for the nodes and 3 for the mean.
+            // (R >= 0, every I0 >= 0 and every factor on the fast form: each node
+            // value R/k + e (I0 - R/k) is then >= 0, all sign bits tested at
+            // once) it is q R + sum_m e_m/3 I0_m with q = (1 - sum_m e_m/3) / k:
+            // 4 operations and one for R, against 3 subtractions, 3 FMAs and 2 for
+            // R/k without the stored q, and 11 node by node.
             double mean;
-            if (unit_i && !ball &&
-                (__double2hiint(e3[0]) | __double2hiint(e3[1]) | __double2hiint(e3[2]) | __double2hiint(I0[0]) |
-                 __double2hiint(I0[1]) | __double2hiint(I0[2]) | __double2hiint(cell.Rk)) >= 0) {
-                const double Rk = cell.Rk;
-                mean = fma(e3[0], I0[0] - Rk, fma(e3[1], I0[1] - Rk, fma(e3[2], I0[2] - Rk, Rk)));
-            } else {
-                mean = 0.0;
-#pragma unroll
-                for (int m = 0; m < 3; ++m) {
-                    const CellTerms t =
-                        inb[m] ? cell_terms(a.md, unit_i, unit_s, a.ball[0], a.ball[1], a.ball[2], a.ball[3], Sc)
-                               : cell;
-                    mean += node_third(a.md, unit_i, t, e3[m], sr + m, I0[m]);
-                }
-            }
-            const double old_f = pick(f, f01.x, f01.y, f23.x, f23.y);
-            norm_term(old_f, mean, loc);
-            Il[4 * c + f] = mean;
-            const int nb = pick(f, pr.x, pr.y, pr.z, pr.w);
-            if (nb >= 0) {
-                // the neighbour's copy usually holds the value this face held
-                // (both were written together by the last sweep): the same
-                // term again, skipped after an integer compare of the bits
-                const double old_n = Il[nb];
-                if (__double_as_longlong(old_n) != __double_as_longlong(old_f)) norm_term(old_n, mean, loc);
-                Il[nb] = mean;
-            }
+            if (kPlain && (__double2hiint(e0) | __double2hiint(e1) | __double2hiint(e2) | __double2hiint(v0) |
+                           __double2hiint(v1) | __double2hiint(v2) | __double2hiint(R)) >= 0)
+                mean = fma(e0, v0, fma(e1, v1, fma(e2, v2, q * R)));
+            else
+                mean = mean_by_nodes(a, cur.w, unit_i, cur.bq.x, cur.bq.y, cur.S, recs + 3 * (size_t)i, e0, e1, e2, v0,
+                                     v1, v2, in0, in1, in2);
+            // the neighbour's copy usually holds the value this face held (both
+            // were written together by the last sweep): the same term again
+            const bool copy = (int)cur.cp >= 0;
+            norm.term(cur.old, mean, copy && __double_as_longlong(cur.old_n) != __double_as_longlong(cur.old),
+                      cur.old_n);
+            Il[4 * (cur.w >> 8) + ((cur.w >> 6) & 3u)] = mean;
+            if (copy) Il[cur.cp & kCopyIndex] = mean;
+            // the copy that the item after the next replaces, on its way into L2
+            if (it.valid() && (int)cp1 >= 0) prefetch_l2(Il + (cp1 & kCopyIndex));
+            cur = nxt;
+            i = i1;
+            lev = lev1;
+            have = more;
         }
         __syncthreads();
+        // any thread's max serves the warp: fewer terms need the FP64 operations
+        norm.skip = __reduce_max_sync(0xffffffffu, norm.skip);
     }
     // max over the block, then over directions (non-negative doubles order
     // as their bit patterns; +1 keeps 0 for "no term")
+    double loc = norm.loc;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) loc = fmax(loc, __shfl_xor_sync(0xffffffffu, loc, o));
-    __shared__ double red[SWEEP_THREADS / 32];
+    __shared__ double red[T / 32];
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = loc;
     __syncthreads();
     if (threadIdx.x == 0) {
         double m = red[0];
-        for (int i = 1; i < SWEEP_THREADS / 32; ++i) m = fmax(m, red[i]);
+        for (int j = 1; j < T / 32; ++j) m = fmax(m, red[j]);
         if (m >= 0) atomicMax(a.norm, (unsigned long long)__double_as_longlong(m) + 1ull);
     }
 }
 
 // ---------------------------------------------------------------- host side
 
-void exp2_table(double* tab)
+// (a b) >> 128
+unsigned __int128 mul_hi128(unsigned __int128 a, unsigned __int128 b)
 {
-    for (int j = 0; j < kExpTable; ++j) tab[j] = exp2((double)j / kExpTable);
+    const uint64_t a1 = (uint64_t)(a >> 64), a0 = (uint64_t)a, b1 = (uint64_t)(b >> 64), b0 = (uint64_t)b;
+    const unsigned __int128 lo = (unsigned __int128)a0 * b0, m1 = (unsigned __int128)a1 * b0,
+                            m2 = (unsigned __int128)a0 * b1;
+    const unsigned __int128 mid = (lo >> 64) + (uint64_t)m1 + (uint64_t)m2;
+    return (unsigned __int128)a1 * b1 + (m1 >> 64) + (m2 >> 64) + (mid >> 64);
 }
 
-// exp_neg against CUDA's exp at n points spread over [-700, 0] (and the 1e-3
-// end): the largest difference in units in the last place of CUDA's value.
-__global__ void exp_check_kernel(int64_t n, const double* __restrict__ tab_in, double* out)
+// v 2^(-j/256) for j < 256, rounded to 64 bits from a 128-bit first entry v
+// (the table of exp_fixed: the factor times 2^129).
+void exp2_table(unsigned __int128 v, uint64_t* tab)
 {
-    __shared__ double tab[kExpTable];
+    // 2^(-1/256) * 2^128
+    const unsigned __int128 step = ((unsigned __int128)0xFF4ECB59511EC8A5ull << 64) | 0x301BA217EF18DD7Cull;
+    for (int j = 0; j < kExpTable; ++j) {
+        tab[j] = (uint64_t)((v + ((unsigned __int128)1 << 63)) >> 64);
+        v = mul_hi128(v, step);
+    }
+}
+constexpr unsigned __int128 kExpThird = ((unsigned __int128)0xAAAAAAAAAAAAAAAAull << 64) | 0xAAAAAAAAAAAAAAAAull;  // 1/3
+constexpr unsigned __int128 kExpQuarter = (unsigned __int128)1 << 127;                                              // 1/4
+
+// exp_fixed against CUDA's exp at n points spread over [-700, 0] (and the 1e-3
+// end): the largest difference in units in the last place of CUDA's value.
+__global__ void exp_check_kernel(int64_t n, const uint64_t* __restrict__ tab_in, double* out)
+{
+    __shared__ uint64_t tab[kExpTable];
     for (int i = threadIdx.x; i < kExpTable; i += blockDim.x) tab[i] = tab_in[i];
     __syncthreads();
     double worst = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double u = (double)i / (double)(n - 1);
-        const double x = i & 1 ? -700.0 * u : -1e-3 - u * u;  // the whole range, and densely near 0
-        const double a = exp_neg(x, tab), b = exp(x);
+        // the whole range from the fast form's lower end, and densely near it
+        const double x = i & 1 ? fmin(-700.0 * u, -1e-3) : -1e-3 - u * u;
+        const double a = 4.0 * exp_fixed(-x, tab), b = exp(x);
         const double ulp = fabs(__longlong_as_double(__double_as_longlong(b) + 1) - b);
         worst = fmax(worst, fabs(a - b) / ulp);
     }
@@ -677,6 +848,7 @@ void free_blocks(rts_ctx* ctx, rts_sweep_state& sw)
 {
     for (auto& b : sw.blocks) rts_dfree(ctx, b.first, b.second);
     sw.blocks.clear();
+    sw.copy_words = true;
     rts_dfree(ctx, sw.att_blk, sw.att_bytes);
     sw.att_blk = nullptr;
     sw.att_bytes = 0;
@@ -698,6 +870,19 @@ int alloc_block(rts_ctx* ctx, rts_sweep_state& sw, void** p, size_t bytes, const
     int rc = rts_dmalloc(ctx, p, bytes, what);
     if (rc == RTS_OK) sw.blocks.push_back({*p, bytes});
     return rc;
+}
+
+// Room for n items and, if it can be had, their copy words behind them; without
+// it the sweep forms the words itself.
+int alloc_items(rts_ctx* ctx, rts_sweep_state& sw, void** p, int64_t n)
+{
+    if (sw.copy_words) {
+        const std::string keep = ctx->last_error;
+        if (alloc_block(ctx, sw, p, rts_bytes<uint32_t>(2 * n), "sweep items") == RTS_OK) return RTS_OK;
+        ctx->last_error = keep;
+        sw.copy_words = false;
+    }
+    return alloc_block(ctx, sw, p, rts_bytes<uint32_t>(n), "sweep items");
 }
 
 int upload_tables(rts_ctx* ctx, rts_sweep_state& sw, cudaStream_t st)
@@ -843,14 +1028,14 @@ extern "C" int rts_sweep_build(rts_ctx* ctx, int64_t* records, int64_t* levels)
     }
     void *iblk = nullptr, *rblk = nullptr, *lblk = nullptr, *bblk = nullptr, *sblk = nullptr;
     int rc;
-    if ((rc = alloc_block(ctx, sw, &iblk, rts_bytes<uint32_t>(ni), "sweep items")) != RTS_OK) return rc;
+    if ((rc = alloc_items(ctx, sw, &iblk, ni)) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &rblk, rts_bytes<double>(3 * ni), "sweep node records")) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &lblk, rts_bytes<int32_t>(nl), "sweep steps")) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &bblk, rts_bytes<uint32_t>(nbd), "sweep boundary faces")) != RTS_OK) return rc;
     cudaStream_t st = ctx->streams[RTS_STREAM_SCATTERING_1];
     int64_t io = 0, lo = 0, bo = 0;
     for (int64_t d = 0; d < D; ++d) {
-        sw.h_items[d] = (uint32_t*)iblk + io;
+        sw.h_items[d] = (uint32_t*)iblk + (sw.copy_words ? 2 : 1) * io;
         sw.h_recs[d] = (double*)rblk + 3 * io;
         sw.h_steps[d] = (int32_t*)lblk + lo;
         sw.h_bnd[d] = (uint32_t*)bblk + bo;
@@ -892,6 +1077,7 @@ extern "C" int rts_sweep_build(rts_ctx* ctx, int64_t* records, int64_t* levels)
     a.vert = sw.d_vert;
     a.frames = (const double*)fblk;
     a.nodes = sw.d_nodes;
+    a.pairs = sw.d_pairs;
     a.dirs = ctx->d_xyz + 3 * ctx->out_start;
     a.states = (const uint8_t*)sblk;
     a.items = sw.d_items;
@@ -899,6 +1085,7 @@ extern "C" int rts_sweep_build(rts_ctx* ctx, int64_t* records, int64_t* levels)
     a.steps = sw.d_steps;
     a.nsteps = sw.d_nsteps;
     a.N = N;
+    a.words = sw.copy_words;
     a.flag = ctx->d_flag + 2;
     if (D > 0) {
         const int64_t per = std::max<int64_t>(1, std::min<int64_t>((2 * N + 255) / 256, 64));
@@ -1004,13 +1191,19 @@ extern "C" int rts_sweep_import_direction(rts_ctx* ctx, int64_t d, const int32_t
     // this direction's own blocks
     int rc;
     void *iblk = nullptr, *rblk = nullptr, *lblk = nullptr, *bblk = nullptr;
-    if ((rc = alloc_block(ctx, sw, &iblk, rts_bytes<uint32_t>(items.size()), "sweep items")) != RTS_OK) return rc;
+    if ((rc = alloc_items(ctx, sw, &iblk, (int64_t)items.size())) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &rblk, rts_bytes<double>(3 * items.size()), "sweep node records")) != RTS_OK)
         return rc;
     if ((rc = alloc_block(ctx, sw, &lblk, rts_bytes<int32_t>(steps.size()), "sweep steps")) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &bblk, rts_bytes<uint32_t>(bnd.size()), "sweep boundary faces")) != RTS_OK)
         return rc;
     RTS_CUDA_TRY(ctx, cudaMemcpy(iblk, items.data(), rts_bytes<uint32_t>(items.size()), cudaMemcpyHostToDevice));
+    if (sw.copy_words) {
+        std::vector<uint32_t> words(items.size());
+        for (size_t i = 0; i < items.size(); ++i) words[i] = copy_word(pairs, st8.data(), items[i]);
+        RTS_CUDA_TRY(ctx, cudaMemcpy((uint32_t*)iblk + items.size(), words.data(), rts_bytes<uint32_t>(words.size()),
+                                     cudaMemcpyHostToDevice));
+    }
     RTS_CUDA_TRY(ctx, cudaMemcpy(rblk, recs.data(), rts_bytes<double>(3 * items.size()), cudaMemcpyHostToDevice));
     RTS_CUDA_TRY(ctx, cudaMemcpy(lblk, steps.data(), rts_bytes<int32_t>(steps.size()), cudaMemcpyHostToDevice));
     if (!bnd.empty())
@@ -1106,9 +1299,9 @@ static int att_mode(rts_ctx* ctx, rts_sweep_state& sw, cudaStream_t st, int* mod
         *mode = 2;
         return RTS_OK;
     }
-    int64_t nrec = 0;
-    for (int64_t d = 0; d < sw.D; ++d) nrec += 3 * sw.h_nitems[d];
-    const size_t need = rts_bytes<double>(std::max<int64_t>(nrec, 2));
+    int64_t nfac = 0;
+    for (int64_t d = 0; d < sw.D; ++d) nfac += 4 * sw.h_nitems[d];
+    const size_t need = rts_bytes<double>(std::max<int64_t>(nfac, 2));
     if (sw.att_bytes != need) {
         rts_dfree(ctx, sw.att_blk, sw.att_bytes);
         sw.att_blk = nullptr;
@@ -1125,11 +1318,40 @@ static int att_mode(rts_ctx* ctx, rts_sweep_state& sw, cudaStream_t st, int* mod
     int64_t o = 0;
     for (int64_t d = 0; d < sw.D; ++d) {
         sw.h_att[d] = sw.att_blk + o;
-        o += 3 * sw.h_nitems[d];
+        o += 4 * sw.h_nitems[d];
     }
     RTS_CUDA_TRY(ctx, cudaMemcpyAsync(sw.d_att, sw.h_att.data(), sizeof(double*) * sw.D, cudaMemcpyHostToDevice, st));
     *mode = 1;
     return RTS_OK;
+}
+
+template <int T, int kCtas>
+static void launch_sweep(const SweepArgs& a, unsigned grid, int mode, cudaStream_t st)
+{
+    const bool plain = a.md.i_scale == 1.0 && !(a.md.radius > 0);
+    auto* kernel = plain ? (mode == 2   ? sweep_kernel<2, true, T, kCtas>
+                             : mode == 1 ? sweep_kernel<1, true, T, kCtas>
+                                         : sweep_kernel<0, true, T, kCtas>)
+                          : (mode == 2   ? sweep_kernel<2, false, T, kCtas>
+                             : mode == 1 ? sweep_kernel<1, false, T, kCtas>
+                                         : sweep_kernel<0, false, T, kCtas>);
+    kernel<<<grid, T, 0, st>>>(a);
+}
+
+// Threads per direction, up to the mean size of a step, and as many as leave
+// every resident CTA its registers.  Reading form, 82,944 x 400, three CTAs per
+// SM: 192 threads 1.83 ms, 160 1.94, 256 (80 registers, spills) 2.30.  With more
+// directions 128 threads, 5 CTAs per SM while those hold them all (24,576 x 700,
+// five sweeps with their integrals 7.5 ms against 9.6 with 7), then 7 with at
+// most 72 registers: one wave of 152 x 7 CTAs holds 1,000 directions.
+enum class SweepForm { t512, t256, t192, t128, t128x7 };
+static SweepForm sweep_form(const rts_ctx* ctx, const rts_sweep_state& sw)
+{
+    const int64_t items = sw.records / 3, per_step = items / std::max<int64_t>(1, sw.D * sw.max_levels);
+    if (sw.D > 5 * ctx->num_sms) return SweepForm::t128x7;
+    if (sw.D > 3 * ctx->num_sms || per_step <= 128) return SweepForm::t128;
+    if (sw.D > 2 * ctx->num_sms) return SweepForm::t192;
+    return sw.D > ctx->num_sms || per_step <= 256 ? SweepForm::t256 : SweepForm::t512;
 }
 
 static int enqueue_sweep(rts_ctx* ctx, cudaStream_t st)
@@ -1153,28 +1375,21 @@ static int enqueue_sweep(rts_ctx* ctx, cudaStream_t st)
     a.S = ctx->d_S;
     a.illum = ctx->d_illum + ctx->out_start * sw.N * 4;
     a.N = sw.N;
+    a.words = sw.copy_words;
     a.md = sw.md;
     for (int i = 0; i < 4; ++i) a.bc[i] = sw.bc[i];
-    exp2_table(a.exp2tab);
+    exp2_table(kExpThird, a.exptab);
     medium_entry(sw.md.mode, sw.md.ball_alpha, sw.md.ball_beta, sw.md.ball_q, a.ball);
     a.norm = sw.d_norm;
     if (sw.D > 0) {
         rts_timing_begin(ctx, st);
-        const dim3 grid((unsigned)sw.D);
-        if (sw.md.i_scale == 1.0) {
-            if (mode == 2)
-                sweep_kernel<2, true><<<grid, SWEEP_THREADS, 0, st>>>(a);
-            else if (mode == 1)
-                sweep_kernel<1, true><<<grid, SWEEP_THREADS, 0, st>>>(a);
-            else
-                sweep_kernel<0, true><<<grid, SWEEP_THREADS, 0, st>>>(a);
-        } else {
-            if (mode == 2)
-                sweep_kernel<2, false><<<grid, SWEEP_THREADS, 0, st>>>(a);
-            else if (mode == 1)
-                sweep_kernel<1, false><<<grid, SWEEP_THREADS, 0, st>>>(a);
-            else
-                sweep_kernel<0, false><<<grid, SWEEP_THREADS, 0, st>>>(a);
+        const unsigned grid = (unsigned)sw.D;
+        switch (sweep_form(ctx, sw)) {
+        case SweepForm::t512: launch_sweep<512, 1>(a, grid, mode, st); break;
+        case SweepForm::t256: launch_sweep<256, 2>(a, grid, mode, st); break;
+        case SweepForm::t192: launch_sweep<192, 3>(a, grid, mode, st); break;
+        case SweepForm::t128: launch_sweep<128, 5>(a, grid, mode, st); break;
+        case SweepForm::t128x7: launch_sweep<128, 7>(a, grid, mode, st); break;
         }
         rts_timing_end(ctx, st);
         RTS_CHECK_LAUNCH(ctx, "sweep_kernel");
@@ -1262,17 +1477,18 @@ extern "C" int rts_sweep_exp_check(rts_ctx* ctx, int64_t n, double* max_ulp)
 {
     if (!ctx) return RTS_ERR_INVALID_ARGUMENT;
     RTS_REQUIRE(ctx, n >= 2 && max_ulp, RTS_ERR_INVALID_ARGUMENT, "rts_sweep_exp_check: n >= 2 and an output");
-    double tab[kExpTable];
-    exp2_table(tab);
+    uint64_t tab[kExpTable];
+    exp2_table(kExpQuarter, tab);
     void* p = nullptr;
     int rc = rts_dmalloc(ctx, &p, (kExpTable + 1) * sizeof(double), "exp check");
     if (rc != RTS_OK) return rc;
     double* d = (double*)p;
     cudaStream_t st = ctx->streams[RTS_STREAM_SCATTERING_1];
-    cudaError_t e = cudaMemcpyAsync(d, tab, kExpTable * sizeof(double), cudaMemcpyHostToDevice, st);
+    cudaError_t e = cudaMemcpyAsync(d, tab, sizeof(tab), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d + kExpTable, 0, sizeof(double), st);
     if (e == cudaSuccess) {
-        exp_check_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1024), 256, 0, st>>>(n, d, d + kExpTable);
+        exp_check_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 1024), 256, 0, st>>>(n, (const uint64_t*)d,
+                                                                                             d + kExpTable);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)
