@@ -334,7 +334,8 @@ typedef struct rts_problem_desc {
     double g;       /* Henyey-Greenstein asymmetry, (-1, 1) */
     int precision;  /* RTS_PREC_FP16X3 or RTS_PREC_BF16X3 */
     int flush;      /* K-slices per FP32 drain (1 or 2; 0: automatic, see RTS_TUNE_FLUSH) */
-    int bn;         /* out-directions per tile, multiple of 16, <= 256 (0: balanced default) */
+    int bn;         /* out-directions per tile, multiple of 16, <= 256 (0: balanced default;
+                       the kernel's tiles hold at most 160) */
 } rts_problem_desc;
 
 /* Device bytes a problem holds while resident (for admission control). */
@@ -618,7 +619,7 @@ int rts_illum_solve(rts_ctx* ctx, int precision, int max_iter, double accuracy, 
  *   whole step first, later ones only in the budget it leaves: a request
  *   whose step fills the budget runs alone); 1 to 3 within a tile budget; 0
  *   every resident request every step.
- *   RTS_TUNE_SERVE_BUDGET: tiles (128 cells x up to 256 directions) per step
+ *   RTS_TUNE_SERVE_BUDGET: tiles (128 cells x up to 160 directions) per step
  *   under policies 1 to 3; 0 = 8 waves of the SMs.  At least one request
  *   always runs. */
 /*   RTS_TUNE_SERVE_SLACK: policy 1's deadline, arrival + slack/100 x the
@@ -649,7 +650,7 @@ int rts_flush_period(const rts_ctx* ctx, int precision, int* flush);
  * cells (0: four waves of 128-cell row tiles) and M Fibonacci directions at
  * `precision`, every drain period the accuracy rule allows (FP16 / BF16: 1,
  * and 2 where RTS_TUNE_FLUSH's automatic choice gives 2; TF32: 2), every
- * distinct tiling of the M out-directions (tiles of 64..256) and both tile
+ * distinct tiling of the M out-directions (tiles of 64..160) and both tile
  * orders (0: the column tiles of a row tile in turn; 1: the row tiles of a
  * column tile in turn).  The fastest width and order of each period enter
  * the context's table under (M, precision, period, cell bucket), the bucket

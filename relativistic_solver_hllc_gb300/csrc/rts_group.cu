@@ -41,26 +41,40 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn(rts_ctx* ctx)
     return fn;
 }
 
-// 2-D map over interleaved split rows [rows][units] (16-bit units): box of
-// box_cols halves x box_rows; the MMA operands use 64 x rows with a 128-byte
-// swizzle, the relaxation 8 x 32 unswizzled (16 bytes of each of 32 rows).
-int make_map(rts_ctx* ctx, void* map, const void* base, int64_t rows, int64_t units, int box_rows, int box_cols = 64,
-             bool swizzle = true)
+int encode(rts_ctx* ctx, void* map, const void* base, int dims_n, const cuuint64_t* dims, const cuuint64_t* strides,
+           const cuuint32_t* box, bool swizzle)
 {
     auto enc = encode_fn(ctx);
     if (!enc) return RTS_ERR_CUDA;
-    cuuint64_t dims[2] = {(cuuint64_t)units, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)(units * 2)};
-    cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1u, 1u};
-    CUresult r = enc(reinterpret_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base),
-                     dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    cuuint32_t estr[3] = {1u, 1u, 1u};
+    CUresult r = enc(reinterpret_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_UINT16, dims_n,
+                     const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
-        return rts_fail(ctx, RTS_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for %lld x %lld", (int)r,
-                        (long long)rows, (long long)units);
+        return rts_fail(ctx, RTS_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for %llu x %llu", (int)r,
+                        (unsigned long long)dims[0], (unsigned long long)dims[1]);
     return RTS_OK;
+}
+
+// 2-D map over interleaved split rows [rows][units] (16-bit units): the MMA
+// operands, boxes of 64 halves x box_rows with a 128-byte swizzle.
+int make_map(rts_ctx* ctx, void* map, const void* base, int64_t rows, int64_t units, int box_rows)
+{
+    const cuuint64_t dims[2] = {(cuuint64_t)units, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)(units * 2)};
+    const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
+    return encode(ctx, map, base, 2, dims, strides, box, true);
+}
+
+// 3-D map over the same rows as [parts][rows][32 units], the parts (high, low,
+// high, ... of a row's blocks) 64 bytes apart: the relaxation's boxes, 32 bytes
+// high and 32 bytes low of each of 32 rows.
+int make_relax_map(rts_ctx* ctx, void* map, const void* base, int64_t rows, int64_t units)
+{
+    const cuuint64_t dims[3] = {32u, (cuuint64_t)rows, (cuuint64_t)(units / 32)};
+    const cuuint64_t strides[2] = {(cuuint64_t)(units * 2), 64u};
+    const cuuint32_t box[3] = {16u, 32u, 2u};
+    return encode(ctx, map, base, 3, dims, strides, box, false);
 }
 
 }  // namespace
@@ -115,7 +129,7 @@ void free_prob(rts_ctx* ctx, GProb* p, cudaStream_t st)
     rts_pfree(ctx, p->lam, (size_t)(p->groups * 4), st);
     rts_pfree(ctx, p->S32, (size_t)(p->rows * p->Mout * 4), st);
     rts_pfree(ctx, p->vrow, (size_t)((p->kpad + 4) * 4), st);
-    rts_pfree(ctx, p->part, (size_t)(p->n_tiles * 4 * p->rows_pad * 16), st);
+    rts_pfree(ctx, p->part, (size_t)(p->n_tiles * G_SLICES * p->rows_pad * 16), st);
     rts_pfree(ctx, p->delta, (size_t)(p->rows_pad * 4), st);
     rts_pfree(ctx, p->ex, (size_t)(p->rows_pad * 8), st);
     delete p;
@@ -159,10 +173,10 @@ float rts_group_bias(const rts_ctx* ctx, int, int)
 
 int64_t rts_group_energy_bytes(int64_t kpad, int64_t rows_pad, int n_tiles)
 {
-    return (kpad + 4) * 4 + (int64_t)n_tiles * 4 * rows_pad * 16 + rows_pad * 12;
+    return (kpad + 4) * 4 + (int64_t)n_tiles * G_SLICES * rows_pad * 16 + rows_pad * 12;
 }
 
-// Tile geometry of a problem: out-direction tiles of at most G_BN (256), balanced.
+// Tile geometry of a problem: out-direction tiles of at most G_BN, balanced.
 void rts_group_geometry(int64_t Min, int64_t Mout, int64_t rows, int bn_override, int* bn, int* n_tiles,
                         int64_t* kpad, int64_t* mpad, int64_t* rows_pad, int64_t* m_tiles)
 {
@@ -258,7 +272,7 @@ int rts_group_new_problem(rts_batch* b, int64_t N, int64_t Min, int64_t Mout, in
     }
     if (energy) {
         GP_ALLOC(vrow, (size_t)((p->kpad + 4) * 4), "W row sums");
-        GP_ALLOC(part, (size_t)(p->n_tiles * 4 * p->rows_pad * 16), "energy partial sums");
+        GP_ALLOC(part, (size_t)(p->n_tiles * G_SLICES * p->rows_pad * 16), "energy partial sums");
         GP_ALLOC(delta, (size_t)(p->rows_pad * 4), "energy corrections");
         GP_ALLOC(ex, (size_t)(p->rows_pad * 8), "conserved sums");
     }
@@ -270,8 +284,8 @@ int rts_group_new_problem(rts_batch* b, int64_t N, int64_t Min, int64_t Mout, in
     if (rc == RTS_OK) rc = make_map(ctx, p->maps[2], p->wc, p->mpad, p->units, p->bn);
     if (rc == RTS_OK) rc = make_map(ctx, p->maps[0], p->a[0], p->rows_pad, p->units, G_BM);
     if (rc == RTS_OK && p->a[1]) rc = make_map(ctx, p->maps[1], p->a[1], p->rows_pad, p->units, G_BM);
-    if (rc == RTS_OK) rc = make_map(ctx, p->rmaps[0], p->a[0], p->rows_pad, p->units, 32, 8, false);
-    if (rc == RTS_OK && p->a[1]) rc = make_map(ctx, p->rmaps[1], p->a[1], p->rows_pad, p->units, 32, 8, false);
+    if (rc == RTS_OK) rc = make_relax_map(ctx, p->rmaps[0], p->a[0], p->rows_pad, p->units);
+    if (rc == RTS_OK && p->a[1]) rc = make_relax_map(ctx, p->rmaps[1], p->a[1], p->rows_pad, p->units);
     if (rc != RTS_OK) {
         free_prob(ctx, p, st);
         return rc;
@@ -392,8 +406,7 @@ static void fill_entry(rts_batch* b, GProb* p, int relax, size_t i, int64_t& til
     g.bias = rts_group_bias(ctx, p->mode, p->flush);
     g.fp16 = p->fp16 ? 1 : 0;
     g.tf32 = p->mode == 2 ? 1 : 0;
-    // a quarter of the tile per epilogue column slice, so that narrow tiles keep every epilogue warp busy
-    g.sw = std::min(64, (int)round_up((p->bn + 3) / 4, 16));
+    g.sw = (int)round_up((p->bn + G_SLICES - 1) / G_SLICES, 16);
     g.cur = p->cur;
     g.relax = relaxes(p, relax) ? 1 : 0;
     g.flip = g.relax;

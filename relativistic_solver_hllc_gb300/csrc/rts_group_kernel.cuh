@@ -2,35 +2,40 @@
 // split-precision scattering integral (included by rts_group.cu).
 //
 // One launch runs one source-iteration step of every problem of a batch: the
-// tiles of all problems (128 cells x up to 256 out-directions each; problems
+// tiles of all problems (128 cells x up to 160 out-directions each; problems
 // of different cell and direction counts, phase kernels and precisions) form
 // one list that persistent CTAs (one per SM) walk with a fixed stride.
 //
-// Measured on GB300: one thread issuing M = 128, N = 256 MMAs back to back
-// reaches 0.83 of the SM's tensor rate, two threads with an accumulator each
-// its full rate.  A CTA runs two issuing warps, each with N up to 256, on
-// alternate chunks of the in-direction range of the same tile (split K
-// inside the CTA), so that each accumulator is drained while the other
-// fills; of the issue schemes measured (one issuer for both accumulators,
-// both issuers on every chunk with a column half each) this was the fastest.
+// A tile's epilogue moves 16 bytes of HBM per output (the previous S read, S,
+// Ibar and the next Ibar), about as long as its contraction takes, so the two
+// overlap: 512 TMEM columns hold two accumulators of up to 160 columns and the
+// finished sums of the tile before, which warps of their own work on.  (With
+// 256-column tiles there was no room: the warps that drained also ran the
+// epilogue while the tensor cores waited, 1.29 ms a step of 162,000 x 1,000 in
+// FP16, 0.72 of them in the contraction; now 0.89.  Tensor-core time 0.5 ms,
+// HBM 0.4 ms.  The contraction alone takes 0.66 ms: M = 128, N = 144 MMAs run
+// at 0.65 of their rate, bound by the operands' way through shared memory; the
+// epilogue warps' latency is the rest.)
 //
-// Warp roles (19 warps, 608 threads, one CTA per SM):
+// Warp roles (20 warps, 640 threads, one CTA per SM):
 //   warp 0       TMA producer: A (split Ibar rows) and B (split W rows)
-//                K-slices into a 4-stage shared-memory ring;
-//   warps 1, 2   MMA issuers (one thread each); warp 1 also owns TMEM
-//                (512 columns: one 256-column accumulator per issuer);
-//   warps 3..18  drain + epilogue: warp w reads TMEM lanes 32*(w%4).. and a
-//                column slice of the tile (a quarter of it, rounded up to
-//                16 columns, so narrow tiles keep every warp busy).  After
-//                every chunk of `flush` K-slices they add the chunk's
-//                accumulator into FP32
+//                K-slices into a 5-stage shared-memory ring;
+//   warps 1, 2   MMA issuers (one thread each) on alternate chunks of the
+//                in-direction range of a tile, an accumulator each, so that
+//                one is drained while the other fills; warp 1 also owns TMEM.
+//                A stage goes back to the producer as soon as the last MMA
+//                that reads it is done;
+//   warps 4..11  drain: warp w reads TMEM lanes 32*(w%4).. and half of the
+//                tile's columns (rounded up to 16).  After every chunk of
+//                `flush` K-slices they add the chunk's accumulator into FP32
 //                registers (round-to-nearest adds: the tensor core truncates
-//                each accumulate) and release it; the tile's sums go back
-//                into its last accumulator, from which the fused epilogue
-//                (unscaling, source update, residual, S store, relaxation of
-//                Ibar in split form) reads them 8 columns at a time while
-//                the other issuer starts the next tile.  Half-way through a
-//                tile these warps prefetch the epilogue's inputs into L2.
+//                each accumulate) and release it; a finished tile's sums go
+//                to their own TMEM columns;
+//   warps 12..19 epilogue (unscaling, source update, residual, S store,
+//                relaxation of Ibar in split form) of those sums, 16 columns
+//                at a time.
+// The drain warps hold 80 sums a thread: the first warpgroup gives them its
+// registers.
 // Within a chunk the cross products hi*lo and lo*hi (2^-11 or 2^-8 of the
 // result) are issued first, while the accumulator is still small, and the two
 // hi*hi products last: the truncation then costs about one FP32 ulp of the
@@ -65,24 +70,29 @@
 #include <type_traits>
 
 constexpr int G_BM = 128;
-constexpr int G_BN = 256;
-constexpr int G_STAGES = 4;
+constexpr int G_BN = 160;    // at most: two accumulators and the finished sums in 512 TMEM columns
+constexpr int G_STAGES = 5;
 constexpr int G_A_BYTES = G_BM * 128;
 constexpr int G_B_BYTES = G_BN * 128;
 constexpr int G_STAGE_BYTES = G_A_BYTES + G_B_BYTES;
-constexpr int G_EPI_WARPS = 16;
-constexpr int G_EPI_WARP0 = 3;
+constexpr int G_SLICES = 2;  // column slices of a tile, one per warpgroup
+constexpr int G_DRAIN_WARP0 = 4, G_EPI_WARP0 = 12;
+constexpr int G_EPI_WARPS = 4 * G_SLICES;
 constexpr int G_THREADS = (G_EPI_WARP0 + G_EPI_WARPS) * 32;
+// registers a thread: 96 at launch; the first warpgroup gives 64 of them to the two that drain
+constexpr int G_REGS_ISSUE = 32, G_REGS_DRAIN = 128;
+static_assert(G_REGS_ISSUE + 2 * G_REGS_DRAIN + 2 * 96 <= 5 * 96, "registers of the block");
 constexpr int G_CTAS_PER_SM = 1;
 constexpr uint32_t G_TMEM_COLS = 512;
-constexpr int G_MAX_FLUSH = 2;  // K-slices per chunk
-// relaxation row buffers per epilogue warp: G_REL_NB - 1 units are fetched
-// ahead of the one being relaxed
-constexpr int G_REL_NB = 2;
-// ring, accumulator and relaxation barriers (the relaxation's from index 16),
-// then the TMEM address
-constexpr int G_BAR_BYTES = (8 * (17 + G_REL_NB * G_EPI_WARPS) + 127) / 128 * 128;
-constexpr int G_REL_BUF = G_REL_NB * 1024;  // per epilogue warp: buffers of 32 rows x 16 B hi, then 32 rows x 16 B lo
+constexpr uint32_t G_FIN = 2 * G_BN;  // TMEM column of the finished sums
+constexpr int G_MAX_FLUSH = 2;        // K-slices per chunk
+constexpr int G_REL_NB = 2;           // relaxation row buffers per epilogue warp
+constexpr int G_REL_BYTES = 2048;     // 32 rows x 32 B hi, then 32 rows x 32 B lo
+// ring, accumulator and hand-over barriers (the relaxation's from index
+// G_REL_BAR), then the TMEM address
+constexpr int G_REL_BAR = 2 * G_STAGES + 6;
+constexpr int G_BAR_BYTES = (8 * (G_REL_BAR + 1 + G_REL_NB * G_EPI_WARPS) + 127) / 128 * 128;
+constexpr int G_REL_BUF = G_REL_NB * G_REL_BYTES;
 constexpr size_t G_REL_OFF = (size_t)G_STAGES * G_STAGE_BYTES + G_BAR_BYTES;
 constexpr size_t G_SMEM = G_REL_OFF + (size_t)G_EPI_WARPS * G_REL_BUF + 1024;
 static_assert(G_SMEM <= 227 * 1024, "shared memory per CTA");
@@ -90,7 +100,7 @@ static_assert(G_SMEM <= 227 * 1024, "shared memory per CTA");
 struct GroupProblem {  // aligned as its CUtensorMap members
     CUtensorMap mapA[2];  // split Ibar, ping-pong buffers
     CUtensorMap mapW;     // split W^T
-    CUtensorMap mapR[2];  // split Ibar in relaxation boxes (8 columns x 32 rows), ping-pong buffers
+    CUtensorMap mapR[2];  // split Ibar in relaxation boxes (32 + 32 bytes x 32 rows), ping-pong buffers
     int64_t N;            // cells per group
     int64_t ldS;          // row pitch of S32 / S64 in cells (>= N; N unless the output is a cell range of a wider S)
     int64_t rows;         // groups * N
@@ -103,7 +113,7 @@ struct GroupProblem {  // aligned as its CUtensorMap members
     float bias;           // relative correction of the truncation bias of the sums
     int fp16;
     int tf32;             // split TF32 operands (kind::tf32, 16 in-directions per K-slice)
-    int sw;               // columns per epilogue column slice: a quarter of bn rounded up to 16 (at most 64)
+    int sw;               // columns per column slice: half of bn rounded up to 16
     int cur;              // buffer holding the current Ibar
     int relax, residual;
     int flip;             // the step ends in this launch: flip the ping-pong Ibar buffer after it
@@ -120,7 +130,7 @@ struct GroupProblem {  // aligned as its CUtensorMap members
     const float* vrow;    // [kpad + 4] v_j = sum_k W[j][k], 0 past M; vrow[kpad] = q0 (below), then c, D, 1/c:
                           // c the mean of the v_j, D = sum_j (v_j - c); output column Mout holds
                           // sum_j (v_j - c) raw_j
-    int4* part;           // [n_tiles * 4][rows_pad] per-slot partials in quanta (high, low parts):
+    int4* part;           // [n_tiles * G_SLICES][rows_pad] per-slot partials in quanta (high, low parts):
                           // sum_j v_j rs S_j, then sum_k raw_k
     double* ex;           // [rows_pad] sum_j v_j x_j of the current input, in quanta
     float* delta;         // [rows_pad] per-cell correction of the next step (0: none yet)
@@ -166,16 +176,19 @@ __device__ __forceinline__ int find_problem(const GroupProblem* probs, int nprob
     return lo;
 }
 
+// a / b of non-negative values, in 32 bits where they fit (a 64-bit division
+// is some 200 instructions on the tiles' serial path)
+__device__ __forceinline__ int64_t divide(int64_t a, int64_t b)
+{
+    return ((a | b) >> 32) == 0 ? (int64_t)((uint32_t)a / (uint32_t)b) : a / b;
+}
+
 // Row and column tile of a problem's tile lt (0 <= lt < m_tiles * n_tiles).
 __device__ __forceinline__ void tile_coords(const GroupProblem& P, int64_t lt, int& m_tile, int& n_tile)
 {
-    if (P.order) {
-        m_tile = (int)(lt % P.m_tiles);
-        n_tile = (int)(lt / P.m_tiles);
-    } else {
-        m_tile = (int)(lt / P.n_tiles);
-        n_tile = (int)(lt % P.n_tiles);
-    }
+    const int per = P.order ? P.m_tiles : P.n_tiles, hi = (int)divide(lt, per), lo = (int)(lt - (int64_t)hi * per);
+    m_tile = P.order ? lo : hi;
+    n_tile = P.order ? hi : lo;
 }
 
 // Relaxation of 8 columns of one split row in place (shared memory):
@@ -183,7 +196,7 @@ __device__ __forceinline__ void tile_coords(const GroupProblem& P, int64_t lt, i
 // past `nk` become zero (the padding of the split rows).  Returns true when
 // an FP16 value leaves the range the row scale allows.
 template <bool kFp16>
-__device__ __forceinline__ bool relax8(uint4* hp, uint4* lp, const float (&snew)[8], float hrsc, int nk)
+__device__ __forceinline__ bool relax8(uint4* hp, uint4* lp, const float* snew, float hrsc, int nk)
 {
     const uint4 rh = *hp, rl = *lp;
     const uint32_t hw[4] = {rh.x, rh.y, rh.z, rh.w};
@@ -226,26 +239,29 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + G_STAGES * G_STAGE_BYTES);  // G_BAR_BYTES
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16 + G_REL_NB * G_EPI_WARPS);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + G_REL_BAR + G_REL_NB * G_EPI_WARPS);
     const uint32_t smem_base = smem_u32(smem);
     const uint32_t bar_base = smem_u32(bars);
-    auto full_bar = [&](int s) { return bar_base + 8u * s; };
-    auto empty_bar = [&](int s) { return bar_base + 8u * (G_STAGES + s); };
-    auto acc_full_bar = [&](int a) { return bar_base + 8u * (2 * G_STAGES + a); };
-    auto acc_empty_bar = [&](int a) { return bar_base + 8u * (2 * G_STAGES + 2 + a); };
+    auto full_bar = [&](uint32_t s) { return bar_base + 8u * s; };
+    auto empty_bar = [&](uint32_t s) { return bar_base + 8u * (G_STAGES + s); };
+    auto acc_full_bar = [&](uint32_t a) { return bar_base + 8u * (2 * G_STAGES + a); };
+    auto acc_empty_bar = [&](uint32_t a) { return bar_base + 8u * (2 * G_STAGES + 2 + a); };
+    const uint32_t fin_full = bar_base + 8u * (2 * G_STAGES + 4), fin_empty = fin_full + 8u;
     // relaxation row buffers: barrier of buffer b of epilogue warp w
-    auto rel_bar = [&](int w, uint32_t b) { return bar_base + 8u * (16 + G_REL_NB * w + (int)b); };
+    auto rel_bar = [&](int w, uint32_t b) { return bar_base + 8u * (G_REL_BAR + G_REL_NB * w + (int)b); };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < G_STAGES; ++s) {
+        for (uint32_t s = 0; s < G_STAGES; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
-        for (int a = 0; a < 2; ++a) {
+        for (uint32_t a = 0; a < 2; ++a) {
             mbar_init(acc_full_bar(a), 1);
-            mbar_init(acc_empty_bar(a), G_EPI_WARPS);
+            mbar_init(acc_empty_bar(a), 4 * G_SLICES);
         }
+        mbar_init(fin_full, 4 * G_SLICES);
+        mbar_init(fin_empty, G_EPI_WARPS);
         for (int w = 0; w < G_EPI_WARPS; ++w)
             for (int b = 0; b < G_REL_NB; ++b) mbar_init(rel_bar(w, (uint32_t)b), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -258,351 +274,347 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
     const uint32_t tmem = *tmem_slot;
     const bool live = *(volatile int*)flag == 0;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ producer
-        if (lane == 0 && live) {
-            uint32_t it = 0;
-            bool ok = true;
-            for (int64_t t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-                const GroupProblem& P = probs[find_problem(probs, nprob, t)];
-                const int64_t lt = t - P.tile_begin + P.tile_off;
-                const int nkb = P.kblocks, bn = P.bn;
-                int m_tile, n_tile;
-                tile_coords(P, lt, m_tile, n_tile);
-                const int m0 = m_tile * G_BM, n0 = n_tile * bn;
-                const void* mapA = &P.mapA[P.cur];
-                const void* mapW = &P.mapW;
-                const uint32_t tx = (uint32_t)(G_A_BYTES + bn * 128);
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
-                    const int s = (int)(it % G_STAGES);
-                    if (it >= (uint32_t)G_STAGES &&
-                        !mbar_wait(empty_bar(s), ((it / G_STAGES) - 1) & 1, flag, FLAG_WAIT_PRODUCER)) {
-                        ok = false;
-                        break;
-                    }
-                    mbar_expect_tx(full_bar(s), tx);
-                    const uint32_t sa = smem_base + s * G_STAGE_BYTES;
-                    tma_load_2d(sa, mapA, kb * 64, m0, full_bar(s));
-                    tma_load_2d(sa + G_A_BYTES, mapW, kb * 64, n0, full_bar(s));
-                }
-            }
-            // no copy may still be in flight when the CTA exits
-            for (uint32_t i = (it > (uint32_t)G_STAGES ? it - G_STAGES : 0); i < it; ++i)
-                mbar_wait(full_bar(i % G_STAGES), (i / G_STAGES) & 1, flag, FLAG_WAIT_PRODUCER);
-        }
-    } else if (warp == 1 || warp == 2) {
-        // ------------------------------------------------------------ MMA issuers
-        const uint32_t me = (uint32_t)(warp - 1);
-        if (lane == 0 && live) {
-            const uint32_t acc = tmem + 256u * me;
-            uint32_t gsl = 0, gch = 0;  // K-slice and chunk counters of this CTA (across tiles)
-            bool ok = true;
-            for (int64_t t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-                const GroupProblem& P = probs[find_problem(probs, nprob, t)];
-                const uint32_t idesc = P.idesc;
-                const int nkb = P.kblocks, flush = P.flush;
-                const int nchunks = (nkb + flush - 1) / flush;
-                // the chunk loop, compiled once per MMA kind
-                auto chunks = [&](auto tf32c) {
-                    constexpr bool tf32 = decltype(tf32c)::value;
-                    auto mma = [&](uint64_t a, uint64_t b, uint32_t accumulate) {
-                        if (tf32)
-                            umma_tf32(acc, a, b, idesc, accumulate);
-                        else
-                            umma_f16(acc, a, b, idesc, accumulate);
-                    };
-                    for (int c = 0; c < nchunks; ++c) {
-                        const uint32_t g = gch + (uint32_t)c;
-                        if ((g & 1u) != me) continue;
-                        const int kb0 = c * flush;
-                        const int f = min(flush, nkb - kb0);
-                        if (g >= 2 && !mbar_wait(acc_empty_bar(me), ((g >> 1) - 1) & 1, flag, FLAG_WAIT_MMA)) {
+    if (warp < G_DRAIN_WARP0) {
+        reg_dec<G_REGS_ISSUE>();
+        if (warp == 0) {
+            // -------------------------------------------------------- producer
+            if (lane == 0 && live) {
+                uint32_t it = 0;
+                bool ok = true;
+                for (int64_t t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+                    const GroupProblem& P = probs[find_problem(probs, nprob, t)];
+                    const int64_t lt = t - P.tile_begin + P.tile_off;
+                    const int nkb = P.kblocks, bn = P.bn;
+                    int m_tile, n_tile;
+                    tile_coords(P, lt, m_tile, n_tile);
+                    const int m0 = m_tile * G_BM, n0 = n_tile * bn;
+                    const void* mapA = &P.mapA[P.cur];
+                    const void* mapW = &P.mapW;
+                    const uint32_t tx = (uint32_t)(G_A_BYTES + bn * 128);
+                    for (int kb = 0; kb < nkb; ++kb, ++it) {
+                        const uint32_t s = it % G_STAGES;
+                        if (it >= (uint32_t)G_STAGES &&
+                            !mbar_wait(empty_bar(s), ((it / G_STAGES) - 1) & 1, flag, FLAG_WAIT_PRODUCER)) {
                             ok = false;
                             break;
                         }
-                        uint32_t ad[G_MAX_FLUSH], st[G_MAX_FLUSH];
-                        for (int j = 0; j < f; ++j) {
-                            const uint32_t i2 = gsl + (uint32_t)(kb0 + j);
-                            st[j] = i2 % G_STAGES;
-                            if (!mbar_wait(full_bar((int)st[j]), (i2 / G_STAGES) & 1, flag, FLAG_WAIT_MMA)) {
+                        mbar_expect_tx(full_bar(s), tx);
+                        const uint32_t sa = smem_base + s * G_STAGE_BYTES;
+                        tma_load_2d(sa, mapA, kb * 64, m0, full_bar(s));
+                        tma_load_2d(sa + G_A_BYTES, mapW, kb * 64, n0, full_bar(s));
+                    }
+                }
+                // no copy may still be in flight when the CTA exits
+                for (uint32_t i = (it > (uint32_t)G_STAGES ? it - G_STAGES : 0); i < it; ++i)
+                    mbar_wait(full_bar(i % G_STAGES), (i / G_STAGES) & 1, flag, FLAG_WAIT_PRODUCER);
+            }
+        } else if (warp < 3) {
+            // -------------------------------------------------------- MMA issuers
+            const uint32_t me = (uint32_t)(warp - 1);
+            if (lane == 0 && live) {
+                const uint32_t acc = tmem + G_BN * me;
+                const uint32_t desc0 = (uint32_t)smem_desc_sw128(smem_base);  // low word, stage 0
+                uint32_t gsl = 0, gch = 0;  // K-slice and chunk counters of this CTA (across tiles)
+                bool ok = true;
+                for (int64_t t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+                    const GroupProblem& P = probs[find_problem(probs, nprob, t)];
+                    const uint32_t idesc = P.idesc, nkb = (uint32_t)P.kblocks, flush = (uint32_t)P.flush;
+                    const uint32_t nchunks = (nkb + flush - 1) / flush;
+                    // the chunk loop, compiled once per MMA kind
+                    auto chunks = [&](auto tf32c) {
+                        constexpr bool tf32 = decltype(tf32c)::value;
+                        // a K-slice's cross products (32 bytes high, 32 bytes low parts, twice), its hi*hi
+                        auto cross = [&](uint32_t a, uint32_t accumulate) {
+                            const uint32_t b = a + (G_A_BYTES >> 4);
+                            umma_lo<tf32>(acc, a, b + 4, idesc, accumulate);
+                            umma_lo<tf32>(acc, a + 4, b, idesc, 1u);
+                            umma_lo<tf32>(acc, a + 2, b + 6, idesc, 1u);
+                            umma_lo<tf32>(acc, a + 6, b + 2, idesc, 1u);
+                        };
+                        auto high = [&](uint32_t a) {
+                            const uint32_t b = a + (G_A_BYTES >> 4);
+                            umma_lo<tf32>(acc, a, b, idesc, 1u);
+                            umma_lo<tf32>(acc, a + 2, b + 2, idesc, 1u);
+                        };
+#pragma unroll 1
+                        for (uint32_t c = (gch ^ me) & 1u; c < nchunks; c += 2) {
+                            const uint32_t g = gch + c, i0 = gsl + c * flush, i1 = i0 + 1;
+                            const bool two = flush > 1 && c * flush + 1 < nkb;
+                            const uint32_t s0 = i0 % G_STAGES, s1 = i1 % G_STAGES;
+                            if ((g >= 2 && !mbar_wait(acc_empty_bar(me), ((g >> 1) - 1) & 1, flag, FLAG_WAIT_MMA)) ||
+                                !mbar_wait(full_bar(s0), (i0 / G_STAGES) & 1, flag, FLAG_WAIT_MMA) ||
+                                (two && !mbar_wait(full_bar(s1), (i1 / G_STAGES) & 1, flag, FLAG_WAIT_MMA))) {
                                 ok = false;
                                 break;
                             }
-                            ad[j] = smem_base + st[j] * G_STAGE_BYTES;
+                            tc_fence_after();
+                            const uint32_t a0 = desc0 + s0 * (G_STAGE_BYTES >> 4);
+                            const uint32_t a1 = desc0 + s1 * (G_STAGE_BYTES >> 4);
+                            // cross products first (the accumulator starts from zero), hi*hi last
+                            cross(a0, 0u);
+                            if (two) cross(a1, 1u);
+                            high(a0);
+                            umma_commit(empty_bar(s0));
+                            if (two) {
+                                high(a1);
+                                umma_commit(empty_bar(s1));
+                            }
+                            umma_commit(acc_full_bar(me));
                         }
-                        if (!ok) break;
-                        tc_fence_after();
-                        const uint64_t hi0 = 0, hi1 = 32 >> 4, lo0 = 64 >> 4, lo1 = 96 >> 4;
-                        // cross products first (the accumulator starts from zero), hi*hi last
-                        for (int j = 0; j < f; ++j) {
-                            const uint64_t A = smem_desc_sw128(ad[j]), Bd = smem_desc_sw128(ad[j] + G_A_BYTES);
-                            mma(A + hi0, Bd + lo0, j != 0 ? 1u : 0u);
-                            mma(A + lo0, Bd + hi0, 1u);
-                            mma(A + hi1, Bd + lo1, 1u);
-                            mma(A + lo1, Bd + hi1, 1u);
-                        }
-                        for (int j = 0; j < f; ++j) {
-                            const uint64_t A = smem_desc_sw128(ad[j]), Bd = smem_desc_sw128(ad[j] + G_A_BYTES);
-                            mma(A + hi0, Bd + hi0, 1u);
-                            mma(A + hi1, Bd + hi1, 1u);
-                        }
-                        for (int j = 0; j < f; ++j) umma_commit(empty_bar((int)st[j]));
-                        umma_commit(acc_full_bar((int)me));
-                    }
-                };
-                if (P.tf32)
-                    chunks(std::true_type{});
-                else
-                    chunks(std::false_type{});
-                gch += (uint32_t)nchunks;
-                gsl += (uint32_t)nkb;
+                    };
+                    if (P.tf32)
+                        chunks(std::true_type{});
+                    else
+                        chunks(std::false_type{});
+                    gch += nchunks;
+                    gsl += nkb;
+                }
             }
         }
+    } else if (warp < G_EPI_WARP0) {
+        // ------------------------------------------------------------ drain warps
+        reg_inc<G_REGS_DRAIN>();
+        const int q = warp & 3;                      // TMEM lane quarter
+        const int cs = (warp - G_DRAIN_WARP0) >> 2;  // column slice of the tile
+        const uint32_t lane_off = (uint32_t)(q * 32) << 16;
+        uint32_t gch = 0, tiles = 0;
+        bool ok = live;
+        // one lane's wait, for the warp
+        auto wait = [&](uint32_t bar, uint32_t parity) {
+            bool got = true;
+            if (lane == 0) got = mbar_wait(bar, parity, flag, FLAG_WAIT_EPILOGUE);
+            return __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
+        };
+        for (int64_t t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tiles) {
+            const GroupProblem& P = probs[find_problem(probs, nprob, t)];
+            const int nchunks = (P.kblocks + P.flush - 1) / P.flush;
+            const int sw = P.sw;                          // columns per slice (multiple of 16)
+            const int ncols = min(sw, P.bn - sw * cs);    // columns of this warp (multiple of 16; <= 0: none)
+            const uint32_t col = lane_off + (uint32_t)(sw * cs);
+            float run[G_BN / G_SLICES];
+#pragma unroll
+            for (int j = 0; j < G_BN / G_SLICES; ++j) run[j] = 0.0f;
+#pragma unroll 1
+            for (int c = 0; c < nchunks; ++c) {
+                const uint32_t g = gch + (uint32_t)c, a = g & 1u;
+                if (!wait(acc_full_bar(a), (g >> 1) & 1)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t acc = tmem + G_BN * a + col;
+#pragma unroll
+                for (int j0 = 0; j0 < G_BN / G_SLICES; j0 += 32) {
+                    if (j0 + 32 <= G_BN / G_SLICES && j0 + 32 <= ncols) {
+                        float v[32];
+                        tmem_ld32(acc + (uint32_t)j0, v);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j)
+                            if (j0 + j < G_BN / G_SLICES) run[j0 + j] += v[j];
+                    } else if (j0 + 16 <= ncols) {
+                        float v[16];
+                        tmem_ld16(acc + (uint32_t)j0, v);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) run[j0 + j] += v[j];
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(acc_empty_bar(a));
+            }
+            gch += (uint32_t)nchunks;
+            if (!ok) break;
+            // hand the sums over, once the epilogue has read the previous tile's
+            if (tiles > 0 && !wait(fin_empty, (tiles - 1) & 1)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int j0 = 0; j0 < G_BN / G_SLICES; j0 += 16) {
+                if (j0 < ncols) {
+                    float v[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = run[j0 + j];
+                    tmem_st16(tmem + G_FIN + col + (uint32_t)j0, v);
+                }
+            }
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(fin_full);
+        }
     } else {
-        // ------------------------------------------------------------ drain + epilogue warps
-        const int q = warp & 3;                    // TMEM lane quarter
-        const int cs = (warp - G_EPI_WARP0) >> 2;  // column slice of the tile
+        // ------------------------------------------------------------ epilogue warps
+        const int q = warp & 3;
+        const int cs = (warp - G_EPI_WARP0) >> 2;
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;
         const int ew = warp - G_EPI_WARP0;
         uint8_t* rbuf = smem + G_REL_OFF + (size_t)ew * G_REL_BUF;
         const uint32_t rbuf_s = smem_u32(rbuf);
         uint32_t rel_issued = 0, rel_used = 0;  // relaxation row blocks fetched / consumed by this warp
-        uint32_t gch = 0;
+        uint32_t tiles = 0;
         bool ok = live;
-        for (int64_t t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+        for (int64_t t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tiles) {
             const GroupProblem& P = probs[find_problem(probs, nprob, t)];
-            const int nkb = P.kblocks, flush = P.flush, bn = P.bn;
-            const int nchunks = (nkb + flush - 1) / flush;
-            const int sw = P.sw;                         // columns per slice (multiple of 16, <= 64)
-            const int ncols = min(sw, bn - sw * cs);  // columns of this warp (multiple of 16; <= 0: none)
+            const int sw = P.sw;
+            const int ncols = min(sw, P.bn - sw * cs);
             const int64_t lt = t - P.tile_begin + P.tile_off;
             int m_tile, n_tile;
             tile_coords(P, lt, m_tile, n_tile);
-            float run[64];
-#pragma unroll
-            for (int j = 0; j < 64; ++j) run[j] = 0.0f;
-            uint32_t last_acc = 0;
-            int last_a = 0;
-            for (int c = 0; c < nchunks; ++c) {
-                const uint32_t g = gch + (uint32_t)c;
-                const int a = (int)(g & 1u);
-                const uint32_t acc = tmem + 256u * (uint32_t)a + lane_off + (uint32_t)(sw * cs);
+            const uint32_t fin = tmem + G_FIN + lane_off + (uint32_t)(sw * cs);
+            auto wait_sums = [&]() {
                 bool got = true;
-                if (lane == 0) got = mbar_wait(acc_full_bar(a), (g >> 1) & 1, flag, FLAG_WAIT_EPILOGUE);
-                if (!__shfl_sync(0xffffffffu, got ? 1 : 0, 0)) {
-                    ok = false;
-                    break;
-                }
+                if (lane == 0) got = mbar_wait(fin_full, tiles & 1, flag, FLAG_WAIT_EPILOGUE);
+                ok = __shfl_sync(0xffffffffu, got ? 1 : 0, 0) != 0;
                 tc_fence_after();
-#pragma unroll
-                for (int gi = 0; gi < 4; ++gi) {
-                    if (16 * gi < ncols) {
-                        float v[16];
-                        tmem_ld16(acc + 16u * gi, v);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) run[16 * gi + j] += v[j];
-                    }
-                }
-                if (c + 1 < nchunks) {
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(acc_empty_bar(a));
-                    // a few chunks before the end of the tile, pull the epilogue's
-                    // inputs (the previous S and the Ibar rows it relaxes) into L2
-                    if (c == max(0, nchunks - 4) && ncols > 0) {
-                        const int64_t r = (int64_t)m_tile * G_BM + q * 32 + lane;
-                        if (r < P.rows) {
-                            const int64_t Nc = P.N, ld = P.ldS;
-                            const int Mout = P.Mout, kb0 = n_tile * bn + sw * cs;
-                            const int64_t grp = r / Nc;
-                            if (P.S32 && P.residual) {
-                                const float* Sp = P.S32 + grp * (int64_t)Mout * ld + (r - grp * Nc);
-                                for (int j = 0; j < ncols && kb0 + j < Mout; ++j)
-                                    prefetch_l2(Sp + (int64_t)(kb0 + j) * ld);
-                            }
-                            if (P.relax && P.S32 && !P.S64 && kb0 < P.kpad) {
-                                const uint16_t* ar = P.a[P.cur] + r * 2 * (int64_t)P.kpad;
-                                const int b0 = kb0 >> 5, b1 = min(kb0 + ncols - 1, P.kpad - 1) >> 5;
-                                for (int b = b0; b <= b1; ++b) prefetch_l2(ar + 64 * (int64_t)b);
-                            }
-                        }
-                    }
-                } else {
-                    // the finished sums go back into the last accumulator, which
-                    // this warp keeps until the epilogue below has read them
-#pragma unroll
-                    for (int gi = 0; gi < 4; ++gi) {
-                        if (16 * gi < ncols) {
-                            float v[16];
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) v[j] = run[16 * gi + j];
-                            tmem_st16(acc + 16u * gi, v);
-                        }
-                    }
-                    tmem_wait_st();
-                    last_acc = acc;
-                    last_a = a;
-                }
-            }
-            gch += (uint32_t)nchunks;
-            if (!ok) break;
-            auto release_last = [&]() {
+                return ok;
+            };
+            auto release_sums = [&]() {
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(acc_empty_bar(last_a));
+                if (lane == 0) mbar_arrive(fin_empty);
             };
             if (ncols <= 0) {
-                release_last();
+                if (wait_sums()) release_sums();
                 continue;
             }
 
-            // ---- fused epilogue, reading the sums back 8 columns at a time:
+            // ---- fused epilogue, reading the sums 16 columns at a time:
             //   S = (1 - lam) B + lam * rs_inv[row] * cs_inv[k] * acc
             //   Ibar' = 0.5 Ibar + 0.5 rs[row] * S   (relaxation, split again)
             const int64_t r = (int64_t)m_tile * G_BM + q * 32 + lane;
             const int64_t Nc = P.N, ld = P.ldS;
             const int Mout = P.Mout;
             const bool in_row = r < P.rows;
-            const int64_t grp = in_row ? r / Nc : 0;
+            const int64_t grp = in_row ? divide(r, Nc) : 0;
             const int64_t cc = in_row ? r - grp * Nc : 0;
             const bool fp16 = P.fp16 != 0;
             // the energy instantiation runs relaxed source-iteration steps only
             const bool relax = kEnergy || P.relax != 0, residual = kEnergy || P.residual != 0;
-            const float* __restrict__ cs_inv = P.cs_inv;
             const bool has_B = kEnergy || P.B != nullptr;
-            const float lam = (in_row && has_B) ? P.lam[grp] : 1.0f;
-            const float lr = lam * ((fp16 && in_row) ? P.rs_inv[r] : 1.0f);
-            const float bterm = (in_row && has_B) ? (1.0f - lam) * P.B[r] : 0.0f;
-            const float hrsc = 0.5f * ((fp16 && in_row) ? P.rs[r] : 1.0f);
             const bool want_rel = kEnergy || (relax && P.S64 == nullptr);  // relax implies Mout == M <= kpad
+            // the row's parameters: loads only, used once the sums are there
+            const float r_lam = (in_row && has_B) ? P.lam[grp] : 1.0f;
+            const float r_inv = (fp16 && in_row) ? P.rs_inv[r] : 1.0f;
+            const float r_B = (in_row && has_B) ? P.B[r] : 0.0f;
+            const float r_rs = (fp16 && in_row) ? P.rs[r] : 1.0f;
             // energy-conservation correction (relaxed steps): this cell's delta
             // from the previous step; the partial sums of this one.
             const bool ewarp = kEnergy && want_rel && P.part != nullptr;
-            const float qrow = (ewarp && in_row) ? energy_scale(P, r, fp16) : 0.0f;
-            const bool cons = qrow > 0.0f;
-            const float bias = P.bias + (cons ? P.delta[r] : 0.0f);
+            const float r_q = (ewarp && in_row) ? energy_scale(P, r, fp16) : 0.0f;
+            const float r_delta = (ewarp && in_row) ? P.delta[r] : 0.0f;
             // the partial sums: sum_k raw_k in fixed point, and the raw value
             // of the extra column Mout (sum_j (v_j - c) raw_j) where this warp
             // holds it; group_energy_kernel derives sum_j v_j S_j from them
             int th = 0, tl = 0;
             float raw_e = 0.0f;
-            const int kbase = n_tile * bn + sw * cs;
+            const int kbase = n_tile * P.bn + sw * cs;
             float* __restrict__ S = P.S32 ? P.S32 + grp * (int64_t)Mout * ld + cc : nullptr;
             // (the energy instantiation runs relaxed source iterations, whose output is S32)
             double* __restrict__ S64 = (!kEnergy && P.S64) ? P.S64 + grp * (int64_t)Mout * ld + cc : nullptr;
-            // The relaxation's split rows move by TMA in units of 16 B hi and
-            // 16 B lo of each of the warp's 32 rows (8 columns of a 16-bit
-            // split, 4 of a TF32 split): a 2-D box load into one of two
-            // shared-memory buffers per warp, one unit ahead, and after the
-            // update a box store back into the other ping-pong buffer.  A buffer
-            // is refilled only once the store that read it has finished reading
-            // (rows 4*kpad bytes apart would otherwise cost a line per lane on
-            // every access).
+            // the column unscales of this warp's columns, a column per lane
+            float cs_lane[(G_BN / G_SLICES + 31) / 32];
+#pragma unroll
+            for (int j = 0; j < (G_BN / G_SLICES + 31) / 32; ++j)
+                cs_lane[j] = fp16 && 32 * j + lane < ncols ? __ldg(P.cs_inv + kbase + 32 * j + lane) : 1.0f;
+            // The relaxation's split rows move by TMA in units of 32 B hi and
+            // 32 B lo of each of the warp's 32 rows (16 columns of a 16-bit
+            // split, 8 of a TF32 split): a box load into one of two shared-memory
+            // buffers per warp, one unit ahead, and after the update a box store
+            // back into the other ping-pong buffer (rows 4*kpad bytes apart would
+            // otherwise cost a line per lane on every access).
             float rmax = 0.0f;
             bool overflow = false;
             // the steps, compiled once per split format (columns per relaxation unit)
             auto run_steps = [&](auto tf32c) {
                 constexpr bool tf32 = decltype(tf32c)::value;
-                constexpr int ucols = tf32 ? 4 : 8;
+                constexpr int ucols = tf32 ? 8 : 16, ublock = tf32 ? 4 : 5;  // columns per unit, log2 of a block's
                 const int row0 = m_tile * G_BM + q * 32;
                 const void* map_in = &P.mapR[P.cur];
                 const void* map_out = &P.mapR[P.cur ^ 1];
                 // units of this warp's columns that hold outputs
                 const int u_real = want_rel ? max(0, min(ncols, Mout - kbase) + ucols - 1) / ucols : 0;
-                auto unit_x = [&](int u) {  // box column (16-bit units) of unit u's high parts
-                    const int k0 = kbase + u * ucols;
-                    return tf32 ? (k0 >> 4) * 64 + (k0 & 15) * 2 : (k0 >> 5) * 64 + (k0 & 31);
-                };
+                auto unit_x = [&](int k0) { return (k0 & ((1 << ublock) - 1)) * (tf32 ? 2 : 1); };
+                auto unit_z = [&](int k0) { return (k0 >> ublock) * 2; };
                 int u_next = 0;  // next unit to fetch
-                auto pump = [&](int u_cons) {  // keep G_REL_NB - 1 units fetched beyond the one being consumed
-                    while (u_next < u_real && u_next <= u_cons + (G_REL_NB - 1)) {
+                // fetches up to unit u_max, once the store that last read its buffer has done so
+                auto pump = [&](int u_max) {
+                    for (; u_next < u_real && u_next <= u_max; ++u_next, ++rel_issued) {
                         if (lane == 0) {
-                            const uint32_t b = rel_issued % G_REL_NB, dst = rbuf_s + b * 1024u;
-                            const int x = unit_x(u_next);
-                            bulk_wait_read0();  // the store that last read this buffer
-                            mbar_expect_tx(rel_bar(ew, b), 1024);
-                            tma_load_2d(dst, map_in, x, row0, rel_bar(ew, b));
-                            tma_load_2d(dst + 512u, map_in, x + 32, row0, rel_bar(ew, b));
+                            const uint32_t b = rel_issued % G_REL_NB;
+                            const int k0 = kbase + u_next * ucols;
+                            bulk_wait_read0();
+                            mbar_expect_tx(rel_bar(ew, b), G_REL_BYTES);
+                            tma_load_3d(rbuf_s + b * G_REL_BYTES, map_in, unit_x(k0), row0, unit_z(k0), rel_bar(ew, b));
                         }
-                        ++rel_issued;
-                        ++u_next;
                     }
                 };
-                // previous S of a block of 8 columns, loaded one block ahead
-                auto load_old = [&](int e0, float (&o)[8]) {
+                // previous S of a block of 16 columns, loaded one block ahead
+                float old[16];
+                auto load_old = [&](int e0) {
                     const int k0 = kbase + e0;
-                    const int nk = min(8, Mout - k0);
-                    if (in_row && nk > 0 && residual && S && e0 < ncols) {
-                        const float* sp = S + (int64_t)k0 * ld;
-    #pragma unroll
-                        for (int j = 0; j < 8; ++j, sp += ld) o[j] = j < nk ? *sp : 0.0f;
-                    } else {
-    #pragma unroll
-                        for (int j = 0; j < 8; ++j) o[j] = 0.0f;
-                    }
+                    const int nk = e0 < ncols ? min(16, Mout - k0) : 0;
+                    const bool on = in_row && residual && S;
+                    const float* sp = S + (int64_t)k0 * ld;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j, sp += ld) old[j] = on && j < nk ? *sp : 0.0f;
                 };
-                float old_next[8];
-                load_old(0, old_next);
-                pump(-1);
-    #pragma unroll 1
-                for (int e0 = 0; e0 < ncols; e0 += 8) {
+                pump(0);
+                if (!wait_sums()) return;
+                const float lr = r_lam * r_inv, bterm = (1.0f - r_lam) * r_B, hrsc = 0.5f * r_rs;
+                const float qrow = r_q;
+                const bool cons = qrow > 0.0f;
+                const float bias = P.bias + (cons ? r_delta : 0.0f);
+                load_old(0);
+#pragma unroll 1
+                for (int e0 = 0; e0 < ncols; e0 += 16) {
                     const int k0 = kbase + e0;
-                    const int nk = min(8, Mout - k0);  // valid columns of this block (same for all lanes)
+                    const int nk = min(16, Mout - k0);  // valid columns of this block (same for all lanes)
                     const bool live_k = in_row && nk > 0;
-                    float old[8];
-    #pragma unroll
-                    for (int j = 0; j < 8; ++j) old[j] = old_next[j];
-                    load_old(e0 + 8, old_next);
-                    float cin[8];
-                    if (fp16) {
-                        const float4 c0 = __ldg(reinterpret_cast<const float4*>(cs_inv + k0));
-                        const float4 c1 = __ldg(reinterpret_cast<const float4*>(cs_inv + k0) + 1);
-                        cin[0] = c0.x, cin[1] = c0.y, cin[2] = c0.z, cin[3] = c0.w;
-                        cin[4] = c1.x, cin[5] = c1.y, cin[6] = c1.z, cin[7] = c1.w;
-                    } else {
-    #pragma unroll
-                        for (int j = 0; j < 8; ++j) cin[j] = 1.0f;
-                    }
-                    float v[8];
-                    tmem_ld8(last_acc + (uint32_t)e0, v);
-                    float snew[8];
-                    float eb = 0.0f;  // these columns' raw integrals, in column order
-    #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float raw = v[j] * cin[j];  // cin is a power of two: exact
-                        snew[j] = fmaf(fmaf(raw, bias, raw), lr, bterm);
-                        if (kEnergy && j < nk) eb += raw;
+                    float v[16];
+                    tmem_ld16(fin + (uint32_t)e0, v);
+                    if (e0 + 16 >= ncols) release_sums();
+                    float eb[2] = {0.0f, 0.0f};  // raw integrals of 8 columns each, in column order
+                    const float cl = e0 < 32 ? cs_lane[0] : e0 < 64 ? cs_lane[1] : cs_lane[2];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        // the unscale is a power of two: exact
+                        const float raw = v[j] * __shfl_sync(0xffffffffu, cl, (e0 & 31) + j);
+                        v[j] = fmaf(fmaf(raw, bias, raw), lr, bterm);
+                        if (kEnergy && j < nk) eb[j >> 3] += raw;
                         if (kEnergy && j == nk) raw_e = raw;  // column Mout (one block of one warp)
                     }
                     // blocks of 8 columns start at multiples of 8 of the out-directions
-                    if (kEnergy && cons && live_k) fixed_add(eb * qrow, th, tl);
+                    if (kEnergy && cons && live_k) {
+                        fixed_add(eb[0] * qrow, th, tl);
+                        if (nk > 8) fixed_add(eb[1] * qrow, th, tl);
+                    }
                     if (live_k) {
                         if (S64) {
                             double* dp = S64 + (int64_t)k0 * ld;
-    #pragma unroll
-                            for (int j = 0; j < 8; ++j, dp += ld)
-                                if (j < nk) *dp = (double)snew[j];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j, dp += ld)
+                                if (j < nk) *dp = (double)v[j];
                         } else {
                             float* sp = S + (int64_t)k0 * ld;
-    #pragma unroll
-                            for (int j = 0; j < 8; ++j, sp += ld)
+#pragma unroll
+                            for (int j = 0; j < 16; ++j, sp += ld)
                                 if (j < nk) {
-                                    *sp = snew[j];
-                                    rmax = fmaxf(rmax, fabsf(snew[j] - old[j]));
+                                    *sp = v[j];
+                                    rmax = fmaxf(rmax, fabsf(v[j] - old[j]));
                                 }
                         }
                     }
-                    // fetch one unit ahead only now: the buffer it fills was read by
-                    // the previous step's store, which has had the TMEM read and the
-                    // S stores above to finish, so lane 0 rarely waits on it
-                    pump(e0 / ucols);
-                    // this step's units: wait for the load, relax this lane's row in
+                    load_old(e0 + 16);
+                    // this block's units: wait for the load, relax this lane's row in
                     // place (rows outside the problem stay unchanged), store the box
                     // into the other ping-pong buffer
                     bool stop = false;
-                    for (int ui = 0; ui < 8 / ucols; ++ui) {
+#pragma unroll
+                    for (int ui = 0; ui < 16 / ucols; ++ui) {
                         const int u = e0 / ucols + ui;
                         if (u >= u_real) break;
+                        // the buffer was read by the previous unit's store, issued before the
+                        // TMEM read and the S stores above
+                        pump(u + 1);
                         const uint32_t b = rel_used % G_REL_NB;
                         const bool got =
                             mbar_wait(rel_bar(ew, b), (rel_used / G_REL_NB) & 1u, flag, FLAG_WAIT_EPILOGUE);
@@ -611,30 +623,31 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                             stop = true;
                             break;
                         }
-                        uint8_t* rb = rbuf + b * 1024u;
-                        const int nku = min(ucols, Mout - (kbase + u * ucols));
+                        uint8_t* hi = rbuf + b * G_REL_BYTES + 32 * lane;
+                        uint8_t* lo = hi + G_REL_BYTES / 2;
+                        const int ku = kbase + u * ucols;
                         if (in_row) {
-                            if (tf32) {
-                                relax4_tf32(reinterpret_cast<float4*>(rb + 16 * lane),
-                                            reinterpret_cast<float4*>(rb + 512 + 16 * lane), snew + 4 * ui, hrsc, nku);
-                            } else {
-                                uint4* hp = reinterpret_cast<uint4*>(rb + 16 * lane);
-                                uint4* lp = reinterpret_cast<uint4*>(rb + 512 + 16 * lane);
-                                if (fp16)
-                                    overflow |= relax8<true>(hp, lp, snew, hrsc, nku);
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {  // 16 bytes of each part
+                                const int nku = min(ucols / 2, Mout - ku - h * (ucols / 2));
+                                const float* x = v + ui * ucols + h * (ucols / 2);
+                                if (tf32)
+                                    relax4_tf32(reinterpret_cast<float4*>(hi) + h, reinterpret_cast<float4*>(lo) + h, x,
+                                                hrsc, nku);
+                                else if (fp16)
+                                    overflow |= relax8<true>(reinterpret_cast<uint4*>(hi) + h,
+                                                             reinterpret_cast<uint4*>(lo) + h, x, hrsc, nku);
                                 else
-                                    relax8<false>(hp, lp, snew, hrsc, nku);
+                                    relax8<false>(reinterpret_cast<uint4*>(hi) + h, reinterpret_cast<uint4*>(lo) + h, x,
+                                                  hrsc, nku);
                             }
                         }
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) {
-                            const int x = unit_x(u);
-                            tma_store_2d(map_out, x, row0, rbuf_s + b * 1024u);
-                            tma_store_2d(map_out, x + 32, row0, rbuf_s + b * 1024u + 512u);
+                            tma_store_3d(map_out, unit_x(ku), row0, unit_z(ku), rbuf_s + b * G_REL_BYTES);
                             bulk_commit();
                         }
-                        pump(u);
                     }
                     if (stop) {
                         ok = false;
@@ -646,10 +659,10 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                 run_steps(std::true_type{});
             else
                 run_steps(std::false_type{});
-            release_last();
-            if (kEnergy && ewarp && in_row && ok) {  // this slot's partial sums (zero: no correction)
-                const int64_t slot = (int64_t)n_tile * 4 + cs;
-                P.part[slot * (P.m_tiles * (int64_t)G_BM) + r] = make_int4(cons ? __float_as_int(raw_e) : 0, 0, th, tl);
+            if (!ok) break;
+            if (kEnergy && ewarp && in_row) {  // this slot's partial sums (zero: no correction)
+                const int64_t slot = (int64_t)n_tile * G_SLICES + cs;
+                P.part[slot * (P.m_tiles * (int64_t)G_BM) + r] = make_int4(r_q > 0.0f ? __float_as_int(raw_e) : 0, 0, th, tl);
             }
             if (overflow) atomicOr(flag, FLAG_SCALE_OVERFLOW);
             if (residual) {
@@ -659,7 +672,10 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                     atomicMax(P.resid, (unsigned long long)__double_as_longlong((double)rmax));
             }
         }
-        if (lane == 0) bulk_wait0();  // the relaxation's stores are complete before the CTA exits
+        // no copy may still be in flight when the CTA exits (loads are left only by a wait that gave up)
+        for (; rel_used < rel_issued; ++rel_used)
+            mbar_wait(rel_bar(ew, rel_used % G_REL_NB), (rel_used / G_REL_NB) & 1u, flag, FLAG_WAIT_EPILOGUE);
+        if (lane == 0) bulk_wait0();
     }
     tc_fence_before();
     __syncthreads();
@@ -684,9 +700,9 @@ __global__ void group_energy_kernel(const GroupProblem* __restrict__ probs, int 
         long long et = 0;  // exact: in units of 2^-22 of the row's quantum
         float raw_e = 0.0f;  // held by one slot, zero in the others
         for (int nt = 0; nt < P.n_tiles; ++nt)
-            for (int cs = 0; cs < 4; ++cs) {
+            for (int cs = 0; cs < G_SLICES; ++cs) {
                 if (P.sw * cs >= P.bn) continue;  // a column slice without columns
-                const int4 v = P.part[((int64_t)nt * 4 + cs) * ld + r];
+                const int4 v = P.part[((int64_t)nt * G_SLICES + cs) * ld + r];
                 raw_e += __int_as_float(v.x);
                 et += ((long long)v.z << 22) + v.w;
             }

@@ -87,14 +87,23 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, int x
         : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, int x, int y, int z, uint32_t bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+}
+
 // Bulk tensor store of a shared-memory box to global memory (bulk-group
 // completion), its commit, and the waits: until the sources have been read
 // (the shared memory may be reused) or until the writes are done.
-__device__ __forceinline__ void tma_store_2d(const void* map, int x, int y, uint32_t src)
+__device__ __forceinline__ void tma_store_3d(const void* map, int x, int y, int z, uint32_t src)
 {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
                      reinterpret_cast<uint64_t>(map)),
-                 "r"(x), "r"(y), "r"(src)
+                 "r"(x), "r"(y), "r"(z), "r"(src)
                  : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
@@ -119,28 +128,42 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate)
+// tcgen05.mma from the low words of the descriptors of smem_desc_sw128 (their
+// high word, the swizzle, version and stride fields, is the same for all):
+// kind::f16 (K = 16) or kind::tf32 (K = 8), 32 bytes of each row either way.
+constexpr uint32_t DESC_HI = (uint32_t)((((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
+template <bool kTf32>
+__device__ __forceinline__ void umma_lo(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t accumulate)
 {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    if (kTf32)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
+            "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(DESC_HI)
+            : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+            "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
+            "r"(a), "r"(b), "r"(idesc), "r"(accumulate), "r"(DESC_HI)
+            : "memory");
 }
 
-// tcgen05.mma kind::tf32 (K = 8 per instruction: 32 bytes of each row, the
-// same bytes as one kind::f16 step).
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate)
+// Register shares of a kernel's warpgroups (their sum over threads must stay
+// within what the block was launched with).
+template <int kRegs>
+__device__ __forceinline__ void reg_dec()
 {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
+}
+template <int kRegs>
+__device__ __forceinline__ void reg_inc()
+{
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
 }
 
 __device__ __forceinline__ void umma_commit(uint32_t bar)

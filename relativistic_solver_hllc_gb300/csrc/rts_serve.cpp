@@ -95,12 +95,12 @@ int wait_event(rts_ctx* ctx, cudaEvent_t ev, int64_t timeout_us)
 }
 
 // Solve time of a request alone: per step a fixed launch and host overhead
-// plus its tiles in waves over the SMs, each tile taking about 1 us per
-// 32-direction K-slice (two issuers, measured on GB300 at N = 256 columns).
+// plus its tiles in waves over the SMs, each tile taking about 0.5 us per
+// 32-direction K-slice (measured on GB300 at N = 144 columns).
 double isolated_estimate(int64_t tiles, int64_t M, int iterations, int num_sms)
 {
     const double waves = std::ceil((double)tiles / (double)num_sms);
-    const double tile_s = 1.0e-6 * (double)((M + 31) / 32);
+    const double tile_s = 0.5e-6 * (double)((M + 31) / 32);
     return (double)iterations * (30e-6 + waves * tile_s);
 }
 

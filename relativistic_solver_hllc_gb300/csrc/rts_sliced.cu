@@ -80,17 +80,6 @@ constexpr int S_REGS = 96, S_REGS_ISSUE = 32, S_REGS_DRAIN = 112;
 static_assert(S_DRAIN_WARP0 * S_REGS_ISSUE + S_DRAIN_WARPS * S_REGS_DRAIN <=
                   (S_DRAIN_WARP0 + S_DRAIN_WARPS) * S_REGS,
               "the register split within the launch's registers");
-template <int kRegs>
-__device__ __forceinline__ void reg_dec()
-{
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs));
-}
-template <int kRegs>
-__device__ __forceinline__ void reg_inc()
-{
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegs));
-}
-
 struct SlicedArgs {
     int64_t n;               // cells
     int64_t ld;              // row pitch of S in cells
@@ -107,20 +96,6 @@ struct SlicedArgs {
     unsigned long long* resid;
     int* flag;
 };
-
-// tcgen05.mma from the descriptors' low words (the high word is the same for
-// all: the swizzle, version and stride fields).
-constexpr uint32_t DESC_HI = (uint32_t)((((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61)) >> 32);
-__device__ __forceinline__ void umma(uint32_t acc, uint32_t a, uint32_t w, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 da, dw;\n\t"
-        "mov.b64 da, {%1, %5};\n\tmov.b64 dw, {%2, %5};\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, dw, %3, p;\n\t}" ::"r"(acc),
-        "r"(a), "r"(w), "r"(idesc), "r"(accumulate), "r"(DESC_HI)
-        : "memory");
-}
 
 // The total's unit is 2^-UNIT_BITS of 2^(e_c + e_k): that of D_4.
 constexpr int UNIT_BITS = 2 * (rts_rows::SLICE_BITS - 45) + 36;
@@ -295,8 +270,8 @@ sliced_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
                         for (int i = 0; i <= d; ++i) {
                             const uint32_t a = A + (uint32_t)((i >> 1) * (S_BOX >> 4) + (i & 1) * 4);
                             const uint32_t w = W + (uint32_t)(((d - i) >> 1) * (S_BOX >> 4) + ((d - i) & 1) * 4);
-                            umma(acc, a, w, idesc, i != 0 ? 1u : 0u);
-                            umma(acc, a + 2, w + 2, idesc, 1u);
+                            umma_lo<false>(acc, a, w, idesc, i != 0 ? 1u : 0u);
+                            umma_lo<false>(acc, a + 2, w + 2, idesc, 1u);
                         }
                         if (d + 2 >= SLICES) umma_commit(empty_bar(s));  // the chunk's last MMAs of this issuer
                         umma_commit(acc_full(slot));

@@ -8,7 +8,7 @@
 //   * drain period: those the accuracy rule allows (rts_auto_flush: FP16 and
 //     BF16 one K-slice, or one and two for smooth kernels; TF32 two);
 //   * tile width: every distinct tiling of the out-directions (n tiles of
-//     bn = 16 ceil(M / (16 n)) directions, bn from 64 to 256);
+//     bn = 16 ceil(M / (16 n)) directions, bn from 64 to 160);
 //   * tile order: the column tiles of a row tile in turn (a 128-row slab of
 //     the split Ibar is read from DRAM once while its column tiles run side
 //     by side on neighbouring SMs), or the row tiles of a column tile in turn.
@@ -16,8 +16,8 @@
 // table, keyed by (M, precision, drain period, cell bucket).  A problem then
 // takes -- unless its caller fixes them -- the drain period with the shorter
 // tuned time among those its own kernel allows (rts_tuned_flush), and that
-// period's width and order (rts_tuned_tile), from the entry of the nearest
-// cell bucket.  Width and order do not change any output's arithmetic (each
+// period's width and order (rts_tuned_tile), or those of the other period if
+// its own was not timed, from the entry of the nearest cell bucket.  Width and order do not change any output's arithmetic (each
 // output is summed over the same K-slices in the same order), so they give
 // bit-identical results; the drain period changes the rounding, within the
 // accuracy the rule guarantees.  rts_autotune is the width-only search at one
@@ -97,13 +97,14 @@ int auto_period(int64_t M, int precision)
 std::vector<int> widths(int64_t M)
 {
     std::vector<int> cand;
-    for (int64_t nt = (M + 255) / 256; nt <= (M + 63) / 64; ++nt) {
+    constexpr int64_t most = 160;  // the kernel's widest tile
+    for (int64_t nt = (M + most - 1) / most; nt <= (M + 63) / 64; ++nt) {
         const int bn = (int)(((M + nt - 1) / nt + 15) / 16 * 16);
-        if (bn > 256 || bn < 16) continue;
+        if (bn > most || bn < 16) continue;
         if (std::find(cand.begin(), cand.end(), bn) == cand.end()) cand.push_back(bn);
         if (cand.size() >= 8) break;
     }
-    if (cand.empty()) cand.push_back((int)std::min<int64_t>(256, (M + 15) / 16 * 16));
+    if (cand.empty()) cand.push_back((int)std::min<int64_t>(most, (M + 15) / 16 * 16));
     return cand;
 }
 
@@ -180,7 +181,10 @@ int rts_tuned_flush(const rts_ctx* ctx, int64_t M, int precision, int64_t rows, 
 
 bool rts_tuned_tile(const rts_ctx* ctx, int64_t M, int mode, int flush, int64_t rows, int* bn, int* order)
 {
-    const rts_tune_entry* e = match(ctx, M, mode_precision(mode), std::max(flush, 1), rts_cells_bucket(ctx, rows));
+    const int bucket = rts_cells_bucket(ctx, rows);
+    const rts_tune_entry* e = match(ctx, M, mode_precision(mode), std::max(flush, 1), bucket);
+    // a period that was not timed takes the schedule of one that was
+    if (!e) e = match(ctx, M, mode_precision(mode), 3 - std::max(flush, 1), bucket);
     if (!e) return false;
     *bn = e->bn;
     *order = e->order;
