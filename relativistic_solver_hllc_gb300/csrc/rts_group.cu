@@ -116,6 +116,9 @@ struct rts_batch {
 
 namespace {
 
+// the slots' partial sums and the extra column of every row
+size_t part_bytes(const GProb* p) { return (size_t)p->rows_pad * ((size_t)p->n_tiles * G_SLICES * 8 + 4); }
+
 // frees are stream-ordered: after the work already queued on `st`
 void free_prob(rts_ctx* ctx, GProb* p, cudaStream_t st)
 {
@@ -129,7 +132,7 @@ void free_prob(rts_ctx* ctx, GProb* p, cudaStream_t st)
     rts_pfree(ctx, p->lam, (size_t)(p->groups * 4), st);
     rts_pfree(ctx, p->S32, (size_t)(p->rows * p->Mout * 4), st);
     rts_pfree(ctx, p->vrow, (size_t)((p->kpad + 4) * 4), st);
-    rts_pfree(ctx, p->part, (size_t)(p->n_tiles * G_SLICES * p->rows_pad * 16), st);
+    rts_pfree(ctx, p->part, part_bytes(p), st);
     rts_pfree(ctx, p->delta, (size_t)(p->rows_pad * 4), st);
     rts_pfree(ctx, p->ex, (size_t)(p->rows_pad * 8), st);
     delete p;
@@ -173,7 +176,7 @@ float rts_group_bias(const rts_ctx* ctx, int, int)
 
 int64_t rts_group_energy_bytes(int64_t kpad, int64_t rows_pad, int n_tiles)
 {
-    return (kpad + 4) * 4 + (int64_t)n_tiles * G_SLICES * rows_pad * 16 + rows_pad * 12;
+    return (kpad + 4) * 4 + (int64_t)n_tiles * G_SLICES * rows_pad * 8 + rows_pad * 16;
 }
 
 // Tile geometry of a problem: out-direction tiles of at most G_BN, balanced.
@@ -272,7 +275,7 @@ int rts_group_new_problem(rts_batch* b, int64_t N, int64_t Min, int64_t Mout, in
     }
     if (energy) {
         GP_ALLOC(vrow, (size_t)((p->kpad + 4) * 4), "W row sums");
-        GP_ALLOC(part, (size_t)(p->n_tiles * G_SLICES * p->rows_pad * 16), "energy partial sums");
+        GP_ALLOC(part, part_bytes(p), "energy partial sums");
         GP_ALLOC(delta, (size_t)(p->rows_pad * 4), "energy corrections");
         GP_ALLOC(ex, (size_t)(p->rows_pad * 8), "conserved sums");
     }
@@ -426,7 +429,8 @@ static void fill_entry(rts_batch* b, GProb* p, int relax, size_t i, int64_t& til
     // applies to relaxed steps (a step without relaxation leaves the input)
     const bool energy = p->part != nullptr && ctx->split_bias >= 0 && relaxes(p, relax);
     g.vrow = energy ? p->vrow : nullptr;
-    g.part = energy ? reinterpret_cast<int4*>(p->part) : nullptr;
+    g.part = energy ? reinterpret_cast<int2*>(p->part) : nullptr;
+    g.extra = energy ? reinterpret_cast<float*>(g.part + (int64_t)p->n_tiles * G_SLICES * p->rows_pad) : nullptr;
     g.delta = energy ? p->delta : nullptr;
     g.ex = energy ? p->ex : nullptr;
     g.rsb = p->rs;

@@ -41,7 +41,7 @@ struct GProb {
     size_t bytes = 0;
     // energy-conservation correction of relaxed steps (iterative problems)
     float* vrow = nullptr;   // [kpad + 4] v_j = sum_k W[j][k]; then the quantum scale, c, D, 1/c (rts_pp_w_stats)
-    void* part = nullptr;    // [n_tiles * 4][rows_pad] int4 per-slot partial sums of a step (fixed point)
+    void* part = nullptr;    // per-slot partial sums of a step (fixed point), then the rows' extra column
     float* delta = nullptr;  // [rows_pad] per-row correction of the next step
     double* ex = nullptr;    // [rows_pad] sum_j v_j x_j of the current input (fixed-point quanta)
     alignas(64) unsigned char maps[3][128];

@@ -12,10 +12,13 @@
 // finished sums of the tile before, which warps of their own work on.  (With
 // 256-column tiles there was no room: the warps that drained also ran the
 // epilogue while the tensor cores waited, 1.29 ms a step of 162,000 x 1,000 in
-// FP16, 0.72 of them in the contraction; now 0.89.  Tensor-core time 0.5 ms,
-// HBM 0.4 ms.  The contraction alone takes 0.66 ms: M = 128, N = 144 MMAs run
-// at 0.65 of their rate, bound by the operands' way through shared memory; the
-// epilogue warps' latency is the rest.)
+// FP16; now 0.82.  Tensor-core time 0.5 ms, HBM 0.4 ms.  The contraction alone
+// takes 0.62 ms: an accumulator is used again after its chunk's MMAs, the
+// drain and the hand-overs between the warps; the epilogue warps' instruction
+// fetch and latency are the rest.  Three accumulators of 128 columns instead:
+// the copies from L2 take as long as the MMAs, 0.81; with the pair of an SM's
+// neighbours on one MMA (cta_group::2) as well, 0.77, but 0.3 more for a queue
+// of small problems.)
 //
 // Warp roles (20 warps, 640 threads, one CTA per SM):
 //   warp 0       TMA producer: A (split Ibar rows) and B (split W rows)
@@ -32,7 +35,7 @@
 //                each accumulate) and release it; a finished tile's sums go
 //                to their own TMEM columns;
 //   warps 12..19 epilogue (unscaling, source update, residual, S store,
-//                relaxation of Ibar in split form) of those sums, 16 columns
+//                relaxation of Ibar in split form) of those sums, 8 columns
 //                at a time.
 // The drain warps hold 80 sums a thread: the first warpgroup gives them its
 // registers.
@@ -70,27 +73,30 @@
 #include <type_traits>
 
 constexpr int G_BM = 128;
-constexpr int G_BN = 160;    // at most: two accumulators and the finished sums in 512 TMEM columns
+constexpr int G_BN = 160;    // at most: the accumulators and the finished sums in 512 TMEM columns
+constexpr int G_ACCS = 2;    // accumulators
 constexpr int G_STAGES = 5;
 constexpr int G_A_BYTES = G_BM * 128;
 constexpr int G_B_BYTES = G_BN * 128;
 constexpr int G_STAGE_BYTES = G_A_BYTES + G_B_BYTES;
-constexpr int G_SLICES = 2;  // column slices of a tile, one per warpgroup
-constexpr int G_DRAIN_WARP0 = 4, G_EPI_WARP0 = 12;
-constexpr int G_EPI_WARPS = 4 * G_SLICES;
+constexpr int G_SLICES = 2;  // column slices of a tile: a warpgroup drains each, another runs its epilogue
+constexpr int G_DRAIN_WARP0 = 4, G_DRAIN_WARPS = 4 * G_SLICES;
+constexpr int G_EPI_WARP0 = G_DRAIN_WARP0 + G_DRAIN_WARPS, G_EPI_WARPS = 4 * G_SLICES;
+constexpr int G_COLS = G_BN / G_SLICES;  // columns of a slice, at most (a multiple of 16)
 constexpr int G_THREADS = (G_EPI_WARP0 + G_EPI_WARPS) * 32;
-// registers a thread: 96 at launch; the first warpgroup gives 64 of them to the two that drain
-constexpr int G_REGS_ISSUE = 32, G_REGS_DRAIN = 128;
-static_assert(G_REGS_ISSUE + 2 * G_REGS_DRAIN + 2 * 96 <= 5 * 96, "registers of the block");
+// registers a thread: G_REGS at launch; the first warpgroup gives most of its
+// own to the two that drain.  Fewer than 40 for it spill in the issuing loop.
+constexpr int G_REGS = 96, G_REGS_ISSUE = 40, G_REGS_DRAIN = 120;
+static_assert(G_REGS_ISSUE + 2 * G_REGS_DRAIN + 2 * G_REGS <= 5 * G_REGS, "registers of the block");
 constexpr int G_CTAS_PER_SM = 1;
 constexpr uint32_t G_TMEM_COLS = 512;
-constexpr uint32_t G_FIN = 2 * G_BN;  // TMEM column of the finished sums
-constexpr int G_MAX_FLUSH = 2;        // K-slices per chunk
+constexpr uint32_t G_FIN = G_ACCS * G_BN;  // TMEM column of the finished sums
+constexpr int G_MAX_FLUSH = 2;             // K-slices per chunk
 constexpr int G_REL_NB = 2;           // relaxation row buffers per epilogue warp
 constexpr int G_REL_BYTES = 2048;     // 32 rows x 32 B hi, then 32 rows x 32 B lo
 // ring, accumulator and hand-over barriers (the relaxation's from index
 // G_REL_BAR), then the TMEM address
-constexpr int G_REL_BAR = 2 * G_STAGES + 6;
+constexpr int G_REL_BAR = 2 * G_STAGES + 2 * G_ACCS + 2;
 constexpr int G_BAR_BYTES = (8 * (G_REL_BAR + 1 + G_REL_NB * G_EPI_WARPS) + 127) / 128 * 128;
 constexpr int G_REL_BUF = G_REL_NB * G_REL_BYTES;
 constexpr size_t G_REL_OFF = (size_t)G_STAGES * G_STAGE_BYTES + G_BAR_BYTES;
@@ -130,8 +136,8 @@ struct GroupProblem {  // aligned as its CUtensorMap members
     const float* vrow;    // [kpad + 4] v_j = sum_k W[j][k], 0 past M; vrow[kpad] = q0 (below), then c, D, 1/c:
                           // c the mean of the v_j, D = sum_j (v_j - c); output column Mout holds
                           // sum_j (v_j - c) raw_j
-    int4* part;           // [n_tiles * G_SLICES][rows_pad] per-slot partials in quanta (high, low parts):
-                          // sum_j v_j rs S_j, then sum_k raw_k
+    int2* part;           // [n_tiles * G_SLICES][rows_pad] sum_k raw_k in quanta (high, low part) per slot
+    float* extra;         // [rows_pad] the raw value of column Mout
     double* ex;           // [rows_pad] sum_j v_j x_j of the current input, in quanta
     float* delta;         // [rows_pad] per-cell correction of the next step (0: none yet)
     const float* rsb;     // [rows_pad] power of two with rsb * 2 max(|Ibar|, |B|) < 2^14 (all modes)
@@ -142,9 +148,9 @@ struct GroupProblem {  // aligned as its CUtensorMap members
 // q0 = 2^(7 - ceil(log2 sum_jk |W_jk|)) comes with vrow; values in the units
 // the epilogue sees are below 2^14 (FP16, scaled) or 2^14 / rsb (BF16,
 // TF32).  0 when out of FP32 range (no correction for the row).
-__device__ __forceinline__ float energy_scale(const GroupProblem& P, int64_t r, bool fp16)
+__device__ __forceinline__ float energy_scale(float q0, float rsb)  // rsb: 1 in FP16 mode
 {
-    const float q = P.vrow[P.kpad] * (fp16 ? 1.0f : P.rsb[r]);
+    const float q = q0 * rsb;
     return (q > 0.0f && q < 3.0e38f) ? q : 0.0f;
 }
 
@@ -245,8 +251,8 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
     auto full_bar = [&](uint32_t s) { return bar_base + 8u * s; };
     auto empty_bar = [&](uint32_t s) { return bar_base + 8u * (G_STAGES + s); };
     auto acc_full_bar = [&](uint32_t a) { return bar_base + 8u * (2 * G_STAGES + a); };
-    auto acc_empty_bar = [&](uint32_t a) { return bar_base + 8u * (2 * G_STAGES + 2 + a); };
-    const uint32_t fin_full = bar_base + 8u * (2 * G_STAGES + 4), fin_empty = fin_full + 8u;
+    auto acc_empty_bar = [&](uint32_t a) { return bar_base + 8u * (2 * G_STAGES + G_ACCS + a); };
+    const uint32_t fin_full = bar_base + 8u * (2 * G_STAGES + 2 * G_ACCS), fin_empty = fin_full + 8u;
     // relaxation row buffers: barrier of buffer b of epilogue warp w
     auto rel_bar = [&](int w, uint32_t b) { return bar_base + 8u * (G_REL_BAR + G_REL_NB * w + (int)b); };
 
@@ -256,11 +262,11 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
-        for (uint32_t a = 0; a < 2; ++a) {
+        for (uint32_t a = 0; a < G_ACCS; ++a) {
             mbar_init(acc_full_bar(a), 1);
-            mbar_init(acc_empty_bar(a), 4 * G_SLICES);
+            mbar_init(acc_empty_bar(a), G_DRAIN_WARPS);
         }
-        mbar_init(fin_full, 4 * G_SLICES);
+        mbar_init(fin_full, G_DRAIN_WARPS);
         mbar_init(fin_empty, G_EPI_WARPS);
         for (int w = 0; w < G_EPI_WARPS; ++w)
             for (int b = 0; b < G_REL_NB; ++b) mbar_init(rel_bar(w, (uint32_t)b), 1);
@@ -312,7 +318,6 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
             // -------------------------------------------------------- MMA issuers
             const uint32_t me = (uint32_t)(warp - 1);
             if (lane == 0 && live) {
-                const uint32_t acc = tmem + G_BN * me;
                 const uint32_t desc0 = (uint32_t)smem_desc_sw128(smem_base);  // low word, stage 0
                 uint32_t gsl = 0, gch = 0;  // K-slice and chunk counters of this CTA (across tiles)
                 bool ok = true;
@@ -323,6 +328,7 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                     // the chunk loop, compiled once per MMA kind
                     auto chunks = [&](auto tf32c) {
                         constexpr bool tf32 = decltype(tf32c)::value;
+                        uint32_t acc = 0;
                         // a K-slice's cross products (32 bytes high, 32 bytes low parts, twice), its hi*hi
                         auto cross = [&](uint32_t a, uint32_t accumulate) {
                             const uint32_t b = a + (G_A_BYTES >> 4);
@@ -338,16 +344,18 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                         };
 #pragma unroll 1
                         for (uint32_t c = (gch ^ me) & 1u; c < nchunks; c += 2) {
-                            const uint32_t g = gch + c, i0 = gsl + c * flush, i1 = i0 + 1;
+                            const uint32_t g = gch + c, a = g % G_ACCS, i0 = gsl + c * flush, i1 = i0 + 1;
                             const bool two = flush > 1 && c * flush + 1 < nkb;
                             const uint32_t s0 = i0 % G_STAGES, s1 = i1 % G_STAGES;
-                            if ((g >= 2 && !mbar_wait(acc_empty_bar(me), ((g >> 1) - 1) & 1, flag, FLAG_WAIT_MMA)) ||
+                            if ((g >= G_ACCS &&
+                                 !mbar_wait(acc_empty_bar(a), (g / G_ACCS - 1) & 1, flag, FLAG_WAIT_MMA)) ||
                                 !mbar_wait(full_bar(s0), (i0 / G_STAGES) & 1, flag, FLAG_WAIT_MMA) ||
                                 (two && !mbar_wait(full_bar(s1), (i1 / G_STAGES) & 1, flag, FLAG_WAIT_MMA))) {
                                 ok = false;
                                 break;
                             }
                             tc_fence_after();
+                            acc = tmem + G_BN * a;
                             const uint32_t a0 = desc0 + s0 * (G_STAGE_BYTES >> 4);
                             const uint32_t a1 = desc0 + s1 * (G_STAGE_BYTES >> 4);
                             // cross products first (the accumulator starts from zero), hi*hi last
@@ -359,7 +367,7 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                                 high(a1);
                                 umma_commit(empty_bar(s1));
                             }
-                            umma_commit(acc_full_bar(me));
+                            umma_commit(acc_full_bar(a));
                         }
                     };
                     if (P.tf32)
@@ -391,27 +399,21 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
             const int sw = P.sw;                          // columns per slice (multiple of 16)
             const int ncols = min(sw, P.bn - sw * cs);    // columns of this warp (multiple of 16; <= 0: none)
             const uint32_t col = lane_off + (uint32_t)(sw * cs);
-            float run[G_BN / G_SLICES];
+            float run[G_COLS];
 #pragma unroll
-            for (int j = 0; j < G_BN / G_SLICES; ++j) run[j] = 0.0f;
+            for (int j = 0; j < G_COLS; ++j) run[j] = 0.0f;
 #pragma unroll 1
             for (int c = 0; c < nchunks; ++c) {
-                const uint32_t g = gch + (uint32_t)c, a = g & 1u;
-                if (!wait(acc_full_bar(a), (g >> 1) & 1)) {
+                const uint32_t g = gch + (uint32_t)c, a = g % G_ACCS;
+                if (!wait(acc_full_bar(a), (g / G_ACCS) & 1)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
                 const uint32_t acc = tmem + G_BN * a + col;
 #pragma unroll
-                for (int j0 = 0; j0 < G_BN / G_SLICES; j0 += 32) {
-                    if (j0 + 32 <= G_BN / G_SLICES && j0 + 32 <= ncols) {
-                        float v[32];
-                        tmem_ld32(acc + (uint32_t)j0, v);
-#pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            if (j0 + j < G_BN / G_SLICES) run[j0 + j] += v[j];
-                    } else if (j0 + 16 <= ncols) {
+                for (int j0 = 0; j0 < G_COLS; j0 += 16) {
+                    if (j0 < ncols) {
                         float v[16];
                         tmem_ld16(acc + (uint32_t)j0, v);
 #pragma unroll
@@ -428,7 +430,7 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
             if (tiles > 0 && !wait(fin_empty, (tiles - 1) & 1)) break;
             tc_fence_after();
 #pragma unroll
-            for (int j0 = 0; j0 < G_BN / G_SLICES; j0 += 16) {
+            for (int j0 = 0; j0 < G_COLS; j0 += 16) {
                 if (j0 < ncols) {
                     float v[16];
 #pragma unroll
@@ -452,8 +454,22 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
         uint32_t rel_issued = 0, rel_used = 0;  // relaxation row blocks fetched / consumed by this warp
         uint32_t tiles = 0;
         bool ok = live;
+        // the largest change over this warp's tiles of a problem
+        float rmax = 0.0f;
+        unsigned long long* resid = nullptr;
+        auto flush_residual = [&]() {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
+            if (lane == 0 && rmax > 0.0f)
+                atomicMax(resid, (unsigned long long)__double_as_longlong((double)rmax));
+            rmax = 0.0f;
+        };
         for (int64_t t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tiles) {
             const GroupProblem& P = probs[find_problem(probs, nprob, t)];
+            if (P.resid != resid) {
+                flush_residual();
+                resid = P.resid;
+            }
             const int sw = P.sw;
             const int ncols = min(sw, P.bn - sw * cs);
             const int64_t lt = t - P.tile_begin + P.tile_off;
@@ -477,7 +493,7 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                 continue;
             }
 
-            // ---- fused epilogue, reading the sums 16 columns at a time:
+            // ---- fused epilogue, reading the sums 8 columns at a time:
             //   S = (1 - lam) B + lam * rs_inv[row] * cs_inv[k] * acc
             //   Ibar' = 0.5 Ibar + 0.5 rs[row] * S   (relaxation, split again)
             const int64_t r = (int64_t)m_tile * G_BM + q * 32 + lane;
@@ -499,8 +515,9 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
             // energy-conservation correction (relaxed steps): this cell's delta
             // from the previous step; the partial sums of this one.
             const bool ewarp = kEnergy && want_rel && P.part != nullptr;
-            const float r_q = (ewarp && in_row) ? energy_scale(P, r, fp16) : 0.0f;
-            const float r_delta = (ewarp && in_row) ? P.delta[r] : 0.0f;
+            const float r_q0 = ewarp ? P.vrow[P.kpad] : 0.0f, r_rsb = (ewarp && in_row && !fp16) ? P.rsb[r] : 1.0f;
+            const float r_delta = (ewarp && in_row) ? P.delta[r] : 0.0f, r_bias = P.bias;
+            float qrow = 0.0f;
             // the partial sums: sum_k raw_k in fixed point, and the raw value
             // of the extra column Mout (sum_j (v_j - c) raw_j) where this warp
             // holds it; group_energy_kernel derives sum_j v_j S_j from them
@@ -511,9 +528,9 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
             // (the energy instantiation runs relaxed source iterations, whose output is S32)
             double* __restrict__ S64 = (!kEnergy && P.S64) ? P.S64 + grp * (int64_t)Mout * ld + cc : nullptr;
             // the column unscales of this warp's columns, a column per lane
-            float cs_lane[(G_BN / G_SLICES + 31) / 32];
+            float cs_lane[(G_COLS + 31) / 32];
 #pragma unroll
-            for (int j = 0; j < (G_BN / G_SLICES + 31) / 32; ++j)
+            for (int j = 0; j < (G_COLS + 31) / 32; ++j)
                 cs_lane[j] = fp16 && 32 * j + lane < ncols ? __ldg(P.cs_inv + kbase + 32 * j + lane) : 1.0f;
             // The relaxation's split rows move by TMA in units of 32 B hi and
             // 32 B lo of each of the warp's 32 rows (16 columns of a 16-bit
@@ -521,7 +538,6 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
             // buffers per warp, one unit ahead, and after the update a box store
             // back into the other ping-pong buffer (rows 4*kpad bytes apart would
             // otherwise cost a line per lane on every access).
-            float rmax = 0.0f;
             bool overflow = false;
             // the steps, compiled once per split format (columns per relaxation unit)
             auto run_steps = [&](auto tf32c) {
@@ -547,111 +563,102 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                         }
                     }
                 };
-                // previous S of a block of 16 columns, loaded one block ahead
-                float old[16];
+                // previous S of a block of 8 columns, loaded one block ahead
+                float old[8];
                 auto load_old = [&](int e0) {
                     const int k0 = kbase + e0;
-                    const int nk = e0 < ncols ? min(16, Mout - k0) : 0;
+                    const int nk = e0 < ncols ? min(8, Mout - k0) : 0;
                     const bool on = in_row && residual && S;
                     const float* sp = S + (int64_t)k0 * ld;
 #pragma unroll
-                    for (int j = 0; j < 16; ++j, sp += ld) old[j] = on && j < nk ? *sp : 0.0f;
+                    for (int j = 0; j < 8; ++j, sp += ld) old[j] = on && j < nk ? *sp : 0.0f;
                 };
                 pump(0);
+                load_old(0);
                 if (!wait_sums()) return;
                 const float lr = r_lam * r_inv, bterm = (1.0f - r_lam) * r_B, hrsc = 0.5f * r_rs;
-                const float qrow = r_q;
+                qrow = in_row ? energy_scale(r_q0, r_rsb) : 0.0f;
                 const bool cons = qrow > 0.0f;
-                const float bias = P.bias + (cons ? r_delta : 0.0f);
-                load_old(0);
+                const float bias = r_bias + (cons ? r_delta : 0.0f);
 #pragma unroll 1
-                for (int e0 = 0; e0 < ncols; e0 += 16) {
+                for (int e0 = 0; e0 < ncols; e0 += 8) {
                     const int k0 = kbase + e0;
-                    const int nk = min(16, Mout - k0);  // valid columns of this block (same for all lanes)
+                    const int nk = min(8, Mout - k0);  // valid columns of this block (same for all lanes)
                     const bool live_k = in_row && nk > 0;
-                    float v[16];
-                    tmem_ld16(fin + (uint32_t)e0, v);
-                    if (e0 + 16 >= ncols) release_sums();
-                    float eb[2] = {0.0f, 0.0f};  // raw integrals of 8 columns each, in column order
-                    const float cl = e0 < 32 ? cs_lane[0] : e0 < 64 ? cs_lane[1] : cs_lane[2];
+                    float v[8];
+                    tmem_ld8(fin + (uint32_t)e0, v);
+                    if (e0 + 8 >= ncols) release_sums();
+                    float eb = 0.0f;  // raw integrals, in column order
+                    const float cl = e0 < 32 ? cs_lane[0] : e0 < 64 ? cs_lane[1] : cs_lane[(G_COLS - 1) / 32];
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) {
+                    for (int j = 0; j < 8; ++j) {
                         // the unscale is a power of two: exact
                         const float raw = v[j] * __shfl_sync(0xffffffffu, cl, (e0 & 31) + j);
                         v[j] = fmaf(fmaf(raw, bias, raw), lr, bterm);
-                        if (kEnergy && j < nk) eb[j >> 3] += raw;
+                        if (kEnergy && j < nk) eb += raw;
                         if (kEnergy && j == nk) raw_e = raw;  // column Mout (one block of one warp)
                     }
                     // blocks of 8 columns start at multiples of 8 of the out-directions
-                    if (kEnergy && cons && live_k) {
-                        fixed_add(eb[0] * qrow, th, tl);
-                        if (nk > 8) fixed_add(eb[1] * qrow, th, tl);
-                    }
+                    if (kEnergy && cons && live_k) fixed_add(eb * qrow, th, tl);
                     if (live_k) {
                         if (S64) {
                             double* dp = S64 + (int64_t)k0 * ld;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j, dp += ld)
+                            for (int j = 0; j < 8; ++j, dp += ld)
                                 if (j < nk) *dp = (double)v[j];
                         } else {
                             float* sp = S + (int64_t)k0 * ld;
 #pragma unroll
-                            for (int j = 0; j < 16; ++j, sp += ld)
+                            for (int j = 0; j < 8; ++j, sp += ld)
                                 if (j < nk) {
                                     *sp = v[j];
-                                    rmax = fmaxf(rmax, fabsf(v[j] - old[j]));
+                                    if (residual) rmax = fmaxf(rmax, fabsf(v[j] - old[j]));
                                 }
                         }
                     }
-                    load_old(e0 + 16);
-                    // this block's units: wait for the load, relax this lane's row in
+                    load_old(e0 + 8);
+                    // this block's unit: wait for the load, relax this lane's row in
                     // place (rows outside the problem stay unchanged), store the box
                     // into the other ping-pong buffer
-                    bool stop = false;
-#pragma unroll
-                    for (int ui = 0; ui < 16 / ucols; ++ui) {
-                        const int u = e0 / ucols + ui;
-                        if (u >= u_real) break;
-                        // the buffer was read by the previous unit's store, issued before the
-                        // TMEM read and the S stores above
+                    const int u = e0 / ucols, ku = kbase + u * ucols;
+                    if (u >= u_real) continue;
+                    const uint32_t b = rel_used % G_REL_NB;
+                    if (tf32 || !(e0 & 8)) {
+                        // the buffer fetched into was read by the previous unit's store, issued
+                        // before the TMEM read and the S stores above
                         pump(u + 1);
-                        const uint32_t b = rel_used % G_REL_NB;
                         const bool got =
                             mbar_wait(rel_bar(ew, b), (rel_used / G_REL_NB) & 1u, flag, FLAG_WAIT_EPILOGUE);
-                        ++rel_used;
                         if (!__all_sync(0xffffffffu, got)) {
-                            stop = true;
+                            ok = false;
                             break;
                         }
-                        uint8_t* hi = rbuf + b * G_REL_BYTES + 32 * lane;
-                        uint8_t* lo = hi + G_REL_BYTES / 2;
-                        const int ku = kbase + u * ucols;
-                        if (in_row) {
+                    }
+                    uint8_t* hi = rbuf + b * G_REL_BYTES + 32 * lane;
+                    uint8_t* lo = hi + G_REL_BYTES / 2;
+                    if (in_row) {
+                        if (tf32) {
 #pragma unroll
-                            for (int h = 0; h < 2; ++h) {  // 16 bytes of each part
-                                const int nku = min(ucols / 2, Mout - ku - h * (ucols / 2));
-                                const float* x = v + ui * ucols + h * (ucols / 2);
-                                if (tf32)
-                                    relax4_tf32(reinterpret_cast<float4*>(hi) + h, reinterpret_cast<float4*>(lo) + h, x,
-                                                hrsc, nku);
-                                else if (fp16)
-                                    overflow |= relax8<true>(reinterpret_cast<uint4*>(hi) + h,
-                                                             reinterpret_cast<uint4*>(lo) + h, x, hrsc, nku);
-                                else
-                                    relax8<false>(reinterpret_cast<uint4*>(hi) + h, reinterpret_cast<uint4*>(lo) + h, x,
-                                                  hrsc, nku);
-                            }
+                            for (int h = 0; h < 2; ++h)  // 16 bytes of each part
+                                relax4_tf32(reinterpret_cast<float4*>(hi) + h, reinterpret_cast<float4*>(lo) + h,
+                                            v + 4 * h, hrsc, nk - 4 * h);
+                        } else {
+                            uint4* hp = reinterpret_cast<uint4*>(hi + 2 * (e0 & 8));
+                            uint4* lp = reinterpret_cast<uint4*>(lo + 2 * (e0 & 8));
+                            if (fp16)
+                                overflow |= relax8<true>(hp, lp, v, hrsc, nk);
+                            else
+                                relax8<false>(hp, lp, v, hrsc, nk);
                         }
+                    }
+                    if (tf32 || (e0 & 8)) {
+                        ++rel_used;
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) {
                             tma_store_3d(map_out, unit_x(ku), row0, unit_z(ku), rbuf_s + b * G_REL_BYTES);
                             bulk_commit();
                         }
-                    }
-                    if (stop) {
-                        ok = false;
-                        break;
                     }
                 }
             };
@@ -661,17 +668,12 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                 run_steps(std::false_type{});
             if (!ok) break;
             if (kEnergy && ewarp && in_row) {  // this slot's partial sums (zero: no correction)
-                const int64_t slot = (int64_t)n_tile * G_SLICES + cs;
-                P.part[slot * (P.m_tiles * (int64_t)G_BM) + r] = make_int4(r_q > 0.0f ? __float_as_int(raw_e) : 0, 0, th, tl);
+                P.part[((int64_t)n_tile * G_SLICES + cs) * (P.m_tiles * (int64_t)G_BM) + r] = make_int2(th, tl);
+                if (kbase <= Mout && Mout < kbase + ncols) P.extra[r] = qrow > 0.0f ? raw_e : 0.0f;
             }
             if (overflow) atomicOr(flag, FLAG_SCALE_OVERFLOW);
-            if (residual) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, o));
-                if (lane == 0 && rmax > 0.0f)
-                    atomicMax(P.resid, (unsigned long long)__double_as_longlong((double)rmax));
-            }
         }
+        flush_residual();
         // no copy may still be in flight when the CTA exits (loads are left only by a wait that gave up)
         for (; rel_used < rel_issued; ++rel_used)
             mbar_wait(rel_bar(ew, rel_used % G_REL_NB), (rel_used / G_REL_NB) & 1u, flag, FLAG_WAIT_EPILOGUE);
@@ -698,18 +700,17 @@ __global__ void group_energy_kernel(const GroupProblem* __restrict__ probs, int 
     for (int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; r < P.rows;
          r += (int64_t)gridDim.x * blockDim.x) {
         long long et = 0;  // exact: in units of 2^-22 of the row's quantum
-        float raw_e = 0.0f;  // held by one slot, zero in the others
+        const float raw_e = P.extra[r];
         for (int nt = 0; nt < P.n_tiles; ++nt)
             for (int cs = 0; cs < G_SLICES; ++cs) {
                 if (P.sw * cs >= P.bn) continue;  // a column slice without columns
-                const int4 v = P.part[((int64_t)nt * G_SLICES + cs) * ld + r];
-                raw_e += __int_as_float(v.x);
-                et += ((long long)v.z << 22) + v.w;
+                const int2 v = P.part[((int64_t)nt * G_SLICES + cs) * ld + r];
+                et += ((long long)v.x << 22) + v.y;
             }
         const double q22 = 1.0 / 4194304.0;  // the slots' units, in quanta
         const double ex = P.ex[r];           // sum_j v_j x_j of this step's input, in quanta
         const bool fp16 = P.fp16 != 0;
-        const float qrow = energy_scale(P, r, fp16);
+        const float qrow = energy_scale(P.vrow[P.kpad], fp16 ? 1.0f : P.rsb[r]);
         // the step's S_j = (1 + b) lr raw_j + bterm (lr = lam / rs, rs = 1
         // for the unscaled formats), so with v_j = c + d_j
         //   rs sum_j v_j S_j = (1 + b) lam (c sum_j raw_j + sum_j d_j raw_j) + rs bterm sum_j v_j,
