@@ -304,6 +304,7 @@ int rts_pp_split_w(rts_ctx* ctx, const double* W, int Min, int Mout, int ldw, in
 // rs: per-row power-of-two scales putting 2 max(|Ibar|, |B|) into [2^13, 2^14)
 // (and their inverses), computed in FP16 mode -- where the split applies them --
 // and, with `bound`, in the other modes too, where they only bound the rows.
+bool rts_pp_one_pass(int kpad);  // whether rts_pp_rows_from_faces reads the Illum once
 int rts_pp_rows_from_faces(rts_ctx* ctx, const double* illum, int64_t N, int64_t ld, int M, int kpad, const double* B, int mode,
                            float* rs, int64_t npad, uint16_t* A, cudaStream_t st, bool bound = false);
 int rts_pp_rows_from_f32(rts_ctx* ctx, const float* ibar, int64_t N, int M, int64_t rows, int kpad, const float* B,

@@ -517,6 +517,12 @@ int rts_pp_split_w(rts_ctx* ctx, const double* W, int Min, int Mout, int ldw, in
     return RTS_OK;
 }
 
+bool rts_pp_one_pass(int kpad)
+{
+    size_t smem = 0;
+    return rts_rows::cells_log2(kpad, &smem) > 0;
+}
+
 int rts_pp_rows_from_faces(rts_ctx* ctx, const double* illum, int64_t N, int64_t ld, int M, int kpad, const double* B,
                            int mode, float* rs, int64_t npad, uint16_t* A, cudaStream_t st, bool bound)
 {
