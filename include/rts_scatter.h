@@ -629,9 +629,11 @@ int rts_illum_solve(rts_ctx* ctx, int precision, int max_iter, double accuracy, 
 #define RTS_TUNE_SERVE_SLACK 5
 /*   RTS_TUNE_SWEEP_CACHE: 1 (default) the first rts_sweep after a change of
  *   the medium or of the structures stores every out-face's attenuation
- *   factors (32 bytes per out-face, its three node records; allocated then;
- *   within budget), and the sweeps after it read them instead of evaluating
- *   the exponentials -- the same numbers; 0 every sweep evaluates them (and the
+ *   factors (32 bytes per out-face, its three node records, or 24 with more
+ *   local directions than five per SM; allocated then; within budget), and the
+ *   sweeps after it read them instead of evaluating the exponentials -- the
+ *   same numbers (with that many directions and over 2^19 cells evaluating is
+ *   faster: nothing is stored); 0 every sweep evaluates them (and the
  *   factors are not allocated).  A sweep that cannot allocate the factors
  *   evaluates them. */
 #define RTS_TUNE_SWEEP_CACHE 6

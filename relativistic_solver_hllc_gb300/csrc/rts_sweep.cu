@@ -215,7 +215,8 @@ __global__ void __launch_bounds__(256) sweep_x0_kernel(X0Args a)
 struct SweepArgs {
     uint32_t* const* items;  // [D]
     double* const* recs;     // [D]
-    double* const* att;      // [D] 4 factors per item (stored or read by the cached forms)
+    double* const* att;      // [D] factors per item (stored or read by the cached forms): e_0, e_1, e_2 and, up to
+                             // five CTAs per SM, q
     int32_t* const* steps;   // [D]
     uint32_t* const* bnd;    // [D]
     const int32_t* nsteps;   // [D]
@@ -406,8 +407,6 @@ struct NormMax {
     }
 };
 
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
-
 // L2 eviction priorities of the sweep's loads.  Every direction reads the
 // cells' medium entries (beta, Q: 16 B of 32 B per cell, 21 MB at 663,552 cells:
 // they fit in L2), while the items, copy words and attenuation factors (4, 4 and
@@ -453,9 +452,9 @@ __device__ __forceinline__ uint32_t ld_hint(const uint32_t* q, uint64_t pol)
 struct ItemData {
     uint32_t w, cp; // item and copy word
     double2 bq;     // beta, Q
-    double2 ki;     // k, 1 / k (kAtt 0, 1)
+    double2 ki;     // k, 1 / k (unless q is stored)
     double S;
-    double2 fa, fb; // kAtt 2: the factors e_0, e_1, e_2 (thirds) and q; else the node distances (fb.y unused)
+    double2 fa, fb; // kAtt 2: the factors e_0, e_1, e_2 (thirds) and, where it is stored, q; else the node distances
     double old, old_n;
 };
 
@@ -510,16 +509,21 @@ __device__ __noinline__ double mean_by_nodes(const SweepArgs& a, uint32_t w, boo
 //
 // A step is a chain: barrier, in-face means, five dependent FP64 operations,
 // store.  Everything else an item needs is known before the step starts, so it
-// is loaded one item ahead, across steps: the item words two, the factors'
-// lines into L2 four, the neighbour's copy into L2 two.  What bounds it: latency
-// (half of the stalls wait for the in-face means, a third of the issue slots are
-// used) and then the FP64 pipe, two operations per SM and cycle, of which an
-// item now takes five (the norm and the exponential are integer work); DRAM is
-// far from its rate.  T threads, kCtas of them per SM with their registers.
+// is loaded one item ahead, across steps (the item words two); seven CTAs per SM
+// hide the latency themselves and load an item's data when they come to it.
+// What bounds it: latency (half of the stalls wait for the in-face means, a
+// third of the issue slots are used), then the FP64 pipe, two operations per SM
+// and cycle, of which an item takes five (the norm and the exponential are
+// integer work), and with many directions the memory system (their steps' cells
+// do not fit L2).  T threads, kCtas of them per SM with their registers.
 // Reading the factors, 82,944 cells x 400 directions (192 threads, 3 CTAs per
-// SM): 1.83 ms, 4.49 with node-by-node means, 24-byte factors, FP64 norm and
+// SM): 1.77 ms, 4.49 with node-by-node means, 24-byte factors, FP64 norm and
 // loads where they are used; storing them 3.0, from 8.22 with FP64 exponentials;
 // 6,000 x 48 (256 threads, one CTA per SM): 0.16 from 0.39 and 0.20 from 0.61.
+// Seven CTAs per SM wait for memory and keep 24 bytes of factors an item, q
+// formed again: 24,576 x 1000 1.43 ms reading and 2.13 storing, from 1.80 and
+// 5.21.  663,552 x 1000, where every sweep evaluates (att_mode): 53.2 ms, from
+// 133 storing and 53.2 reading.
 // kAtt: 0 evaluates every node's attenuation factor, 1 also stores it,
 // 2 reads the stored factors (no exponential).  kPlain: i_scale == 1 and no
 // ball (the one-step face mean).
@@ -558,6 +562,8 @@ __global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__
         }
     }
     __syncthreads();
+    constexpr bool kAhead = kCtas < 7;   // an item's data loaded while the one before is computed
+    constexpr bool kWhole = kCtas < 7;   // q stored beside the three factors
     const uint64_t keep = l2_policy_last(), stream = l2_policy_first();
     const int n_items = ns > 0 ? steps[ns] : 0;
     // cells are below 2^24 and items below 2^26, so 32-bit indexes reach everything
@@ -569,9 +575,13 @@ __global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__
         x.S = Sd[c];
         x.old = Il[4 * c + ((w >> 6) & 3u)];
         x.old_n = (int)cp >= 0 ? Il[cp & kCopyIndex] : 0.0;
-        if (kAtt == 2) {
+        if (kAtt == 2 && kWhole) {
             x.fa = ld_hint(att + 2 * i, stream);
             x.fb = ld_hint(att + 2 * i + 1, stream);
+        } else if (kAtt == 2) {
+            const double* f = reinterpret_cast<const double*>(att) + 3 * (size_t)i;
+            x.ki = ld_hint(reinterpret_cast<const double2*>(a.med) + 2 * c + 1, keep);
+            x.fa.x = f[0], x.fa.y = f[1], x.fb.x = f[2];
         } else {
             x.ki = ld_hint(reinterpret_cast<const double2*>(a.med) + 2 * c + 1, keep);
             x.fa.x = recs[3 * (size_t)i];
@@ -591,17 +601,18 @@ __global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__
     uint32_t w1 = 0, cp1 = 0;
     auto load_words = [&](int idx, uint32_t& w, uint32_t& cp) {
         w = ld_hint(items + idx, stream);
-        cp = a.words ? ld_hint(items + n_items + idx, stream) : copy_word(a.pairs, nullptr, w);
+        cp = !kAhead ? 0 : a.words ? ld_hint(items + n_items + idx, stream) : copy_word(a.pairs, nullptr, w);
     };
     if (have) {
         load_words(i, w1, cp1);
-        load(w1, cp1, (uint32_t)i, cur);
+        if (kAhead) load(w1, cp1, (uint32_t)i, cur);
         it.idx += T;
         it.settle(steps, ns);
-        if (it.valid()) load_words(it.idx, w1, cp1);
+        if (kAhead && it.valid()) load_words(it.idx, w1, cp1);
     }
     for (int L = 0; L < ns; ++L) {
         while (have && lev == L) {
+            if (!kAhead) load(w1, copy_word(a.pairs, nullptr, w1), (uint32_t)i, cur);
             const double* row = Il + 4 * (cur.w >> 8);
             double v0 = row[cur.w & 3u], v1 = row[(cur.w >> 2) & 3u], v2 = row[(cur.w >> 4) & 3u];
             // the next item's data and the words of the one after it
@@ -609,11 +620,13 @@ __global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__
             const bool more = it.valid();
             const int i1 = it.idx, lev1 = it.lev;
             if (more) {
-                load(w1, cp1, (uint32_t)i1, nxt);
+                if (kAhead)
+                    load(w1, cp1, (uint32_t)i1, nxt);
+                else
+                    load_words(i1, w1, cp1);
                 it.idx += T;
                 it.settle(steps, ns);
-                if (it.valid()) load_words(it.idx, w1, cp1);
-                if (kAtt == 2 && i + 4 * T < n_items) prefetch_l2(att + 2 * (uint32_t)(i + 4 * T));
+                if (kAhead && it.valid()) load_words(it.idx, w1, cp1);
             }
             const double R = cell_source(a.md, unit_i, cur.bq.x, cur.bq.y, cur.S);
             double e0, e1, e2, q;
@@ -627,7 +640,8 @@ __global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__
                 in0 = inside(x), in1 = inside(x + 3), in2 = inside(x + 6);
             }
             if (kAtt == 2) {
-                e0 = cur.fa.x, e1 = cur.fa.y, e2 = cur.fb.x, q = cur.fb.y;
+                e0 = cur.fa.x, e1 = cur.fa.y, e2 = cur.fb.x;
+                q = kWhole ? cur.fb.y : (1.0 - ((e0 + e1) + e2)) * cur.ki.y;
             } else {
                 const double ks = a.md.s_scale == 1.0 ? cur.ki.x : cur.ki.x * a.md.s_scale;
                 const double kb = a.md.s_scale == 1.0 ? a.ball[2] : a.ball[2] * a.md.s_scale;
@@ -636,12 +650,15 @@ __global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__
                 e2 = node_att(in2 ? kb : ks, cur.fb.x, tab);
                 // the source's weight in the face mean, (1 - sum_m e_m / 3) / k
                 q = (1.0 - ((e0 + e1) + e2)) * cur.ki.y;
-                if (kAtt == 1) {
+                if (kAtt == 1 && kWhole) {
                     att[2 * (uint32_t)i] = make_double2(e0, e1);
                     att[2 * (uint32_t)i + 1] = make_double2(e2, q);
+                } else if (kAtt == 1) {
+                    double* f = reinterpret_cast<double*>(att) + 3 * (size_t)i;
+                    f[0] = e0, f[1] = e1, f[2] = e2;
                 }
             }
-            if (cur.cp & kSharedOut) {
+            if (kAhead && (cur.cp & kSharedOut)) {
                 // what an earlier step's item may have written
                 cur.old = row[(cur.w >> 6) & 3u];
                 cur.old_n = Il[cur.cp & kCopyIndex];
@@ -676,9 +693,7 @@ __global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__
                       cur.old_n);
             Il[4 * (cur.w >> 8) + ((cur.w >> 6) & 3u)] = mean;
             if (copy) Il[cur.cp & kCopyIndex] = mean;
-            // the copy that the item after the next replaces, on its way into L2
-            if (it.valid() && (int)cp1 >= 0) prefetch_l2(Il + (cp1 & kCopyIndex));
-            cur = nxt;
+            if (kAhead) cur = nxt;
             i = i1;
             lev = lev1;
             have = more;
@@ -876,6 +891,7 @@ int alloc_block(rts_ctx* ctx, rts_sweep_state& sw, void** p, size_t bytes, const
 // it the sweep forms the words itself.
 int alloc_items(rts_ctx* ctx, rts_sweep_state& sw, void** p, int64_t n)
 {
+    if (sw.D > 5 * ctx->num_sms) sw.copy_words = false;  // the form for so many directions does not read them
     if (sw.copy_words) {
         const std::string keep = ctx->last_error;
         if (alloc_block(ctx, sw, p, rts_bytes<uint32_t>(2 * n), "sweep items") == RTS_OK) return RTS_OK;
@@ -1288,19 +1304,42 @@ extern "C" int rts_sweep_set_medium(rts_ctx* ctx, const rts_medium* md, const do
     return RTS_OK;
 }
 
+// Threads per direction, up to the mean size of a step, and as many as leave
+// every resident CTA its registers.  Reading form, 82,944 x 400, three CTAs per
+// SM: 192 threads 1.83 ms, 160 1.94, 256 (80 registers, spills) 2.30.  With more
+// directions 128 threads, 5 CTAs per SM while those hold them all (24,576 x 700,
+// five sweeps with their integrals 7.5 ms against 9.6 with 7), then 7 with at
+// most 72 registers: one wave of 152 x 7 CTAs holds 1,000 directions.
+enum class SweepForm { t512, t256, t192, t128, t128x7 };
+static SweepForm sweep_form(const rts_ctx* ctx, const rts_sweep_state& sw)
+{
+    const int64_t items = sw.records / 3, per_step = items / std::max<int64_t>(1, sw.D * sw.max_levels);
+    if (sw.D > 5 * ctx->num_sms) return SweepForm::t128x7;
+    if (sw.D > 3 * ctx->num_sms || per_step <= 128) return SweepForm::t128;
+    if (sw.D > 2 * ctx->num_sms) return SweepForm::t192;
+    return sw.D > ctx->num_sms || per_step <= 256 ? SweepForm::t256 : SweepForm::t512;
+}
+
 // The form of the next sweep: 2 reads the stored attenuation factors, 1
 // stores them (laying out, and where needed allocating, their block), 0
-// evaluates them (the cache switched off, or no room for the factors).
+// evaluates them (the cache switched off, no room for the factors, or so many
+// cells of so many directions that the reads take longer than the arithmetic:
+// with seven CTAs per SM and 1,000 directions reading takes 1.43 ms and
+// evaluating 1.94 at 24,576 cells, 17.4 and 18.2 at 235,824, 54.8 and 53.4 at
+// 663,552).
+constexpr int64_t kReadCells = (int64_t)1 << 19;
 static int att_mode(rts_ctx* ctx, rts_sweep_state& sw, cudaStream_t st, int* mode)
 {
     *mode = 0;
-    if (!ctx->sweep_cache) return RTS_OK;
+    const bool many = sweep_form(ctx, sw) == SweepForm::t128x7;
+    if (!ctx->sweep_cache || (many && sw.N > kReadCells)) return RTS_OK;
     if (sw.att_valid) {
         *mode = 2;
         return RTS_OK;
     }
     int64_t nfac = 0;
-    for (int64_t d = 0; d < sw.D; ++d) nfac += 4 * sw.h_nitems[d];
+    const int64_t per = many ? 3 : 4;  // factors per item
+    for (int64_t d = 0; d < sw.D; ++d) nfac += per * sw.h_nitems[d];
     const size_t need = rts_bytes<double>(std::max<int64_t>(nfac, 2));
     if (sw.att_bytes != need) {
         rts_dfree(ctx, sw.att_blk, sw.att_bytes);
@@ -1318,7 +1357,7 @@ static int att_mode(rts_ctx* ctx, rts_sweep_state& sw, cudaStream_t st, int* mod
     int64_t o = 0;
     for (int64_t d = 0; d < sw.D; ++d) {
         sw.h_att[d] = sw.att_blk + o;
-        o += 4 * sw.h_nitems[d];
+        o += per * sw.h_nitems[d];
     }
     RTS_CUDA_TRY(ctx, cudaMemcpyAsync(sw.d_att, sw.h_att.data(), sizeof(double*) * sw.D, cudaMemcpyHostToDevice, st));
     *mode = 1;
@@ -1330,28 +1369,12 @@ static void launch_sweep(const SweepArgs& a, unsigned grid, int mode, cudaStream
 {
     const bool plain = a.md.i_scale == 1.0 && !(a.md.radius > 0);
     auto* kernel = plain ? (mode == 2   ? sweep_kernel<2, true, T, kCtas>
-                             : mode == 1 ? sweep_kernel<1, true, T, kCtas>
-                                         : sweep_kernel<0, true, T, kCtas>)
-                          : (mode == 2   ? sweep_kernel<2, false, T, kCtas>
-                             : mode == 1 ? sweep_kernel<1, false, T, kCtas>
-                                         : sweep_kernel<0, false, T, kCtas>);
+                            : mode == 1 ? sweep_kernel<1, true, T, kCtas>
+                                        : sweep_kernel<0, true, T, kCtas>)
+                         : (mode == 2   ? sweep_kernel<2, false, T, kCtas>
+                            : mode == 1 ? sweep_kernel<1, false, T, kCtas>
+                                        : sweep_kernel<0, false, T, kCtas>);
     kernel<<<grid, T, 0, st>>>(a);
-}
-
-// Threads per direction, up to the mean size of a step, and as many as leave
-// every resident CTA its registers.  Reading form, 82,944 x 400, three CTAs per
-// SM: 192 threads 1.83 ms, 160 1.94, 256 (80 registers, spills) 2.30.  With more
-// directions 128 threads, 5 CTAs per SM while those hold them all (24,576 x 700,
-// five sweeps with their integrals 7.5 ms against 9.6 with 7), then 7 with at
-// most 72 registers: one wave of 152 x 7 CTAs holds 1,000 directions.
-enum class SweepForm { t512, t256, t192, t128, t128x7 };
-static SweepForm sweep_form(const rts_ctx* ctx, const rts_sweep_state& sw)
-{
-    const int64_t items = sw.records / 3, per_step = items / std::max<int64_t>(1, sw.D * sw.max_levels);
-    if (sw.D > 5 * ctx->num_sms) return SweepForm::t128x7;
-    if (sw.D > 3 * ctx->num_sms || per_step <= 128) return SweepForm::t128;
-    if (sw.D > 2 * ctx->num_sms) return SweepForm::t192;
-    return sw.D > ctx->num_sms || per_step <= 256 ? SweepForm::t256 : SweepForm::t512;
 }
 
 static int enqueue_sweep(rts_ctx* ctx, cudaStream_t st)

@@ -1,6 +1,7 @@
 """The transport sweep's launch forms (128, 192, 256 and 512 threads per
-direction, chosen from the number of directions and the mean size of a step),
-against the oracle, and a face that two cells write.
+direction, chosen from the number of directions and the mean size of a step;
+with the most directions 128 and three factors an item), against the oracle,
+and a face that two cells write.
 
 Tolerance: 1e-12 relative for Illum and the norm, the FP64 contract of the
 sweep (the longest dependency chain below has under 100 steps, each a few
