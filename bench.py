@@ -177,8 +177,9 @@ def sweep_medium(N: int, seed: int = 11):
 
 
 def read_sweep_profile():
-    """FP64 operations and DRAM bytes per cell-direction of sweep_kernel's read
-    form (the timed steps) from the committed ncu summary."""
+    """FP64 operations and DRAM bytes per cell-direction of sweep_kernel in the
+    form that the timed steps run (663,552 cells x 1000 directions: evaluating)
+    from the committed ncu summary."""
     p = ROOT / "profiles" / "sweep_kernel_24576x1000.json"
     try:
         return json.loads(p.read_text())
@@ -252,7 +253,8 @@ def run_sweep(args, rank, world, local):
     forms = {"read_ms": kern_avg, "store_ms": store_ms, "evaluate_ms": eval_ms,
              "note": "read: the timed steps (attenuation factors exp(-k s) stored by the first sweep of the medium, "
                      "read since); store: the first sweep after a change of medium; evaluate: "
-                     "RTS_TUNE_SWEEP_CACHE 0 (the exponential in every sweep, as the reference)"}
+                     "RTS_TUNE_SWEEP_CACHE 0 (the exponential in every sweep, as the reference). With more than five "
+                     "directions per SM and over 2^19 cells nothing is stored and all three evaluate"}
 
     # parity spot check on two full-size directions against the oracle
     accuracy = None
@@ -305,7 +307,7 @@ def run_sweep(args, rank, world, local):
             "peak_source": "measured FP64 FMA rate of this GPU (rts_measure_fp64_peak)",
             "nominal_fp64_tflops": FP64_NOMINAL_TFLOPS,
             "fp64_pipe_active": prof.get("fp64_pipe_active_frac"),
-            "note": "achieved = FP64 operations per cell-direction of the read form counted by ncu "
+            "note": "achieved = FP64 operations per cell-direction of the evaluating form counted by ncu "
                     "(dadd + dmul + 2 dfma) x the measured cell-direction rate; the pipe also issues the compares, "
                     "so fp64_pipe_active (ncu, 24,576 x 1000) is the binding figure",
             "hbm": {"algorithmic_bytes_per_cell_dir": prof.get("algorithmic_bytes_per_cell_dir"),
@@ -343,8 +345,8 @@ def run_sweep(args, rank, world, local):
                    "cells": N, "dirs": M, "node_records": records, "max_steps": steps_max,
                    "structures_build_s": t_build, "parallelism": "replicas" if world > 1 else "single",
                    "l2": "inputs larger than L2 (no flush)",
-                   "step": "one sweep of every direction within a source iteration (medium unchanged since the "
-                           "first sweep, which stored the attenuation factors: sweep_forms.store_ms)"},
+                   "step": "one sweep of every direction within a source iteration, medium unchanged since the "
+                           "first (sweep_forms)"},
         "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": launches, "clocks": clk,
         "accuracy": accuracy, "norm": norm, "wall_ms_per_step": elapsed / (K + 1) * 1e3, "sweep_forms": forms,
     }
@@ -691,10 +693,11 @@ def run_ours(args, rank, world, local):
         fp64_step = N * M / step64_s / 1e9
         fp64_gpu = {"value": fp64_step, "unit": UNIT, "ms_per_step": step64_s * 1e3,
                     "kernel_ms_avg": k64_ms / max(k64_n, 1), "kernel_launches_timed": k64_n,
-                    "kernel_tflops": 2.0 * N * M * M / (k64_ms / max(k64_n, 1) / 1e3) / 1e12 if k64_n else None,
+                    "kernel_ms_per_step": k64_ms / n_chk,
+                    "kernel_tflops": 2.0 * N * M * M * n_chk / (k64_ms / 1e3) / 1e12 if k64_n else None,
                     "steps": n_chk, "speedup_of_tensor_path": value / fp64_step,
-                    "note": "scatter_fp64_kernel (FP64 CUDA cores, tiled, W in shared memory) running the same "
-                            "relaxed source iteration on the same inputs; the tensor path's target is >= 5x"}
+                    "note": "the FP64 path (sliced_kernel: exact FP16 digit products on the tensor cores, integer "
+                            "totals) running the same relaxed source iteration on the same inputs"}
         S_64 = ctx.solve_read()
         r64 = ctx.solve_residual_history(n_chk).tolist()
         rel = np.abs(S_t - S_64) / np.abs(S_64)
@@ -761,19 +764,22 @@ def run_ours(args, rank, world, local):
         leg["link_frac"] = floor_s / (leg["ms_per_step"] / 1e3)
     if fp64_gpu and fp64_gpu.get("kernel_tflops"):
         fp64_gpu["fp64_peak_tflops"] = measured["fp64_tflops"]
-        fp64_gpu["roofline_frac"] = fp64_gpu["kernel_tflops"] / measured["fp64_tflops"]
+        fp64_gpu["vs_fp64_peak"] = fp64_gpu["kernel_tflops"] / measured["fp64_tflops"]
 
     # roofline of the dominant kernel
     peaks, src = load_peaks()
     flops = 2.0 * N * M * M
-    kern_avg = kern_ms / max(kern_n, 1) / 1e3
+    # FP64 steps run in several launches over cell ranges
+    kern_avg = (kern_ms / K if prec == "fp64" else kern_ms / max(kern_n, 1)) / 1e3
     achieved = flops / kern_avg / 1e12 if kern_n else None
     traffic = read_traffic().get(f"{prec}:{N}x{M}")
     if prec == "fp64":
-        roof = {"bound": "fp64", "achieved": achieved, "peak": measured["fp64_tflops"], "unit": "TFLOP/s",
-                "frac": achieved / measured["fp64_tflops"] if achieved else None, "traffic": traffic,
-                "peak_source": "measured FP64 FMA rate of this GPU (rts_measure_fp64_peak)",
-                "nominal_fp64_tflops": FP64_NOMINAL_TFLOPS}
+        # sums of six 9-bit digits: 21 tensor products of FP16 digits per FP64 product
+        pk = peak_value(peaks, "bf16_tflops") or FALLBACK_PEAKS["bf16_tflops"]
+        roof = {"bound": "tensor", "achieved": achieved, "peak": pk / 21, "unit": "TFLOP/s",
+                "frac": 21 * achieved / pk if achieved else None, "traffic": traffic,
+                "peak_source": f"bf16 dense burst / 21 digit products, {src}",
+                "measured_fp64_tflops": measured["fp64_tflops"], "nominal_fp64_tflops": FP64_NOMINAL_TFLOPS}
     else:
         pk = peak_value(peaks, "bf16_tflops") or FALLBACK_PEAKS["bf16_tflops"]
         roof = {"bound": "tensor", "achieved": achieved, "peak": pk, "unit": "TFLOP/s",

@@ -23,7 +23,7 @@
 // CalculateDivImpuls compute their moments (their kernels are commented out
 // in the reference, cuda/cuda_solve.cu:182,236,259).
 //
-// Precision: every call is FP64, bit-compatible with the reference, unless
+// Precision: every call is FP64 (the reference to 1e-12), unless
 // the RTS_SCATTER_PRECISION environment variable names a tensor-core
 // precision (fp16x3, bf16x3 or tf32x3).  Then InitDevice sets that precision
 // on the context (rts_set_precision) and every scattering call -- the
