@@ -174,10 +174,11 @@ split_w_kernel(const double* __restrict__ W, int Min, int Mout, int ldw, int kpa
         if (real)
 #pragma unroll 8
             for (int j = warp; j < Min; j += SW_WARPS) {
-                const unsigned long long w =
-                    (unsigned long long)__double_as_longlong(col[j * step]) & 0x7FFFFFFFFFFFFFFFull;
-                if (w <= 0x7FF0000000000000ull && w > m) m = w;
+                // |W| times two as an integer
+                const unsigned long long w = (unsigned long long)__double_as_longlong(col[j * step]) << 1;
+                if (w <= 0xFFE0000000000000ull && w > m) m = w;
             }
+        m >>= 1;
         smax[warp][lane] = m;
         __syncthreads();
 #pragma unroll
@@ -275,10 +276,11 @@ __global__ void __launch_bounds__(256) face_sums_kernel(const double* __restrict
         I += b.x;
         I += b.y;
         sums[(int64_t)j * N + c] = I;
-        const unsigned long long ub = (unsigned long long)__double_as_longlong(I) & 0x7FFFFFFFFFFFFFFFull;
-        if (ub <= 0x7FF0000000000000ull && ub > mx) mx = ub;
+        // |I| times two as an integer (a mask would become an FP64 absolute value)
+        const unsigned long long ub = (unsigned long long)__double_as_longlong(I) << 1;
+        if (ub <= 0xFFE0000000000000ull && ub > mx) mx = ub;
     }
-    if (cmax) atomicMax(cmax + c, mx);
+    if (cmax) atomicMax(cmax + c, mx >> 1);
 }
 
 // Row scales from the per-cell maxima of face_sums_kernel: the scale of

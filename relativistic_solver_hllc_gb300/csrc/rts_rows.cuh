@@ -10,8 +10,10 @@
 // A block owns 8 cells (256 contiguous bytes of each direction) and all
 // directions; at 1000 directions its sums take 66 KB, so three blocks share an
 // SM and one's loads run under another's conversion.  162,000 x 1000 in FP16:
-// 1.50 ms (3.9 TB/s), against 4.28 ms for a pass for the scales and a pass for
-// the rows that did their arithmetic on the FP64 pipe.
+// 1.30 ms (4.5 TB/s), against 4.28 ms for a pass for the scales and a pass for
+// the rows that did their arithmetic on the FP64 pipe; 82,944 x 400: 0.27 ms
+// (0.33 with the sign masked off a sum's bits, which the compiler makes an FP64
+// absolute value: a fourth of the pipe's work).
 #pragma once
 
 #include <cstdint>
@@ -190,16 +192,16 @@ __global__ void __launch_bounds__(THREADS, 3) rows_from_faces_kernel(const Args 
                 if (kMode == 3) {
                     if (ub == 0x8000000000000000ull) ub = 0;  // -0; negative values lie above every other pattern
                 } else {
-                    ub &= 0x7FFFFFFFFFFFFFFFull;
+                    ub <<= 1;  // |I| times two as an integer (a mask would become an FP64 absolute value)
                 }
-                if ((kMode == 3 || ub <= 0x7FF0000000000000ull) && ub > mx) mx = ub;
+                if ((kMode == 3 || ub <= 0xFFE0000000000000ull) && ub > mx) mx = ub;
             }
         }
         for (int o = 16; o >= cells; o >>= 1) {
             const unsigned long long v = __shfl_xor_sync(0xffffffffu, mx, o);
             mx = v > mx ? v : mx;
         }
-        if ((t & 31) < cells) atomicMax(&cmax[cell], mx);
+        if ((t & 31) < cells) atomicMax(&cmax[cell], kMode == 3 ? mx : mx >> 1);
     }
     __syncthreads();
     if (kMode == 3 && t < cells) {

@@ -339,7 +339,7 @@ sliced_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
             const int64_t r = (t / p.n_tiles) * S_BM + q * 32 + lane;
             const int n_tile = (int)(t % p.n_tiles);
             const int kb = n_tile * kBn + cs * kCols;  // first column, relative to k0
-            unsigned long long rmax = 0;  // bits of a non-negative double: they order as integers
+            unsigned long long rmax = 0;  // bits of a non-negative double, times two: they order as integers
             if (r < p.n) {
                 const int er = p.rowexp[r];
                 const double bterm = kUpdate ? (1.0 - p.lambda) * p.B[r] : 0.0;
@@ -366,9 +366,8 @@ sliced_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
                         if (kUpdate) v = fma(p.lambda, v, bterm);
                         dst[(int64_t)(h + j) * p.ld] = v;
                         if (kResidual) {
-                            const unsigned long long ub =
-                                (unsigned long long)__double_as_longlong(v - old[j]) & 0x7FFFFFFFFFFFFFFFull;
-                            if (ub > rmax && ub <= 0x7FF0000000000000ull) rmax = ub;  // NaN drops out, as in fmax
+                            const unsigned long long ub = (unsigned long long)__double_as_longlong(v - old[j]) << 1;
+                            if (ub > rmax && ub <= 0xFFE0000000000000ull) rmax = ub;  // NaN drops out, as in fmax
                         }
                     }
                 }
@@ -382,7 +381,7 @@ sliced_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
                     const unsigned long long x = __shfl_xor_sync(0xffffffffu, rmax, o);
                     rmax = x > rmax ? x : rmax;
                 }
-                if (lane == 0 && rmax > 0) atomicMax(p.resid, rmax);
+                if (lane == 0 && rmax > 0) atomicMax(p.resid, rmax >> 1);
             }
         }
     }

@@ -314,7 +314,7 @@ static bool no_room(int rc);
 static int record_on(rts_ctx* ctx, cudaEvent_t& ev, cudaStream_t st);
 
 // Rows of cells [0, n) of a device Illum whose rows hold `ld` cells into A and
-// rs on `st`: in one pass where a row fits shared memory (82,944 x 400: 0.33 ms,
+// rs on `st`: in one pass where a row fits shared memory (82,944 x 400: 0.27 ms,
 // the staged preparation 0.37 and its staging), else the staged preparation in the integral
 // calls' staging (waiting for their preparation and face sums in flight, and
 // leaving them to prepare their own rows again), or, without room for the
