@@ -393,20 +393,15 @@ weights_normalise_kernel(double* __restrict__ W, int M, int loc)
 }
 
 // Cells (threads) per block of the moment kernels.  Every block walks all
-// directions, so a launch takes as long as the SM with the most blocks: 82,944
-// cells in blocks of 128 are 648, five on some SMs and 4.26 on average.  The first
-// of the given sizes that leaves the fullest SM the fewest cells (82,944 x 400:
-// moments_kernel 509 -> 453 us with 64, illum_params_kernel 2,131 -> 1,964 with 96).
-constexpr int CELL_THREADS_MAX = 128;
-inline int cell_threads(int64_t N, int num_sms, const int (&sizes)[3])
+// directions, so a launch takes as long as the SM with the most cells: 82,944 in
+// blocks of 128 are 648, five on some SMs and 4.26 on average; 64 where that
+// leaves the fullest SM fewer (82,944 x 400: moments_kernel 510 -> 452 us,
+// illum_params_kernel 2,135 -> 2,018).  Below three blocks of 128 a SM a call is
+// bound by one block's walk and keeps 128.
+inline int cell_threads(int64_t N, int num_sms)
 {
-    int best = sizes[0];
-    int64_t least = INT64_MAX;
-    for (int t : sizes) {
-        const int64_t blocks = (N + t - 1) / t, most = (blocks + num_sms - 1) / num_sms * t;
-        if (most < least) least = most, best = t;
-    }
-    return best;
+    auto fullest = [&](int t) { return ((N + t - 1) / t + num_sms - 1) / num_sms * t; };
+    return N > (int64_t)3 * 128 * num_sms && fullest(64) < fullest(128) ? 64 : 128;
 }
 
 constexpr int MOM_DCHUNK = 256;
@@ -416,17 +411,18 @@ constexpr int MOM_DCHUNK = 256;
 // (cell, direction) costs the face sum (3 adds) and four FMAs -- the
 // reference's sum_j (sum_f I_f / 4) area_j w_j regrouped, the FP64 pipe
 // being the bound.
-__global__ void __launch_bounds__(CELL_THREADS_MAX)
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads)
 moments_kernel(const double* __restrict__ illum, const double* __restrict__ xyz,
                const double* __restrict__ area, int64_t N, int M, double full_area,
                double* __restrict__ energy, double* __restrict__ flux)
 {
     __shared__ double sd[MOM_DCHUNK][4];
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t c = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     double e = 0.0, fx = 0.0, fy = 0.0, fz = 0.0;
     for (int j0 = 0; j0 < M; j0 += MOM_DCHUNK) {
         const int nj = min(MOM_DCHUNK, M - j0);
-        for (int t = threadIdx.x; t < nj; t += blockDim.x) {
+        for (int t = threadIdx.x; t < nj; t += kThreads) {
             const double a4 = area[j0 + t] * 0.25;  // exact
             sd[t][0] = a4;
             sd[t][1] = xyz[3 * (j0 + t)] * a4;
@@ -473,7 +469,8 @@ moments_kernel(const double* __restrict__ illum, const double* __restrict__ xyz,
 // the reference's 80.
 constexpr int PAR_DCHUNK = 128;
 
-__global__ void __launch_bounds__(CELL_THREADS_MAX)
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads)
 illum_params_kernel(const double* __restrict__ illum, const double* __restrict__ xyz,
                     const double* __restrict__ area, int64_t N, int M, double full_area,
                     const double* __restrict__ normals, const double* __restrict__ face_areas,
@@ -481,7 +478,7 @@ illum_params_kernel(const double* __restrict__ illum, const double* __restrict__
 {
     // per direction: area, area w (3), area w w^T (xx, xy, xz, yy, yz, zz), w (3)
     __shared__ double sd[PAR_DCHUNK][13];
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t c = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const bool geo = normals != nullptr;
     double nS[4][3];
 #pragma unroll
@@ -493,7 +490,7 @@ illum_params_kernel(const double* __restrict__ illum, const double* __restrict__
     double ds = 0.0, di[3] = {0.0, 0.0, 0.0};
     for (int j0 = 0; j0 < M; j0 += PAR_DCHUNK) {
         const int nj = min(PAR_DCHUNK, M - j0);
-        for (int t = threadIdx.x; t < nj; t += blockDim.x) {
+        for (int t = threadIdx.x; t < nj; t += kThreads) {
             const double x = xyz[3 * (j0 + t)], y = xyz[3 * (j0 + t) + 1], z = xyz[3 * (j0 + t) + 2];
             const double a = area[j0 + t];
             sd[t][0] = a;
@@ -719,10 +716,10 @@ int rts_launch_weights(rts_ctx* ctx)
 
 int rts_launch_moments(rts_ctx* ctx, cudaStream_t st)
 {
-    const int threads = cell_threads(ctx->N, ctx->num_sms, {64, 96, 128});
+    const int threads = cell_threads(ctx->N, ctx->num_sms);
     const int64_t blocks = (ctx->N + threads - 1) / threads;
     rts_timing_begin(ctx, st);
-    moments_kernel<<<(unsigned)blocks, threads, 0, st>>>(ctx->d_illum, ctx->d_xyz, ctx->d_area,
+    (threads == 64 ? moments_kernel<64> : moments_kernel<128>)<<<(unsigned)blocks, threads, 0, st>>>(ctx->d_illum, ctx->d_xyz, ctx->d_area,
                                                              ctx->N, (int)ctx->M, ctx->full_area,
                                                              ctx->d_energy, ctx->d_flux);
     rts_timing_end(ctx, st);
@@ -733,12 +730,12 @@ int rts_launch_moments(rts_ctx* ctx, cudaStream_t st)
 
 int rts_launch_illum_params(rts_ctx* ctx, cudaStream_t st)
 {
-    const int threads = cell_threads(ctx->N, ctx->num_sms, {128, 96, 64});
+    const int threads = cell_threads(ctx->N, ctx->num_sms);
     const int64_t blocks = (ctx->N + threads - 1) / threads;
     const double* geo = ctx->d_geo;
     const int64_t N = ctx->N;
     rts_timing_begin(ctx, st);
-    illum_params_kernel<<<(unsigned)blocks, threads, 0, st>>>(
+    (threads == 64 ? illum_params_kernel<64> : illum_params_kernel<128>)<<<(unsigned)blocks, threads, 0, st>>>(
         ctx->d_illum, ctx->d_xyz, ctx->d_area, N, (int)ctx->M, ctx->full_area, geo, geo ? geo + 12 * N : nullptr,
         geo ? geo + 16 * N : nullptr, ctx->d_params);
     rts_timing_end(ctx, st);

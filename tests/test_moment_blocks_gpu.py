@@ -1,5 +1,5 @@
-"""The moment kernels' block sizes (64, 96 or 128 cells, by the cell count and
-the SMs): a cell's sums run over the directions in order whatever the block, so
+"""The moment kernels' block sizes (64 or 128 cells, by the cell count and the
+SMs): a cell's sums run over the directions in order whatever the block, so
 each size gives the same bits."""
 import numpy as np
 import pytest
@@ -10,7 +10,7 @@ from relativistic_solver_hllc_gb300 import STREAM_PARAMS
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N", [9728, 14590, 19456, 82944])  # 64, 96, 128 and 96 cells a block on 152 SMs
+@pytest.mark.parametrize("N", [9728, 58368, 60000, 82944])  # 128, 128, 64 and 64 cells a block on 152 SMs
 def test_block_sizes_agree(ctx, N):
     M = 7
     rng = np.random.default_rng(N)
