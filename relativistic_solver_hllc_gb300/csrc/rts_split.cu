@@ -252,8 +252,9 @@ static bool pinned(const void* p)
 // beside each other, as above: the integral of 162,000 cells x 1000
 // directions takes 10 ms, its copies 25 ms in and 7 ms out.  A range brings at
 // least 16 MB in (75 us), several times what a range costs in launches; smaller
-// calls and pageable arrays, whose copies the host would carry out piece by
-// piece, run in one piece.
+// calls, pageable arrays, whose copies the host would carry out piece by piece,
+// and rows longer than a strided copy's pitch may be (2^31 - 1 bytes: 67,108,863
+// cells) run in one piece.
 int rts_fp64_host_call(rts_ctx* ctx, const double* illum_host, const double* B_host, double lambda, double* S_host)
 {
     rts_split_state& s = ctx->split;
@@ -262,7 +263,9 @@ int rts_fp64_host_call(rts_ctx* ctx, const double* illum_host, const double* B_h
     cudaStream_t sc = ctx->streams[RTS_STREAM_SCATTERING_1];
     const int64_t tiles = (N + 127) / 128;
     const int64_t pieces = std::min<int64_t>({RTS_HOST_CHUNKS, tiles, M * N * 32 / (16 << 20)});
-    if (pieces < 2 || !pinned(illum_host) || !pinned(S_host)) {
+    int max_pitch = 0;
+    RTS_CUDA_TRY(ctx, cudaDeviceGetAttribute(&max_pitch, cudaDevAttrMaxPitch, ctx->device));
+    if (pieces < 2 || N * 32 > max_pitch || !pinned(illum_host) || !pinned(S_host)) {
         RTS_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_illum, illum_host, (size_t)(M * N * 32), cudaMemcpyHostToDevice, sc));
         if (update) RTS_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_B, B_host, (size_t)N * 8, cudaMemcpyHostToDevice, sc));
         int rc = rts_launch_scatter_fp64(ctx, 0, loc, sc, ctx->d_B, lambda, update, false);
