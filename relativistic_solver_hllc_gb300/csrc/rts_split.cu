@@ -247,14 +247,27 @@ static bool pinned(const void* p)
     return a.type == cudaMemoryTypeHost;
 }
 
+// `rows` rows of `width` bytes, `pitch` apart on both sides: one strided copy,
+// or, past the documented limit of its pitch (cudaDevAttrMaxPitch, 2^31 - 1
+// bytes on GB300: Illum rows of 2^26 cells), a copy per row.
+static cudaError_t copy_rows(double* dst, const double* src, int64_t pitch, int64_t width, int64_t rows,
+                             cudaMemcpyKind kind, cudaStream_t st)
+{
+    if (pitch < ((int64_t)1 << 31))
+        return cudaMemcpy2DAsync(dst, (size_t)pitch, src, (size_t)pitch, (size_t)width, (size_t)rows, kind, st);
+    cudaError_t e = cudaSuccess;
+    for (int64_t r = 0; r < rows && e == cudaSuccess; ++r)
+        e = cudaMemcpyAsync(dst + r * (pitch / 8), src + r * (pitch / 8), (size_t)width, kind, st);
+    return e;
+}
+
 // rts_scattering / rts_scattering_update in FP64.  With pinned host arrays the
 // cells are cut into ranges whose copies in, integrals and copies out run
 // beside each other, as above: the integral of 162,000 cells x 1000
 // directions takes 10 ms, its copies 25 ms in and 7 ms out.  A range brings at
 // least 16 MB in (75 us), several times what a range costs in launches; smaller
-// calls, pageable arrays, whose copies the host would carry out piece by piece,
-// and rows longer than a strided copy's pitch may be (2^31 - 1 bytes: 67,108,863
-// cells) run in one piece.
+// calls and pageable arrays, whose copies the host would carry out piece by
+// piece, run in one piece.
 int rts_fp64_host_call(rts_ctx* ctx, const double* illum_host, const double* B_host, double lambda, double* S_host)
 {
     rts_split_state& s = ctx->split;
@@ -263,9 +276,7 @@ int rts_fp64_host_call(rts_ctx* ctx, const double* illum_host, const double* B_h
     cudaStream_t sc = ctx->streams[RTS_STREAM_SCATTERING_1];
     const int64_t tiles = (N + 127) / 128;
     const int64_t pieces = std::min<int64_t>({RTS_HOST_CHUNKS, tiles, M * N * 32 / (16 << 20)});
-    int max_pitch = 0;
-    RTS_CUDA_TRY(ctx, cudaDeviceGetAttribute(&max_pitch, cudaDevAttrMaxPitch, ctx->device));
-    if (pieces < 2 || N * 32 > max_pitch || !pinned(illum_host) || !pinned(S_host)) {
+    if (pieces < 2 || !pinned(illum_host) || !pinned(S_host)) {
         RTS_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_illum, illum_host, (size_t)(M * N * 32), cudaMemcpyHostToDevice, sc));
         if (update) RTS_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_B, B_host, (size_t)N * 8, cudaMemcpyHostToDevice, sc));
         int rc = rts_launch_scatter_fp64(ctx, 0, loc, sc, ctx->d_B, lambda, update, false);
@@ -285,8 +296,7 @@ int rts_fp64_host_call(rts_ctx* ctx, const double* illum_host, const double* B_h
         e = cudaMemcpyAsync(ctx->d_B, B_host, (size_t)N * 8, cudaMemcpyHostToDevice, s.copy_in);
     for (int i = 0; i * csz < N && rc == RTS_OK && e == cudaSuccess; ++i) {
         const int64_t c0 = i * csz, n = std::min(N, c0 + csz) - c0;
-        e = cudaMemcpy2DAsync(ctx->d_illum + c0 * 4, (size_t)N * 32, illum_host + c0 * 4, (size_t)N * 32, (size_t)n * 32,
-                              (size_t)M, cudaMemcpyHostToDevice, s.copy_in);
+        e = copy_rows(ctx->d_illum + c0 * 4, illum_host + c0 * 4, N * 32, n * 32, M, cudaMemcpyHostToDevice, s.copy_in);
         if (e == cudaSuccess) e = cudaEventRecord(s.ev_in[i], s.copy_in);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(sc, s.ev_in[i], 0);
         if (e != cudaSuccess) break;
@@ -295,8 +305,7 @@ int rts_fp64_host_call(rts_ctx* ctx, const double* illum_host, const double* B_h
         e = cudaEventRecord(s.ev_done[i], sc);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(s.copy_out, s.ev_done[i], 0);
         if (e == cudaSuccess)
-            e = cudaMemcpy2DAsync(S_host + c0, (size_t)N * 8, ctx->d_S + c0, (size_t)N * 8, (size_t)n * 8, (size_t)loc,
-                                  cudaMemcpyDeviceToHost, s.copy_out);
+            e = copy_rows(S_host + c0, ctx->d_S + c0, N * 8, n * 8, loc, cudaMemcpyDeviceToHost, s.copy_out);
     }
     const cudaError_t w[3] = {cudaStreamSynchronize(s.copy_in), cudaStreamSynchronize(sc),
                               cudaStreamSynchronize(s.copy_out)};
