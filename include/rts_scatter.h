@@ -637,6 +637,13 @@ int rts_illum_solve(rts_ctx* ctx, int precision, int max_iter, double accuracy, 
  *   factors are not allocated).  A sweep that cannot allocate the factors
  *   evaluates them. */
 #define RTS_TUNE_SWEEP_CACHE 6
+/*   RTS_TUNE_FP64_DIGITS: arithmetic of the FP64 integrals.  1 (default): the
+ *   tensor cores' exact digit products where the weights and the size suit
+ *   them (rts_set_precision), else the FP64 cores; 0: always the FP64 cores,
+ *   every integral one chain of fused multiply-adds over the in-directions in
+ *   their order, the reference kernel's order of summation.  The two differ in
+ *   the last bits. */
+#define RTS_TUNE_FP64_DIGITS 7
 int rts_set_tuning(rts_ctx* ctx, int key, int value);
 
 /* The drain period (K-slices per FP32 drain) that the context's tensor-core

@@ -24,8 +24,10 @@
 // in the reference, cuda/cuda_solve.cu:182,236,259).
 //
 // Precision: every call is FP64 (the reference to 1e-12), unless
-// the RTS_SCATTER_PRECISION environment variable names a tensor-core
-// precision (fp16x3, bf16x3 or tf32x3).  Then InitDevice sets that precision
+// the RTS_SCATTER_PRECISION environment variable names another arithmetic.
+// fp64_chain keeps the reference kernel's order of summation too: one chain of
+// FP64 multiply-adds per integral (RTS_TUNE_FP64_DIGITS 0).  fp16x3, bf16x3 and
+// tf32x3 are the tensor-core precisions.  With one of those, InitDevice sets that precision
 // on the context (rts_set_precision) and every scattering call -- the
 // asynchronous calls on the device-resident Illum that the source iteration
 // makes (CalculateIntScatteringAsyncMPIStream, ...AsyncMPI, ...Async) and the
@@ -62,7 +64,7 @@ rts_ctx* g_ctx = nullptr;
 int g_device = 0;
 bool g_owns_moments = false;
 
-// RTS_SCATTER_PRECISION: fp64 (default), fp16x3, bf16x3 or tf32x3
+// RTS_SCATTER_PRECISION: fp64 (default), fp64_chain, fp16x3, bf16x3 or tf32x3
 int env_precision()
 {
     const char* v = std::getenv("RTS_SCATTER_PRECISION");
@@ -71,9 +73,16 @@ int env_precision()
     if (s == "fp16x3") return RTS_PREC_FP16X3;
     if (s == "bf16x3") return RTS_PREC_BF16X3;
     if (s == "tf32x3") return RTS_PREC_TF32X3;
-    if (s != "fp64" && !s.empty())
-        std::fprintf(stderr, "RTS_SCATTER_PRECISION=%s is not fp64, fp16x3, bf16x3 or tf32x3: using fp64\n", v);
+    if (s != "fp64" && s != "fp64_chain" && !s.empty())
+        std::fprintf(stderr, "RTS_SCATTER_PRECISION=%s is not fp64, fp64_chain, fp16x3, bf16x3 or tf32x3: using fp64\n",
+                     v);
     return RTS_PREC_FP64;
+}
+
+bool env_fp64_chain()
+{
+    const char* v = std::getenv("RTS_SCATTER_PRECISION");
+    return v && std::string(v) == "fp64_chain";
 }
 
 int report(int rc, const char* where)
@@ -178,6 +187,7 @@ void InitDevice(const grid_directions_t& grid_dir_host, grid_t& grid_host, const
     rts_host_illum(g_ctx, &grid_host.Illum);
     rts_host_scattering(g_ctx, &grid_host.scattering);
     const int precision = env_precision();
+    if (env_fp64_chain()) report(rts_set_tuning(g_ctx, RTS_TUNE_FP64_DIGITS, 0), "InitDevice (FP64 arithmetic)");
     if (report(rts_set_precision(g_ctx, precision), "InitDevice (precision)") == 0)
         tune_schedule(precision, M, grid_host.size);
     if (start == 0) {  // the first rank also receives the moments (cuda/cuda_struct.cu:158-175)

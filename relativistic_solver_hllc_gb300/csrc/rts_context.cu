@@ -863,6 +863,10 @@ int rts_set_tuning(rts_ctx* ctx, int key, int value)
         ctx->sweep_cache = value;
         if (ctx->sweep) ctx->sweep->att_valid = false;
         return RTS_OK;
+    case RTS_TUNE_FP64_DIGITS:
+        RTS_REQUIRE(ctx, value == 0 || value == 1, RTS_ERR_INVALID_ARGUMENT, "FP64 digits switch %d not 0 or 1", value);
+        ctx->fp64_digits = value;
+        return RTS_OK;
     case RTS_TUNE_BIAS:
         RTS_REQUIRE(ctx, value >= -1, RTS_ERR_INVALID_ARGUMENT, "bias correction %d below -1", value);
         ctx->split_bias = value;

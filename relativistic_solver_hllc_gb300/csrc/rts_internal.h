@@ -217,6 +217,7 @@ struct rts_ctx {
     int split_bias = 0;          // truncation correction: 0 conservation-based (relaxed steps), -1 none, >0 constant (1e-10 units)
     int tuning_epoch = 0;        // bumped when a setting that batch tables copy changes
     int64_t w_version = 0;       // bumped whenever d_W is rewritten
+    int fp64_digits = 1;         // FP64 integrals on the tensor cores where they suit (RTS_TUNE_FP64_DIGITS)
     int sweep_cache = 1;         // rts_sweep: store the attenuation factors once per medium (RTS_TUNE_SWEEP_CACHE)
     int serve_policy = 1;        // rts_serve_run: 0 all resident, 1 earliest deadline first, 2 least remaining work first
     int64_t serve_budget = 0;    // tiles per step for policy 1 (0: 8 waves of the SMs)

@@ -545,7 +545,7 @@ constexpr int64_t S_ROWS_BYTES = (int64_t)1 << 31;
 // 100, 40 x 1,000 156 and 313.
 static bool sliced_fits(const rts_ctx* ctx)
 {
-    if (ctx->cc_major != 10) return false;
+    if (ctx->cc_major != 10 || !ctx->fp64_digits) return false;
     const int64_t N = ctx->N, M = ctx->M;
     size_t smem = 0;
     if (M < 48 || N >= ((int64_t)1 << 31) || rts_rows::cells_log2((int)kpad_of(ctx), &smem) == 0) return false;
