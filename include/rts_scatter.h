@@ -642,7 +642,8 @@ int rts_illum_solve(rts_ctx* ctx, int precision, int max_iter, double accuracy, 
  *   them (rts_set_precision), else the FP64 cores; 0: always the FP64 cores,
  *   every integral one chain of fused multiply-adds over the in-directions in
  *   their order, the reference kernel's order of summation.  The two differ in
- *   the last bits. */
+ *   the last bits.  2: as 1, but every contraction is taken to have given up
+ *   (rts_fp64_stats), to check what follows. */
 #define RTS_TUNE_FP64_DIGITS 7
 int rts_set_tuning(rts_ctx* ctx, int key, int value);
 
@@ -713,6 +714,16 @@ int rts_sweep_exp_check(rts_ctx* ctx, int64_t n, double* max_ulp);
  * Each allocates its buffers for the duration of the call. */
 int rts_measure_fp64_peak(rts_ctx* ctx, double seconds, double* tflops);
 int rts_measure_link(rts_ctx* ctx, int64_t bytes, int reps, double* h2d_gbs, double* d2h_gbs, double* both_gbs);
+
+/* What the FP64 integrals' digit products (RTS_TUNE_FP64_DIGITS) have done since
+ * the context was created; waits for the device.  passes: contractions queued (a
+ * call or step takes one, or more where its digit rows exceed their scratch);
+ * listed: rows of them with outputs that the digits cannot carry, computed on
+ * the FP64 cores; gave_up: contractions in which a bounded wait gave up.  All
+ * outputs of those are computed again on the FP64 cores, but a step's residual
+ * is lost: reading it returns RTS_ERR_DEVICE_WAIT until the next
+ * rts_solve_setup. */
+int rts_fp64_stats(rts_ctx* ctx, int64_t* passes, int64_t* listed, int64_t* gave_up);
 
 /* Number of kernels this context has launched so far. */
 int rts_launch_count(const rts_ctx* ctx, int64_t* count);

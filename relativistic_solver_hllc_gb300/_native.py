@@ -125,6 +125,7 @@ _SIGNATURES = {
     "rts_autotune_save": (C.c_int, [_vp, C.c_char_p]),
     "rts_autotune_load": (C.c_int, [_vp, C.c_char_p]),
     "rts_stream_handle": (C.c_int, [_vp, C.c_int, C.POINTER(_vp)]),
+    "rts_fp64_stats": (C.c_int, [_vp, C.POINTER(_i64), C.POINTER(_i64), C.POINTER(_i64)]),
     "rts_launch_count": (C.c_int, [_vp, C.POINTER(_i64)]),
     "rts_measure_fp64_peak": (C.c_int, [_vp, C.c_double, _dp]),
     "rts_measure_link": (C.c_int, [_vp, _i64, C.c_int, _dp, _dp, _dp]),
@@ -655,6 +656,12 @@ class Context:
         self._check(self.lib.rts_measure_link(self.h, int(nbytes), int(reps), C.byref(a), C.byref(b), C.byref(c)),
                     "rts_measure_link")
         return {"h2d_gbs": a.value, "d2h_gbs": b.value, "bidirectional_gbs": c.value, "bytes": int(nbytes)}
+
+    def fp64_stats(self) -> tuple[int, int, int]:
+        """(contractions queued, rows listed, contractions that gave up) of the FP64 integrals' digit products."""
+        v = [_i64() for _ in range(3)]
+        self._check(self.lib.rts_fp64_stats(self.h, *(C.byref(x) for x in v)), "rts_fp64_stats")
+        return tuple(x.value for x in v)
 
     def launch_count(self) -> int:
         v = _i64()

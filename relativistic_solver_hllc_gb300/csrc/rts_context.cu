@@ -232,13 +232,14 @@ int rts_ctx_create(int device, rts_ctx** out)
     }
     ctx->d_resid = (unsigned long long*)p;
     ctx->resid_target = ctx->d_resid;
-    if (rts_dmalloc(ctx, &p, sizeof(int) * 4, "flags") != RTS_OK) {
+    if (rts_dmalloc(ctx, &p, RTS_FLAG_BYTES, "flags") != RTS_OK) {
         rts_ctx_destroy(ctx);
         return RTS_ERR_OUT_OF_MEMORY;
     }
     ctx->d_flag = (int*)p;
+    ctx->d_fp64 = (unsigned long long*)((char*)p + 16);
     cudaMemset(ctx->d_resid, 0, sizeof(unsigned long long) * (RTS_RESID_CAP + 1));
-    cudaMemset(ctx->d_flag, 0, sizeof(int) * 4);
+    cudaMemset(ctx->d_flag, 0, RTS_FLAG_BYTES);
     *out = ctx;
     return RTS_OK;
 }
@@ -251,7 +252,7 @@ int rts_ctx_destroy(rts_ctx* ctx)
         if (ctx->streams[i]) cudaStreamSynchronize(ctx->streams[i]);
     free_grid(ctx);
     rts_dfree(ctx, ctx->d_resid, sizeof(unsigned long long) * (RTS_RESID_CAP + 1));
-    rts_dfree(ctx, ctx->d_flag, sizeof(int) * 4);
+    rts_dfree(ctx, ctx->d_flag, RTS_FLAG_BYTES);
     for (int i = 0; i < RTS_STREAM_COUNT; ++i)
         if (ctx->streams[i]) cudaStreamSynchronize(ctx->streams[i]);
     if (ctx->serve_copy) {
@@ -711,6 +712,7 @@ int rts_solve_setup(rts_ctx* ctx, int precision, const double* B_host, double la
     RTS_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_B, B_host, rts_bytes<double>(ctx->N),
                                       cudaMemcpyHostToDevice, st));
     RTS_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_S, 0, rts_bytes<double>(ctx->M * ctx->N), st));
+    RTS_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_flag + 1, 0, sizeof(int), st));
     rts_inputs_written(ctx);  // S cleared; the steps relax the Illum
     ctx->solve_precision = precision;
     ctx->solve_lambda = lambda;
@@ -747,11 +749,15 @@ int rts_solve_step_async(rts_ctx* ctx, int relax)
 
 static int check_device_flag(rts_ctx* ctx)
 {
-    int flag = 0;
-    RTS_CUDA_TRY(ctx, cudaMemcpy(&flag, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost));
-    if (flag)
+    int flag[2] = {};
+    RTS_CUDA_TRY(ctx, cudaMemcpy(flag, ctx->d_flag, sizeof(flag), cudaMemcpyDeviceToHost));
+    if (flag[0])
         return rts_fail(ctx, RTS_ERR_DEVICE_WAIT,
-                        "a bounded device-side wait gave up (code %d); results are invalid", flag);
+                        "a bounded device-side wait gave up (code %d); results are invalid", flag[0]);
+    if (flag[1])
+        return rts_fail(ctx, RTS_ERR_DEVICE_WAIT,
+                        "a bounded wait of an FP64 step gave up (code %d): its S was computed again, its residual is "
+                        "not known", flag[1]);
     return RTS_OK;
 }
 
@@ -837,6 +843,18 @@ int rts_synth_illum(rts_ctx* ctx, uint64_t seed, double mu, double sigma, int in
     return rts_launch_synth(ctx, seed, mu, sigma, independent_faces);
 }
 
+int rts_fp64_stats(rts_ctx* ctx, int64_t* passes, int64_t* listed, int64_t* gave_up)
+{
+    if (!ctx) return RTS_ERR_INVALID_ARGUMENT;
+    unsigned long long n[2] = {};
+    RTS_CUDA_TRY(ctx, cudaDeviceSynchronize());
+    RTS_CUDA_TRY(ctx, cudaMemcpy(n, ctx->d_fp64, sizeof(n), cudaMemcpyDeviceToHost));
+    if (passes) *passes = ctx->fp64_passes;
+    if (listed) *listed = (int64_t)n[0];
+    if (gave_up) *gave_up = (int64_t)n[1];
+    return RTS_OK;
+}
+
 int rts_set_tuning(rts_ctx* ctx, int key, int value)
 {
     if (!ctx) return RTS_ERR_INVALID_ARGUMENT;
@@ -864,7 +882,7 @@ int rts_set_tuning(rts_ctx* ctx, int key, int value)
         if (ctx->sweep) ctx->sweep->att_valid = false;
         return RTS_OK;
     case RTS_TUNE_FP64_DIGITS:
-        RTS_REQUIRE(ctx, value == 0 || value == 1, RTS_ERR_INVALID_ARGUMENT, "FP64 digits switch %d not 0 or 1", value);
+        RTS_REQUIRE(ctx, value >= 0 && value <= 2, RTS_ERR_INVALID_ARGUMENT, "FP64 digits switch %d not 0 to 2", value);
         ctx->fp64_digits = value;
         return RTS_OK;
     case RTS_TUNE_BIAS:

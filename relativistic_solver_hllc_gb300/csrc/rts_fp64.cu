@@ -265,18 +265,27 @@ scatter_fp64_small_kernel(const double* __restrict__ illum, const double* __rest
 // The outputs that the tensor-core route left (rts_launch_scatter_list): a few
 // CTAs walk the tiles of the listed cells; count and list are the device's, so
 // nothing waits on the host.  Usually there are none and the launch costs its
-// latency.
+// latency.  stats: counts of listed rows and of contractions that gave up;
+// residual_flag: set where one of a step with a residual did.
 template <bool kUpdate, bool kResidual>
 __global__ void __launch_bounds__(F64_THREADS, 2)
 scatter_list_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t n, int64_t N, int M,
                     int ldw, int k_begin, int k_end, double* __restrict__ S, const double* __restrict__ B,
                     double lambda, unsigned long long* __restrict__ resid, ListArgs fx,
-                    const unsigned int* __restrict__ count)
+                    const unsigned int* __restrict__ count, unsigned long long* stats, int* residual_flag)
 {
     __shared__ double sI[F64_KC][F64_TC];
     __shared__ double sW[F64_KC][F64_TK];
     const bool whole = count[1] != 0;  // the contraction gave up: every output of the range
     const int64_t cells = whole ? n : (int64_t)count[0];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (whole) {
+            atomicAdd(stats + 1, 1ull);
+            if (kResidual) atomicOr(residual_flag, (int)count[1]);
+        } else if (count[0]) {
+            atomicAdd(stats, (unsigned long long)count[0]);
+        }
+    }
     if (whole) fx.list = fx.mask = nullptr;
     const int gy = (k_end - k_begin + F64_TK - 1) / F64_TK;
     const int64_t work = (cells + F64_TC - 1) / F64_TC * gy;
@@ -698,7 +707,7 @@ int rts_launch_scatter_list(rts_ctx* ctx, int64_t c0, int64_t n, int64_t k_begin
                                       : scatter_list_kernel<false, false>;
     kernel<<<grid, F64_THREADS, 0, st>>>(ctx->d_illum + 4 * c0, ctx->d_W, n, ctx->N, (int)ctx->M, (int)ctx->local(),
                                          (int)k_begin, (int)k_end, ctx->d_S + c0, update ? B + c0 : nullptr, lambda,
-                                         ctx->resid_target, fx, count);
+                                         ctx->resid_target, fx, count, ctx->d_fp64, ctx->d_flag + 1);
     RTS_CHECK_LAUNCH(ctx, "scatter_list_kernel");
     ctx->launches++;
     return RTS_OK;

@@ -158,6 +158,8 @@ struct rts_sweep_state {
 };
 void rts_sweep_free(rts_ctx* ctx);
 
+constexpr size_t RTS_FLAG_BYTES = 32;  // rts_ctx::d_flag (4 words) and d_fp64 (2)
+
 struct rts_ctx {
     int device = 0;
     int num_sms = 0;
@@ -194,7 +196,11 @@ struct rts_ctx {
     // rts_source_update, slots 1..RTS_RESID_CAP a ring of per-step residuals
     unsigned long long* d_resid = nullptr;
     unsigned long long* resid_target = nullptr;  // slot the next kernels reduce into
-    int* d_flag = nullptr;       // device-side error flag of bounded waits
+    // device-side error flags of bounded waits: [0] the tensor precisions', [1] an FP64 step's whose residual is
+    // lost; [2] the sweep structures'
+    int* d_flag = nullptr;
+    unsigned long long* d_fp64 = nullptr;  // behind them, counts: rows listed, contractions that gave up (rts_sliced.cu)
+    int64_t fp64_passes = 0;     // its contractions queued
     cudaMemPool_t pool = nullptr;  // stream-ordered pool of the batched problems' buffers (created on first use)
     cudaStream_t serve_copy = nullptr;  // read-backs of finished serving requests
     cudaStream_t serve_admit = nullptr;  // set-up of admitted serving requests (lowest priority)
@@ -263,7 +269,8 @@ void rts_sliced_free(rts_ctx* ctx);
 // Its rows that the digits could not carry, by the FP64 kernel: cells
 // list[0..*count) of the range starting at c0, the outputs marked in mask
 // [quarter tile][mask_ld], a bit per column (tiles of bn columns).  With
-// count[1] set (a bounded wait of the contraction gave up) all n cells whole.
+// count[1] set (a bounded wait of the contraction gave up) all n cells whole; a
+// residual asked for is then lost (S was partly replaced): d_flag[1] says so.
 int rts_launch_scatter_list(rts_ctx* ctx, int64_t c0, int64_t n, int64_t k_begin, int64_t k_end, int bn,
                             int64_t mask_ld, const unsigned int* mask, const unsigned int* list,
                             const unsigned int* count, cudaStream_t st, const double* B, double lambda, bool update,

@@ -614,6 +614,7 @@ int rts_sliced_scatter(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_b
             const int64_t n = std::min(step, c_end - c0);
             const double* illum = ctx->d_illum + 4 * c0;
             RTS_CUDA_TRY(ctx, cudaMemsetAsync(rows.count, 0, 8, st));
+            if (ctx->fp64_digits == 2) RTS_CUDA_TRY(ctx, cudaMemsetAsync(rows.count + 1, 1, 4, st));
             if ((rc2 = rts_pp_slice_rows(ctx, illum, n, N, (int)M, (int)kpad, A, rows.exps, rows.flags, rows.list,
                                          rows.count, st)) != RTS_OK)
                 return rc2;
@@ -642,6 +643,7 @@ int rts_sliced_scatter(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_b
             rts_timing_end(ctx, st);
             RTS_CHECK_LAUNCH(ctx, "sliced_kernel");
             ctx->launches++;
+            ctx->fp64_passes++;
             if ((rc2 = rts_launch_scatter_list(ctx, c0, n, k_begin, k_end, bn, step, mask, rows.list, rows.count, st, B,
                                                lambda, update, residual)) != RTS_OK)
                 return rc2;

@@ -1,0 +1,87 @@
+"""What the FP64 integrals' digit products report of themselves: that they ran,
+which rows they left to the FP64 cores, and contractions that gave up."""
+import numpy as np
+import pytest
+
+import oracle
+from relativistic_solver_hllc_gb300 import PHASE_HG, RtsError, _native
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12  # the FP64 contract, relative
+
+
+def rel_err(a, b):
+    return float(np.max(np.abs(a - b) / np.abs(b)))
+
+
+def hg_weights(xyz, area, g):
+    w = area[:, None] * (1 - g * g) / (4 * np.pi * (1 + g * g - 2 * g * (xyz @ xyz.T)) ** 1.5)
+    return w / w.sum(axis=0, keepdims=True)
+
+
+def rows_left(W, il, N, M):
+    """Rows with an output below half of 2^(exponent of the row's largest face
+    sum + exponent of the column's largest weight), or without digits."""
+    sums = 4.0 * oracle.face_mean(il, N, M)
+    top = sums.max(axis=0)
+    bad = (sums.min(axis=0) < 0) | ~np.isfinite(top) | (np.abs(np.frexp(top)[1]) > 900)
+    e_row, e_col = np.frexp(top)[1], np.frexp(W.max(axis=0))[1]
+    with np.errstate(all="ignore"):
+        low = (W.T @ sums < 0.5 * np.ldexp(1.0, e_row[None, :] + e_col[:, None])).any(axis=0)
+    return int((bad | (low & (top > 0))).sum())
+
+
+@pytest.mark.parametrize("M,N,g,sigma", [(64, 4001, None, 1.0), (100, 3000, None, 1.5), (257, 300, None, 1.0),
+                                         (200, 1001, 0.5, 1.0), (200, 1001, 0.6, 1.5)])
+def test_digits_run_and_list_their_rows(ctx, M, N, g, sigma):
+    xyz, area, fa = oracle.fibonacci_directions(M)
+    il = oracle.illum(M, 0.0, sigma, N, M, independent_faces=True).reshape(M, N, 4)
+    il[M // 2, 11::401] *= 1e6   # one direction carries these rows
+    il[0, 7::301, 1] *= -1e5     # and these have a negative value
+    il[:, 5::211] = 0.0
+    il = np.ascontiguousarray(il).ravel()
+    ctx.init(xyz, area, fa, N)
+    if g is not None:
+        ctx.set_phase(PHASE_HG, g)
+    W = hg_weights(xyz, area, g) if g is not None else oracle.weights_thomson(xyz, area, fa)
+    left = rows_left(W, il, N, M)
+    assert left > 0
+    assert ctx.fp64_stats() == (0, 0, 0)
+    ctx.scattering(il)
+    assert ctx.fp64_stats() == (1, left, 0)
+    ctx.set_tuning(_native.TUNE_FP64_DIGITS, 0)
+    ctx.scattering(il)
+    assert ctx.fp64_stats() == (1, left, 0)
+
+
+@pytest.mark.parametrize("M,N", [(100, 1500), (200, 700)])
+def test_a_contraction_that_gives_up(ctx, M, N):
+    """Its outputs are computed again as the FP64 cores' chain; a step's residual
+    is reported as lost, until the next set-up."""
+    xyz, area, fa = oracle.fibonacci_directions(M)
+    il = oracle.illum(M, 0.0, 1.0, N, M, independent_faces=True)
+    B = oracle.uniform(2, 2, 0.1, 1.0, N)
+    ctx.init(xyz, area, fa, N)
+    S = {}
+    for mode in (0, 2):
+        ctx.set_tuning(_native.TUNE_FP64_DIGITS, mode)
+        S[mode] = ctx.scattering(il)
+    assert np.array_equal(S[0], S[2])
+    assert rel_err(S[2], oracle.calculate_int_cpu(N, xyz, area, fa, il)) <= TOL
+    assert ctx.fp64_stats() == (1, 0, 1)
+    ctx.copy_illum(il)
+    ctx.solve_setup("fp64", B, 0.9)
+    with pytest.raises(RtsError) as err:
+        ctx.solve_step(True)
+    assert err.value.status == _native.ERR_DEVICE_WAIT
+    ctx.set_tuning(_native.TUNE_FP64_DIGITS, 1)
+    ctx.solve_step_async(True)
+    with pytest.raises(RtsError):
+        ctx.solve_residual_history(2)
+    ctx.copy_illum(il)
+    ctx.solve_setup("fp64", B, 0.9)
+    W = oracle.weights_thomson(xyz, area, fa)
+    _, ref, _ = oracle.iterate(W, oracle.face_mean(il, N, M), B, 0.9, 2, True)
+    res = [ctx.solve_step(True) for _ in range(2)]
+    assert np.max(np.abs(np.array(res) - np.array(ref)) / np.array(ref)) <= 1e-11
+    assert ctx.fp64_stats()[2] == 2
