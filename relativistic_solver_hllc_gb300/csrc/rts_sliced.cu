@@ -532,9 +532,9 @@ constexpr int64_t S_ROWS_BYTES = (int64_t)1 << 31;
 // without a sharp peak (Thomson, or Henyey-Greenstein, whose largest weight
 // over the column mean is at most M / 16; the outputs of rows whose largest
 // value towers above the mean are then rarely below the accuracy limit), and
-// enough work.  Depends on the grid and the weights only, so that every range
-// of cells and out-directions of a context takes the same route and rows
-// covered by two calls agree bit for bit.
+// enough work.  Depends on the whole grid and the weights only, so that every
+// range of cells and out-directions, and every shard of the out-directions,
+// takes the same route and outputs covered twice agree bit for bit.
 //
 // The size limit.  The digit rows, the contraction and the list pass take about
 // 22 us + 0.14 us M at the smallest sizes, whatever the cells; the 32 x 32 tiles
@@ -549,7 +549,7 @@ static bool sliced_fits(const rts_ctx* ctx)
     const int64_t N = ctx->N, M = ctx->M;
     size_t smem = 0;
     if (M < 48 || N >= ((int64_t)1 << 31) || rts_rows::cells_log2((int)kpad_of(ctx), &smem) == 0) return false;
-    if (M < 160 && (double)N * (double)M * (double)ctx->local() < 1.0e7) return false;
+    if (M < 160 && (double)N * (double)M * (double)M < 1.0e7) return false;  // M, not the shard's share of it
     double peak;
     if (ctx->phase == RTS_PHASE_THOMSON)
         peak = 1.5;

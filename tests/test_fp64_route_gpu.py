@@ -85,3 +85,16 @@ def test_a_contraction_that_gives_up(ctx, M, N):
     res = [ctx.solve_step(True) for _ in range(2)]
     assert np.max(np.abs(np.array(res) - np.array(ref)) / np.array(ref)) <= 1e-11
     assert ctx.fp64_stats()[2] == 2
+
+
+@pytest.mark.parametrize("M,N", [(64, 2600), (100, 1500), (159, 500)])
+def test_shards_take_the_route_of_the_whole(ctx, M, N):
+    """Just above the size limit of the whole direction set: a shard of the
+    out-directions gives the bits that all of them give."""
+    xyz, area, fa = oracle.fibonacci_directions(M)
+    il = oracle.illum(M, 0.0, 1.0, N, M, independent_faces=True)
+    ctx.init(xyz, area, fa, N)
+    whole = ctx.scattering(il)
+    for lo, hi in ((0, M // 2), (M // 2, M - 3), (M - 3, M)):
+        ctx.init(xyz, area, fa, N, lo, hi)
+        assert np.array_equal(ctx.scattering(il), whole[lo:hi])
