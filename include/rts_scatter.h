@@ -150,8 +150,9 @@ int rts_copy_illum(rts_ctx* ctx, int64_t size, const double* illum_host);
  * RTS_PREC_FP64 computes with FP64's accuracy on either the FP64 CUDA cores
  * or, for Thomson and smooth Henyey-Greenstein kernels on sm_10x, the tensor
  * cores (exact products of FP16 digits, integer sums), which hold 12 bytes per
- * direction pair and, during a call, up to 2 GB of scratch; without that room
- * the CUDA cores run. */
+ * direction pair and, during a call, up to 2 GB of scratch (with less room the
+ * call takes more passes, down to some 30 MB; without it, or on a capturing
+ * stream, the CUDA cores run, whose results differ in the last bits). */
 int rts_set_precision(rts_ctx* ctx, int precision);
 int rts_get_precision(const rts_ctx* ctx, int* precision);
 

@@ -523,7 +523,7 @@ int ensure_w(rts_ctx* ctx, cudaStream_t st)
     return RTS_OK;
 }
 
-// Device bytes of the digit rows of one pass over a range of cells.
+// Device bytes of the digit rows of one pass over a range of cells, at most.
 constexpr int64_t S_ROWS_BYTES = (int64_t)1 << 31;
 
 }  // namespace
@@ -534,7 +534,9 @@ constexpr int64_t S_ROWS_BYTES = (int64_t)1 << 31;
 // value towers above the mean are then rarely below the accuracy limit), and
 // enough work.  Depends on the whole grid and the weights only, so that every
 // range of cells and out-directions, and every shard of the out-directions,
-// takes the same route and outputs covered twice agree bit for bit.
+// takes the same route and outputs covered twice agree bit for bit.  A call
+// without room for its scratch, or on a capturing stream, takes the FP64 cores
+// all the same, and differs in the last bits.
 //
 // The size limit.  The digit rows, the contraction and the list pass take about
 // 22 us + 0.14 us M at the smallest sizes, whatever the cells; the 32 x 32 tiles
@@ -589,16 +591,22 @@ int rts_sliced_scatter(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_b
     const int n_tiles = (int)((cols + S_BN - 1) / S_BN);
     // tile width: the out-directions balanced over the tiles, in steps of 16 and at least 64
     const int bn = (int)std::max<int64_t>(64, ((cols + n_tiles - 1) / n_tiles + 15) / 16 * 16);
-    // cells per pass: whole 128-cell tiles within the scratch limit
-    const int64_t row_bytes = SLICES * kpad * 2;
-    const int64_t per = std::max<int64_t>(1, S_ROWS_BYTES / (S_BM * row_bytes)) * S_BM;
-    const int64_t passes = (c_end - c_begin + per - 1) / per;
-    const int64_t step = ((c_end - c_begin + passes - 1) / passes + S_BM - 1) / S_BM * S_BM;
-    const size_t a_bytes = (size_t)(step * row_bytes), m_bytes = (size_t)(n_tiles * 4 * step * 4);
-    const size_t l_bytes = (size_t)(step * 12 + 16);
-    const size_t bytes = a_bytes + m_bytes + l_bytes;
+    // cells per pass: whole 128-cell tiles within the scratch limit, and half as many as long as there is no room for
+    // them and they make a tile for every SM (the passes change no output)
+    const int64_t row_bytes = SLICES * kpad * 2, wave = (ctx->num_sms + n_tiles - 1) / n_tiles * S_BM;
+    int64_t per = std::max<int64_t>(1, S_ROWS_BYTES / (S_BM * row_bytes)) * S_BM, step;
+    size_t a_bytes, m_bytes, bytes;
     void* scratch = nullptr;
-    if ((rc = rts_pmalloc(ctx, &scratch, bytes, "FP64 digit rows", st)) != RTS_OK) return no_room(rc);
+    for (;; per = step / 2) {
+        const int64_t passes = (c_end - c_begin + per - 1) / per;
+        step = ((c_end - c_begin + passes - 1) / passes + S_BM - 1) / S_BM * S_BM;
+        a_bytes = (size_t)(step * row_bytes), m_bytes = (size_t)(n_tiles * 4 * step * 4);
+        bytes = a_bytes + m_bytes + (size_t)(step * 12 + 16);  // and the row list
+        rc = rts_pmalloc(ctx, &scratch, bytes, "FP64 digit rows", st);
+        if (rc == RTS_OK) break;
+        if ((rc != RTS_ERR_OVER_BUDGET && rc != RTS_ERR_OUT_OF_MEMORY) || step / 2 < wave) return no_room(rc);
+    }
+    ctx->last_error = keep;
     uint16_t* A = (uint16_t*)scratch;
     unsigned int* mask = (unsigned int*)((char*)scratch + a_bytes);
     int* exps = (int*)((char*)scratch + a_bytes + m_bytes);

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 import oracle
-from relativistic_solver_hllc_gb300 import PHASE_HG, RtsError, _native
+from relativistic_solver_hllc_gb300 import PHASE_HG, STREAM_SCATTERING_1, RtsError, _native
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-12  # the FP64 contract, relative
@@ -98,3 +98,47 @@ def test_shards_take_the_route_of_the_whole(ctx, M, N):
     for lo, hi in ((0, M // 2), (M // 2, M - 3), (M - 3, M)):
         ctx.init(xyz, area, fa, N, lo, hi)
         assert np.array_equal(ctx.scattering(il), whole[lo:hi])
+
+
+def test_less_scratch_takes_more_passes(ctx):
+    """A tight budget cuts a call into passes with the same bits; without room for
+    a tile per SM the FP64 cores run, within the same tolerance."""
+    M, N = 200, 60001
+    xyz, area, fa = oracle.fibonacci_directions(M)
+    il = oracle.illum(8, 0.0, 1.0, N, M, independent_faces=True).reshape(M, N, 4)
+    il[M // 2, 11::4001] *= 1e6  # rows left to the FP64 cores, in every pass
+    il = np.ascontiguousarray(il).ravel()
+    ctx.init(xyz, area, fa, N)
+    S = ctx.scattering(il)
+    used = ctx.hbm_used()
+    one, listed, _ = ctx.fp64_stats()
+    assert one == 1 and listed == len(range(11, N, 4001))
+    ctx.set_hbm_budget(used + (50 << 20))  # the digit rows of all cells take 161 MB
+    assert np.array_equal(ctx.scattering(il), S)
+    assert ctx.fp64_stats() == (5, 2 * listed, 0)
+    ctx.set_hbm_budget(used + (4 << 20))
+    chain = ctx.scattering(il)
+    assert ctx.fp64_stats() == (5, 2 * listed, 0)
+    ctx.set_hbm_budget(1 << 36)
+    ctx.set_tuning(_native.TUNE_FP64_DIGITS, 0)
+    assert np.array_equal(chain, ctx.scattering(il)) and rel_err(chain, S) <= TOL
+
+
+def test_a_capturing_stream_takes_the_chain(ctx):
+    torch = pytest.importorskip("torch")
+    M, N = 100, 1500
+    xyz, area, fa = oracle.fibonacci_directions(M)
+    il = oracle.illum(4, 0.0, 1.0, N, M, independent_faces=True)
+    ctx.init(xyz, area, fa, N)
+    ctx.set_tuning(_native.TUNE_FP64_DIGITS, 0)
+    chain = ctx.scattering(il)
+    ctx.set_tuning(_native.TUNE_FP64_DIGITS, 1)
+    out = ctx.host_scattering()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.ExternalStream(ctx.stream_handle(STREAM_SCATTERING_1))):
+        ctx.scattering_async(0, M, STREAM_SCATTERING_1, out)
+    out[:] = 0.0
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(out.reshape(M, N), chain)
+    assert ctx.fp64_stats() == (0, 0, 0)
