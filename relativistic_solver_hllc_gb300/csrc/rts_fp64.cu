@@ -21,6 +21,7 @@
 // design; memory traffic is ~40 B per cell-direction pair over M in-directions.
 #include <cstdint>
 #include <mutex>
+#include <type_traits>
 
 #include "rts_internal.h"
 
@@ -189,19 +190,20 @@ scatter_fp64_kernel(const double* __restrict__ illum, const double* __restrict__
 // leave SMs idle: 2,000 x 64 makes 16 of those, each a serial loop of loads,
 // barriers and FMAs (152 us), and 126 of these (23 us).  A chunk's operands are
 // loaded while the previous one is multiplied, one barrier a chunk.  Every output
-// is the same FMA chain as in the larger tiles.
+// is the same FMA chain as in the larger tiles.  kList as in scatter_tile.
 constexpr int S64_T = 32, S64_KC = 16, S64_THREADS = 256;
-template <bool kUpdate>
-__global__ void __launch_bounds__(S64_THREADS)
-scatter_fp64_small_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t n, int64_t N, int M,
-                          int ldw, int k_begin, int k_end, double* __restrict__ S, const double* __restrict__ B,
-                          double lambda, unsigned long long* __restrict__ resid)
+template <bool kUpdate, bool kList = false>
+__device__ __forceinline__ void scatter_small_tile(double (*sI)[S64_KC][S64_T], double (*sW)[S64_KC][S64_T],
+                                                   const double* __restrict__ illum, const double* __restrict__ W,
+                                                   int64_t c0, int64_t n, int64_t N, int M, int ldw, int k0, int k_end,
+                                                   double* __restrict__ S, const double* __restrict__ B, double lambda,
+                                                   unsigned long long* __restrict__ resid,
+                                                   const ListArgs& fx = ListArgs())
 {
-    __shared__ double sI[2][S64_KC][S64_T], sW[2][S64_KC][S64_T];
     constexpr int PER = S64_KC * S64_T / S64_THREADS;  // pairs of a chunk per thread: 2
     const int tx = threadIdx.x & (S64_T - 1), ty = threadIdx.x / S64_T;
-    const int64_t c = (int64_t)blockIdx.x * S64_T + tx;
-    const int k0 = k_begin + (int)blockIdx.y * S64_T;
+    const bool in = c0 + tx < n;
+    const int64_t c = kList && in && fx.list ? (int64_t)fx.list[c0 + tx] : c0 + tx;
     double2 p[PER], q[PER];
     double w[PER];
     auto load = [&](int j0) {
@@ -209,7 +211,7 @@ scatter_fp64_small_kernel(const double* __restrict__ illum, const double* __rest
         for (int i = 0; i < PER; ++i) {
             const int j = j0 + ty + (S64_THREADS / S64_T) * i;
             p[i] = q[i] = make_double2(0.0, 0.0);
-            if (j < M && c < n) {
+            if (j < M && in) {
                 const double2* src = reinterpret_cast<const double2*>(illum + ((int64_t)j * N + c) * 4);
                 p[i] = __ldg(src);
                 q[i] = __ldg(src + 1);
@@ -247,11 +249,11 @@ scatter_fp64_small_kernel(const double* __restrict__ illum, const double* __rest
         }
     }
     double rmax = 0.0;
-    if (c < n) {
+    if (in) {
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
             const int k = k0 + ty + 8 * m;
-            if (k >= k_end) continue;
+            if (k >= k_end || (kList && !fx.marked(c, k))) continue;
             double v = acc[m];
             if (kUpdate) v = (1.0 - lambda) * B[c] + lambda * v;
             double* dst = S + (int64_t)k * N + c;
@@ -262,36 +264,15 @@ scatter_fp64_small_kernel(const double* __restrict__ illum, const double* __rest
     if (resid) residual_max(resid, rmax);
 }
 
-// The outputs that the tensor-core route left (rts_launch_scatter_list): a few
-// CTAs walk the tiles of the listed cells; count and list are the device's, so
-// nothing waits on the host.  Usually there are none and the launch costs its
-// latency.  stats: counts of listed rows and of contractions that gave up;
-// residual_flag: set where one of a step with a residual did.
-template <bool kUpdate, bool kResidual>
-__global__ void __launch_bounds__(F64_THREADS, 2)
-scatter_list_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t n, int64_t N, int M,
-                    int ldw, int k_begin, int k_end, double* __restrict__ S, const double* __restrict__ B,
-                    double lambda, unsigned long long* __restrict__ resid, ListArgs fx,
-                    const unsigned int* __restrict__ count, unsigned long long* stats, int* residual_flag)
+template <bool kUpdate>
+__global__ void __launch_bounds__(S64_THREADS)
+scatter_fp64_small_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t n, int64_t N, int M,
+                          int ldw, int k_begin, int k_end, double* __restrict__ S, const double* __restrict__ B,
+                          double lambda, unsigned long long* __restrict__ resid)
 {
-    __shared__ double sI[F64_KC][F64_TC];
-    __shared__ double sW[F64_KC][F64_TK];
-    const bool whole = count[1] != 0;  // the contraction gave up: every output of the range
-    const int64_t cells = whole ? n : (int64_t)count[0];
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (whole) {
-            atomicAdd(stats + 1, 1ull);
-            if (kResidual) atomicOr(residual_flag, (int)count[1]);
-        } else if (count[0]) {
-            atomicAdd(stats, (unsigned long long)count[0]);
-        }
-    }
-    if (whole) fx.list = fx.mask = nullptr;
-    const int gy = (k_end - k_begin + F64_TK - 1) / F64_TK;
-    const int64_t work = (cells + F64_TC - 1) / F64_TC * gy;
-    for (int64_t w = blockIdx.x; w < work; w += gridDim.x)
-        scatter_tile<kUpdate, kResidual, 4, true>(sI, sW, illum, W, w / gy * F64_TC, cells, N, M, ldw,
-                                                  k_begin + (int)(w % gy) * F64_TK, k_end, S, B, lambda, resid, fx);
+    __shared__ double sI[2][S64_KC][S64_T], sW[2][S64_KC][S64_T];
+    scatter_small_tile<kUpdate>(sI, sW, illum, W, (int64_t)blockIdx.x * S64_T, n, N, M, ldw,
+                                k_begin + (int)blockIdx.y * S64_T, k_end, S, B, lambda, resid);
 }
 
 // The y extent of scatter_fp64_kernel's grid over `width` out-directions.
@@ -306,6 +287,82 @@ inline DirTiles dir_tiles(int64_t width)
     t.nb_last = rem ? (rem + 15) / 16 : 4;
     t.gy = t.n_full + (rem ? 1 : 0);
     return t;
+}
+
+// The outputs that the tensor-core route left (rts_launch_scatter_list): CTAs
+// walk the tiles of the listed cells; count and list are the device's, so nothing
+// waits on the host.  Usually there are none and the launch costs its latency.
+// Rows that fill waves of the large tiles (two a SM) take those, the rest and
+// shorter lists the 32 x 32 tiles, whose serial loop is an eighth as long (0.31
+// us M against 2.2): a step of 40 x 1000 with one listed row 2,355 -> 478 us, of
+// 20,000 x 400 with every row listed 7.70 -> 6.32 ms.  `taken` (zero before the
+// launch) hands out the tiles, large, narrow, small, so that no SM is left with
+// a large one at the end; small ones alone go round the CTAs, so that no SM takes
+// two of the last (865 rows of 20,000 x 400: 0.79 ms a step, 0.90 handed out).
+// stats: counts of listed rows and of contractions that gave up; residual_flag:
+// set where one of a step with a residual did.
+template <bool kUpdate, bool kResidual>
+__global__ void __launch_bounds__(F64_THREADS, 2)
+scatter_list_kernel(const double* __restrict__ illum, const double* __restrict__ W, int64_t n, int64_t N, int M,
+                    int ldw, int k_begin, int k_end, DirTiles dt, int num_sms, double* __restrict__ S,
+                    const double* __restrict__ B, double lambda, unsigned long long* __restrict__ resid, ListArgs fx,
+                    const unsigned int* __restrict__ count, unsigned int* taken, unsigned long long* stats,
+                    int* residual_flag)
+{
+    static_assert(F64_THREADS == S64_THREADS, "one launch for both tiles");
+    __shared__ double mem[F64_KC * (F64_TC + F64_TK)];
+    __shared__ unsigned int next;
+    static_assert(sizeof(mem) >= sizeof(double) * 4 * S64_KC * S64_T, "both tiles' operands");
+    const bool whole = count[1] != 0;  // the contraction gave up: every output of the range
+    const int64_t cells = whole ? n : (int64_t)count[0];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (whole) {
+            atomicAdd(stats + 1, 1ull);
+            if (kResidual) atomicOr(residual_flag, (int)count[1]);
+        } else if (count[0]) {
+            atomicAdd(stats, (unsigned long long)count[0]);
+        }
+    }
+    if (whole) fx.list = fx.mask = nullptr;
+    // whole waves of large tiles, in quarter tiles (16 out-directions); the rest in small ones
+    const int per_row = 4 * dt.n_full + (dt.gy > dt.n_full ? dt.nb_last : 0), wave = 8 * num_sms;
+    const int64_t rows = cells / F64_TC * per_row / wave * wave / per_row;
+    const int64_t full = rows * dt.n_full, large = rows * dt.gy, c_small = rows * F64_TC;
+    const int gs = (k_end - k_begin + S64_T - 1) / S64_T;
+    const int64_t work = large + (cells - c_small + S64_T - 1) / S64_T * gs;
+    auto tile = [&](auto nb, int64_t row, int col) {
+        auto* sI = reinterpret_cast<double(*)[F64_TC]>(mem);
+        auto* sW = reinterpret_cast<double(*)[F64_TK]>(mem + F64_KC * F64_TC);
+        scatter_tile<kUpdate, kResidual, decltype(nb)::value, true>(sI, sW, illum, W, row * F64_TC, cells, N, M, ldw,
+                                                                    k_begin + col * F64_TK, k_end, S, B, lambda, resid,
+                                                                    fx);
+    };
+    int64_t w = blockIdx.x;
+    while (w < work) {
+        if (w < full) {
+            tile(std::integral_constant<int, 4>{}, w / dt.n_full, (int)(w % dt.n_full));
+        } else if (w < large) {
+            switch (dt.nb_last) {
+            case 1: tile(std::integral_constant<int, 1>{}, w - full, dt.n_full); break;
+            case 2: tile(std::integral_constant<int, 2>{}, w - full, dt.n_full); break;
+            case 3: tile(std::integral_constant<int, 3>{}, w - full, dt.n_full); break;
+            default: tile(std::integral_constant<int, 4>{}, w - full, dt.n_full); break;
+            }
+        } else {
+            auto* sI = reinterpret_cast<double(*)[S64_KC][S64_T]>(mem);
+            scatter_small_tile<kUpdate, true>(sI, sI + 2, illum, W, c_small + (w - large) / gs * S64_T, cells, N, M, ldw,
+                                              k_begin + (int)((w - large) % gs) * S64_T, k_end, S, B, lambda,
+                                              kResidual ? resid : nullptr, fx);
+        }
+        __syncthreads();  // the operands and the last number are read
+        if (large == 0) {
+            w += gridDim.x;
+            continue;
+        }
+        if (threadIdx.x == 0) next = atomicAdd(taken, 1u);
+        __syncthreads();
+        w = (int64_t)gridDim.x + next;
+    }
 }
 
 // Which of the two kernels: the larger tiles need four a SM (two resident at a
@@ -696,18 +753,20 @@ int rts_launch_scatter_fp64_cells(rts_ctx* ctx, int64_t c_begin, int64_t c_end, 
 
 int rts_launch_scatter_list(rts_ctx* ctx, int64_t c0, int64_t n, int64_t k_begin, int64_t k_end, int bn,
                             int64_t mask_ld, const unsigned int* mask, const unsigned int* list,
-                            const unsigned int* count, cudaStream_t st, const double* B, double lambda, bool update,
+                            unsigned int* count, cudaStream_t st, const double* B, double lambda, bool update,
                             bool residual)
 {
     const ListArgs fx{list, mask, mask_ld, bn, (int)k_begin};
-    const int64_t tiles = (n + F64_TC - 1) / F64_TC * ((k_end - k_begin + F64_TK - 1) / F64_TK);
+    const dim3 most = small_grid(n, k_end - k_begin);
+    const int64_t tiles = (int64_t)most.x * most.y;
     const unsigned grid = (unsigned)(tiles < 2 * ctx->num_sms ? tiles : 2 * ctx->num_sms);
     auto* kernel = update && residual ? scatter_list_kernel<true, true>
                    : update           ? scatter_list_kernel<true, false>
                                       : scatter_list_kernel<false, false>;
     kernel<<<grid, F64_THREADS, 0, st>>>(ctx->d_illum + 4 * c0, ctx->d_W, n, ctx->N, (int)ctx->M, (int)ctx->local(),
-                                         (int)k_begin, (int)k_end, ctx->d_S + c0, update ? B + c0 : nullptr, lambda,
-                                         ctx->resid_target, fx, count, ctx->d_fp64, ctx->d_flag + 1);
+                                         (int)k_begin, (int)k_end, dir_tiles(k_end - k_begin), ctx->num_sms,
+                                         ctx->d_S + c0, update ? B + c0 : nullptr, lambda, ctx->resid_target, fx, count,
+                                         count + 2, ctx->d_fp64, ctx->d_flag + 1);
     RTS_CHECK_LAUNCH(ctx, "scatter_list_kernel");
     ctx->launches++;
     return RTS_OK;

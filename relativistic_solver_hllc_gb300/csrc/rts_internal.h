@@ -268,12 +268,13 @@ int rts_sliced_scatter(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_b
 void rts_sliced_free(rts_ctx* ctx);
 // Its rows that the digits could not carry, by the FP64 kernel: cells
 // list[0..*count) of the range starting at c0, the outputs marked in mask
-// [quarter tile][mask_ld], a bit per column (tiles of bn columns).  With
+// [quarter tile][mask_ld], a bit per column (tiles of bn columns); count[2] is
+// zero and used up.  With
 // count[1] set (a bounded wait of the contraction gave up) all n cells whole; a
 // residual asked for is then lost (S was partly replaced): d_flag[1] says so.
 int rts_launch_scatter_list(rts_ctx* ctx, int64_t c0, int64_t n, int64_t k_begin, int64_t k_end, int bn,
                             int64_t mask_ld, const unsigned int* mask, const unsigned int* list,
-                            const unsigned int* count, cudaStream_t st, const double* B, double lambda, bool update,
+                            unsigned int* count, cudaStream_t st, const double* B, double lambda, bool update,
                             bool residual);
 int rts_launch_moments(rts_ctx* ctx, cudaStream_t st);
 int rts_launch_illum_params(rts_ctx* ctx, cudaStream_t st);

@@ -530,13 +530,20 @@ constexpr int64_t S_ROWS_BYTES = (int64_t)1 << 31;
 
 // Whether the context's FP64 integrals take the digits: a weight kernel
 // without a sharp peak (Thomson, or Henyey-Greenstein, whose largest weight
-// over the column mean is at most M / 16; the outputs of rows whose largest
-// value towers above the mean are then rarely below the accuracy limit), and
-// enough work.  Depends on the whole grid and the weights only, so that every
+// over the column mean is at most M / 16), and enough work.  Depends on the whole grid and the weights only, so that every
 // range of cells and out-directions, and every shard of the out-directions,
 // takes the same route and outputs covered twice agree bit for bit.  A call
 // without room for its scratch, or on a capturing stream, takes the FP64 cores
 // all the same, and differs in the last bits.
+//
+// The limit of the peak.  How many rows have outputs below the accuracy limit
+// depends on the Illum: few with Thomson's kernel, up to all of them near M / 16
+// where the intensities of a row spread widely (lognormal with sigma 1.5), and
+// then the call pays for the digits and the FP64 cores.  ms a step of 20,000
+// cells, sigma 1 / 1.5, the FP64 cores alone in brackets: M = 100, g = 0.5 0.14 /
+// 0.37 (0.70); 200, 0.6 0.31 / 1.33 (1.87); 400, 0.7 1.18 / 5.98 (6.23); 1000,
+// 0.7 - / 20.7 and 0.8 10.4 / 38.1 (37.1).  With every row listed, whatever the
+// kernel, the digits add 1 to 3 %.
 //
 // The size limit.  The digit rows, the contraction and the list pass take about
 // 22 us + 0.14 us M at the smallest sizes, whatever the cells; the 32 x 32 tiles
@@ -621,7 +628,7 @@ int rts_sliced_scatter(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_b
         for (int64_t c0 = c_begin; c0 < c_end; c0 += step) {
             const int64_t n = std::min(step, c_end - c0);
             const double* illum = ctx->d_illum + 4 * c0;
-            RTS_CUDA_TRY(ctx, cudaMemsetAsync(rows.count, 0, 8, st));
+            RTS_CUDA_TRY(ctx, cudaMemsetAsync(rows.count, 0, 16, st));
             if (ctx->fp64_digits == 2) RTS_CUDA_TRY(ctx, cudaMemsetAsync(rows.count + 1, 1, 4, st));
             if ((rc2 = rts_pp_slice_rows(ctx, illum, n, N, (int)M, (int)kpad, A, rows.exps, rows.flags, rows.list,
                                          rows.count, st)) != RTS_OK)

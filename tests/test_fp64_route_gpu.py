@@ -142,3 +142,30 @@ def test_a_capturing_stream_takes_the_chain(ctx):
     torch.cuda.synchronize()
     assert np.array_equal(out.reshape(M, N), chain)
     assert ctx.fp64_stats() == (0, 0, 0)
+
+
+@pytest.mark.parametrize("M,N", [(80, 32001), (96, 33000), (100, 22501), (120, 19600), (128, 19457),  # waves of large tiles
+                                 (97, 1300), (161, 77)])                                              # small tiles only
+def test_listed_rows_get_the_chain(ctx, M, N):
+    """Rows with a negative value are computed whole on the FP64 cores: with all of
+    them listed every output and the residual have the chain's bits, in the large,
+    the narrow and the small tiles, and for a range of out-directions."""
+    xyz, area, fa = oracle.fibonacci_directions(M)
+    il = oracle.illum(M, 0.0, 1.0, N, M, independent_faces=True).reshape(M, N, 4)
+    il[M // 3] *= -1.0
+    il = np.ascontiguousarray(il).ravel()
+    B = oracle.uniform(2, 2, 0.1, 1.0, N)
+    ctx.init(xyz, area, fa, N)
+    got = {}
+    for mode in (0, 1):
+        ctx.set_tuning(_native.TUNE_FP64_DIGITS, mode)
+        S = ctx.scattering(il)
+        part = np.zeros(M * N)
+        ctx.scattering_async(7, M - 1, STREAM_SCATTERING_1, part)
+        ctx.wait()
+        ctx.solve_setup("fp64", B, 0.9)
+        res = [ctx.solve_step(False) for _ in range(2)]
+        got[mode] = (S, part, ctx.solve_read(), np.array(res))
+    assert ctx.fp64_stats() == (4, 4 * N, 0)
+    for a, b in zip(got[0], got[1]):
+        assert np.array_equal(a, b)
