@@ -730,8 +730,8 @@ int rts_fp64_stats(rts_ctx* ctx, int64_t* passes, int64_t* listed, int64_t* gave
 int rts_launch_count(const rts_ctx* ctx, int64_t* count);
 
 /* CUDA-event timing of the dominant kernel of each integral (the FP64
- * scattering kernel or the tensor-core contraction), recorded on the stream
- * it is launched on.  enable != 0 turns recording on and clears the totals;
+ * scattering kernel or the tensor-core contraction, with what an FP64
+ * contraction left to the FP64 cores), recorded on the stream it is launched on.  enable != 0 turns recording on and clears the totals;
  * total_ms / launches (may be NULL) return what was recorded so far, after
  * synchronising the recorded events. */
 int rts_kernel_timing(rts_ctx* ctx, int enable, double* total_ms, int64_t* launches);

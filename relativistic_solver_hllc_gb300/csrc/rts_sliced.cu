@@ -655,13 +655,13 @@ int rts_sliced_scatter(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_b
             const int64_t grid = std::min<int64_t>(ctx->num_sms, (int64_t)p.m_tiles * n_tiles);
             rts_timing_begin(ctx, st);
             kernel<<<(unsigned)grid, S_THREADS, S_SMEM, st>>>(mapA, mapW, p);
-            rts_timing_end(ctx, st);
             RTS_CHECK_LAUNCH(ctx, "sliced_kernel");
             ctx->launches++;
             ctx->fp64_passes++;
-            if ((rc2 = rts_launch_scatter_list(ctx, c0, n, k_begin, k_end, bn, step, mask, rows.list, rows.count, st, B,
-                                               lambda, update, residual)) != RTS_OK)
-                return rc2;
+            rc2 = rts_launch_scatter_list(ctx, c0, n, k_begin, k_end, bn, step, mask, rows.list, rows.count, st, B, lambda,
+                                          update, residual);
+            rts_timing_end(ctx, st);  // the rows it left are part of the integral's time
+            if (rc2 != RTS_OK) return rc2;
         }
         const int slot = slot_of(ctx, st);
         if (slot >= 0) {

@@ -169,3 +169,24 @@ def test_listed_rows_get_the_chain(ctx, M, N):
     assert ctx.fp64_stats() == (4, 4 * N, 0)
     for a, b in zip(got[0], got[1]):
         assert np.array_equal(a, b)
+
+
+def test_kernel_timing_covers_the_listed_rows(ctx):
+    """With every row listed an integral's time is the FP64 cores' and more."""
+    M, N = 200, 20000
+    xyz, area, fa = oracle.fibonacci_directions(M)
+    il = oracle.illum(M, 0.0, 1.0, N, M, independent_faces=True).reshape(M, N, 4)
+    il[M // 3] *= -1.0
+    ctx.init(xyz, area, fa, N)
+    ctx.copy_illum(il.ravel())
+    ms = {}
+    for mode in (0, 1):
+        ctx.set_tuning(_native.TUNE_FP64_DIGITS, mode)
+        ctx.solve_setup("fp64", np.ones(N), 0.9)
+        ctx.solve_step(False)
+        ctx.kernel_timing(True)
+        for _ in range(3):
+            ctx.solve_step(False)
+        ms[mode], launches = ctx.kernel_timing(False)
+        assert launches == 3
+    assert ms[1] > 0.9 * ms[0]
