@@ -30,10 +30,25 @@ int rts_fail(rts_ctx* ctx, int status, const char* fmt, ...)
     return status;
 }
 
+// Frees what the context can do without, for an allocation that it cannot: no
+// call that fitted before these kept anything may fail for them.
+static bool give_way(rts_ctx* ctx)
+{
+    if (ctx->spare || (!ctx->sliced.w && !ctx->sweep)) return false;
+    if (cudaDeviceSynchronize() != cudaSuccess) {  // kernels in flight may read it
+        cudaGetLastError();
+        return false;
+    }
+    const bool digits = ctx->sliced.w != nullptr;
+    rts_sliced_free(ctx);
+    return rts_sweep_give_way(ctx) || digits;
+}
+
 int rts_dmalloc(rts_ctx* ctx, void** p, size_t bytes, const char* what)
 {
     *p = nullptr;
     if (bytes == 0) return RTS_OK;
+    if (ctx->used_bytes + (int64_t)bytes > ctx->budget_bytes) give_way(ctx);
     if (ctx->used_bytes + (int64_t)bytes > ctx->budget_bytes)
         return rts_fail(ctx, RTS_ERR_OVER_BUDGET,
                         "%s: %zu bytes would exceed the HBM budget (%lld of %lld bytes in use)",
@@ -42,6 +57,10 @@ int rts_dmalloc(rts_ctx* ctx, void** p, size_t bytes, const char* what)
     if (e == cudaErrorMemoryAllocation && ctx->pool) {  // what the scratch pool holds unused goes back first
         cudaGetLastError();
         cudaMemPoolTrimTo(ctx->pool, 0);
+        e = cudaMalloc(p, bytes);
+    }
+    if (e == cudaErrorMemoryAllocation && give_way(ctx)) {
+        cudaGetLastError();
         e = cudaMalloc(p, bytes);
     }
     if (e != cudaSuccess) {
@@ -65,6 +84,7 @@ int rts_pmalloc(rts_ctx* ctx, void** p, size_t bytes, const char* what, cudaStre
 {
     *p = nullptr;
     if (bytes == 0) return RTS_OK;
+    if (ctx->used_bytes + (int64_t)bytes > ctx->budget_bytes) give_way(ctx);
     if (ctx->used_bytes + (int64_t)bytes > ctx->budget_bytes)
         return rts_fail(ctx, RTS_ERR_OVER_BUDGET,
                         "%s: %zu bytes would exceed the HBM budget (%lld of %lld bytes in use)",
@@ -80,6 +100,10 @@ int rts_pmalloc(rts_ctx* ctx, void** p, size_t bytes, const char* what, cudaStre
         RTS_CUDA_TRY(ctx, cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     }
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+    if (e == cudaErrorMemoryAllocation && give_way(ctx)) {
+        cudaGetLastError();
+        e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, st);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         *p = nullptr;
@@ -281,6 +305,7 @@ const char* rts_last_error(const rts_ctx* ctx) { return ctx ? ctx->last_error.c_
 int rts_set_hbm_budget(rts_ctx* ctx, int64_t bytes)
 {
     if (!ctx) return RTS_ERR_INVALID_ARGUMENT;
+    if (bytes < ctx->used_bytes) give_way(ctx);
     RTS_REQUIRE(ctx, bytes >= ctx->used_bytes, RTS_ERR_OVER_BUDGET,
                 "budget %lld below the %lld bytes already held", (long long)bytes,
                 (long long)ctx->used_bytes);

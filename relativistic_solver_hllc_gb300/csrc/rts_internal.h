@@ -116,8 +116,9 @@ struct rts_sliced_state {
 // per-direction structures of the local directions and the medium.  The unit
 // of work is an out-face of a cell (its 3 nodes); per local direction d:
 //   items[d]  out-faces in dependency order: cell << 8 | face << 6 | the
-//             in-faces of its 3 nodes (2 bits each); behind them, with
-//             copy_words, a word per item on the neighbour's copy of its face
+//             in-faces of its 3 nodes (2 bits each)
+//   words[d]  with copy_words, a word per item on the neighbour's copy of its
+//             face; without room for them the sweep forms them itself
 //   recs[d]   3 node distances per item (the LocX0 records' s, same order)
 //   steps[d]  item offsets of the dependency steps (nsteps[d] + 1 entries)
 //   bnd[d]    boundary in-faces, cell * 4 + face (nbnd[d] of them)
@@ -129,20 +130,21 @@ struct rts_sweep_state {
     int32_t* d_pairs = nullptr;      // [N][4]
     double* d_normals = nullptr;     // [N][4][3]
     double* d_nodes = nullptr;       // [N][4][3][3] (MakeArrayX)
-    bool copy_words = true;          // behind every direction's items (false: no room for some)
+    bool copy_words = true;          // false: not wanted, no room for some, or given back
     uint32_t** d_items = nullptr;    // device pointer tables [D]
+    uint32_t** d_words = nullptr;
     double** d_recs = nullptr;
     int32_t** d_steps = nullptr;
     uint32_t** d_bnd = nullptr;
     int32_t* d_nsteps = nullptr;     // [D]
     int32_t* d_nbnd = nullptr;       // [D]
-    std::vector<uint32_t*> h_items;  // host copies of the tables
+    std::vector<uint32_t*> h_items, h_words;  // host copies of the tables
     std::vector<double*> h_recs;
     std::vector<int32_t*> h_steps;
     std::vector<uint32_t*> h_bnd;
     std::vector<int32_t> h_nsteps, h_nbnd;
     std::vector<int64_t> h_nitems;
-    std::vector<std::pair<void*, size_t>> blocks;  // allocations behind the tables
+    std::vector<std::pair<void*, size_t>> blocks, word_blocks;  // allocations behind the tables
     std::vector<char> have;          // direction d built or imported
     double** d_att = nullptr;        // device pointer table [D] of the attenuation factors
     std::vector<double*> h_att;
@@ -157,6 +159,9 @@ struct rts_sweep_state {
     int64_t records = 0, max_levels = 0;
 };
 void rts_sweep_free(rts_ctx* ctx);
+// Frees what the sweep can do without (copy words, attenuation factors), the
+// device being idle; whether there was anything.
+bool rts_sweep_give_way(rts_ctx* ctx);
 
 constexpr size_t RTS_FLAG_BYTES = 32;  // rts_ctx::d_flag (4 words) and d_fp64 (2)
 
@@ -167,6 +172,7 @@ struct rts_ctx {
     cudaStream_t streams[RTS_STREAM_COUNT] = {nullptr, nullptr, nullptr};
     std::string last_error;
 
+    bool spare = false;  // the allocations of the moment are optional (rts_spare)
     int64_t budget_bytes = 0;
     int64_t used_bytes = 0;
 
@@ -252,6 +258,15 @@ void rts_dfree(rts_ctx* ctx, void* p, size_t bytes);
 // Counted against the same HBM budget as rts_dmalloc.
 int rts_pmalloc(rts_ctx* ctx, void** p, size_t bytes, const char* what, cudaStream_t st);
 void rts_pfree(rts_ctx* ctx, void* p, size_t bytes, cudaStream_t st);
+// Allocations in its scope are ones the context can do without.  They fail
+// without room; every other one first takes back what earlier optional ones hold
+// (the digits of W, the sweep's copy words and attenuation factors).
+struct rts_spare {
+    rts_ctx* ctx;
+    bool before;
+    explicit rts_spare(rts_ctx* c) : ctx(c), before(c->spare) { c->spare = true; }
+    ~rts_spare() { ctx->spare = before; }
+};
 
 // Kernel launchers (defined in the .cu files).
 int rts_launch_scatter_fp64(rts_ctx* ctx, int64_t k_begin, int64_t k_end, cudaStream_t st,

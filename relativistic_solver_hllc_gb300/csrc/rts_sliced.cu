@@ -586,6 +586,7 @@ int rts_sliced_scatter(rts_ctx* ctx, int64_t c_begin, int64_t c_end, int64_t k_b
         cudaGetLastError();
         return RTS_OK;  // a captured call allocates nothing
     }
+    const rts_spare spare(ctx);
     const std::string keep = ctx->last_error;
     auto no_room = [&](int rc) {
         if (rc != RTS_ERR_OVER_BUDGET && rc != RTS_ERR_OUT_OF_MEMORY) return rc;

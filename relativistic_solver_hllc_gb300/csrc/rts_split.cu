@@ -442,6 +442,7 @@ static int ensure_staging(rts_ctx* ctx)
     s.call_sums_bytes = s.call_max_bytes = 0;
     s.eager_next = -1;
     void *ib = nullptr, *mx = nullptr;
+    const rts_spare spare(ctx);
     int rc = rts_dmalloc(ctx, &ib, ibytes, "FP64 face sums (staging)");
     if (rc == RTS_OK) rc = rts_dmalloc(ctx, &mx, mbytes, "per-cell maxima (staging)");
     if (rc != RTS_OK) {

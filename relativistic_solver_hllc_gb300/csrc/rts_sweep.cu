@@ -161,7 +161,7 @@ struct X0Args {
     const int32_t* nsteps;   // [D]
     int64_t N;
     int64_t d0;              // first direction of this launch (grid y covers at most 65535)
-    bool words;              // the items are followed by their copy words
+    uint32_t* const* words;  // [D] the items' copy words (null: none)
     int* flag;               // set when a node finds no in-face
 };
 
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(256) sweep_x0_kernel(X0Args a)
             w |= (uint32_t)found << (2 * m);
         }
         items[i] = w;
-        if (a.words) items[n + i] = copy_word(a.pairs, a.states + d * a.N, w);
+        if (a.words) a.words[d][i] = copy_word(a.pairs, a.states + d * a.N, w);
     }
 }
 
@@ -227,7 +227,7 @@ struct SweepArgs {
     const double* S;         // [D][N]
     double* illum;           // [D][N][4], rows of the local directions
     int64_t N;
-    bool words;              // copy words behind the items
+    uint32_t* const* words;  // [D] the items' copy words (null: formed here)
     rts_medium md;
     double bc[4];
     uint64_t exptab[kExpTable];  // 2^(-j/256) / 3, times 2^65
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__
     constexpr bool kAhead = kCtas < 7;   // an item's data loaded while the one before is computed
     constexpr bool kWhole = kCtas < 7;   // q stored beside the three factors
     const uint64_t keep = l2_policy_last(), stream = l2_policy_first();
-    const int n_items = ns > 0 ? steps[ns] : 0;
+    const uint32_t* __restrict__ words = kAhead && a.words ? a.words[d] : nullptr;
     // cells are below 2^24 and items below 2^26, so 32-bit indexes reach everything
     auto load = [&](uint32_t w, uint32_t cp, uint32_t i, ItemData& x) {
         const uint32_t c = w >> 8;
@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(T, kCtas) sweep_kernel(const __grid_constant__
     uint32_t w1 = 0, cp1 = 0;
     auto load_words = [&](int idx, uint32_t& w, uint32_t& cp) {
         w = ld_hint(items + idx, stream);
-        cp = !kAhead ? 0 : a.words ? ld_hint(items + n_items + idx, stream) : copy_word(a.pairs, nullptr, w);
+        cp = !kAhead ? 0 : words ? ld_hint(words + idx, stream) : copy_word(a.pairs, nullptr, w);
     };
     if (have) {
         load_words(i, w1, cp1);
@@ -848,6 +848,7 @@ int alloc_tables(rts_ctx* ctx, rts_sweep_state& sw)
     if ((rc = rts_dmalloc(ctx, &p, rts_bytes<int32_t>(D), "sweep boundary counts")) != RTS_OK) return rc;
     sw.d_nbnd = (int32_t*)p;
     sw.h_items.assign(D, nullptr);
+    sw.h_words.assign(D, nullptr);
     sw.h_recs.assign(D, nullptr);
     sw.h_att.assign(D, nullptr);
     sw.h_steps.assign(D, nullptr);
@@ -859,15 +860,32 @@ int alloc_tables(rts_ctx* ctx, rts_sweep_state& sw)
     return RTS_OK;
 }
 
-void free_blocks(rts_ctx* ctx, rts_sweep_state& sw)
+// the copy words given back, and no more made for these structures
+void drop_words(rts_ctx* ctx, rts_sweep_state& sw)
 {
-    for (auto& b : sw.blocks) rts_dfree(ctx, b.first, b.second);
-    sw.blocks.clear();
-    sw.copy_words = true;
+    for (auto& b : sw.word_blocks) rts_dfree(ctx, b.first, b.second);
+    sw.word_blocks.clear();
+    rts_dfree(ctx, sw.d_words, sizeof(uint32_t*) * sw.D);
+    sw.d_words = nullptr;
+    std::fill(sw.h_words.begin(), sw.h_words.end(), nullptr);
+    sw.copy_words = false;
+}
+
+void drop_att(rts_ctx* ctx, rts_sweep_state& sw)
+{
     rts_dfree(ctx, sw.att_blk, sw.att_bytes);
     sw.att_blk = nullptr;
     sw.att_bytes = 0;
     sw.att_valid = false;
+}
+
+void free_blocks(rts_ctx* ctx, rts_sweep_state& sw)
+{
+    for (auto& b : sw.blocks) rts_dfree(ctx, b.first, b.second);
+    sw.blocks.clear();
+    drop_words(ctx, sw);
+    sw.copy_words = true;
+    drop_att(ctx, sw);
     std::fill(sw.h_items.begin(), sw.h_items.end(), nullptr);
     std::fill(sw.h_recs.begin(), sw.h_recs.end(), nullptr);
     std::fill(sw.h_steps.begin(), sw.h_steps.end(), nullptr);
@@ -887,18 +905,34 @@ int alloc_block(rts_ctx* ctx, rts_sweep_state& sw, void** p, size_t bytes, const
     return rc;
 }
 
-// Room for n items and, if it can be had, their copy words behind them; without
-// it the sweep forms the words itself.
-int alloc_items(rts_ctx* ctx, rts_sweep_state& sw, void** p, int64_t n)
+// Room for the copy words of n items and for their table, after everything that
+// the structures need; null without it (no direction has words then).
+uint32_t* alloc_words(rts_ctx* ctx, rts_sweep_state& sw, int64_t n)
 {
     if (sw.D > 5 * ctx->num_sms) sw.copy_words = false;  // the form for so many directions does not read them
-    if (sw.copy_words) {
-        const std::string keep = ctx->last_error;
-        if (alloc_block(ctx, sw, p, rts_bytes<uint32_t>(2 * n), "sweep items") == RTS_OK) return RTS_OK;
+    if (!sw.copy_words) return nullptr;
+    const rts_spare spare(ctx);
+    const std::string keep = ctx->last_error;
+    const size_t bytes = std::max<size_t>(rts_bytes<uint32_t>(n), 16);
+    void *table = sw.d_words, *p = nullptr;
+    if (!table) rts_dmalloc(ctx, &table, sizeof(uint32_t*) * sw.D, "sweep copy word table");
+    sw.d_words = (uint32_t**)table;
+    if (table) rts_dmalloc(ctx, &p, bytes, "sweep copy words");
+    if (p) {
+        sw.word_blocks.push_back({p, bytes});
+    } else {
         ctx->last_error = keep;
-        sw.copy_words = false;
+        drop_words(ctx, sw);
     }
-    return alloc_block(ctx, sw, p, rts_bytes<uint32_t>(n), "sweep items");
+    return (uint32_t*)p;
+}
+
+int upload_words(rts_ctx* ctx, rts_sweep_state& sw, cudaStream_t st)
+{
+    if (!sw.copy_words) return RTS_OK;
+    RTS_CUDA_TRY(ctx, cudaMemcpyAsync(sw.d_words, sw.h_words.data(), sizeof(uint32_t*) * sw.D, cudaMemcpyHostToDevice, st));
+    RTS_CUDA_TRY(ctx, cudaStreamSynchronize(st));  // pageable source
+    return RTS_OK;
 }
 
 int upload_tables(rts_ctx* ctx, rts_sweep_state& sw, cudaStream_t st)
@@ -927,6 +961,15 @@ int check_flag(rts_ctx* ctx, const char* what)
 }
 
 }  // namespace
+
+bool rts_sweep_give_way(rts_ctx* ctx)
+{
+    rts_sweep_state* sw = ctx->sweep;
+    if (!sw || (!sw->att_blk && !sw->d_words)) return false;
+    drop_att(ctx, *sw);
+    drop_words(ctx, *sw);
+    return true;
+}
 
 void rts_sweep_free(rts_ctx* ctx)
 {
@@ -1044,14 +1087,14 @@ extern "C" int rts_sweep_build(rts_ctx* ctx, int64_t* records, int64_t* levels)
     }
     void *iblk = nullptr, *rblk = nullptr, *lblk = nullptr, *bblk = nullptr, *sblk = nullptr;
     int rc;
-    if ((rc = alloc_items(ctx, sw, &iblk, ni)) != RTS_OK) return rc;
+    if ((rc = alloc_block(ctx, sw, &iblk, rts_bytes<uint32_t>(ni), "sweep items")) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &rblk, rts_bytes<double>(3 * ni), "sweep node records")) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &lblk, rts_bytes<int32_t>(nl), "sweep steps")) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &bblk, rts_bytes<uint32_t>(nbd), "sweep boundary faces")) != RTS_OK) return rc;
     cudaStream_t st = ctx->streams[RTS_STREAM_SCATTERING_1];
     int64_t io = 0, lo = 0, bo = 0;
     for (int64_t d = 0; d < D; ++d) {
-        sw.h_items[d] = (uint32_t*)iblk + (sw.copy_words ? 2 : 1) * io;
+        sw.h_items[d] = (uint32_t*)iblk + io;
         sw.h_recs[d] = (double*)rblk + 3 * io;
         sw.h_steps[d] = (int32_t*)lblk + lo;
         sw.h_bnd[d] = (uint32_t*)bblk + bo;
@@ -1084,6 +1127,13 @@ extern "C" int rts_sweep_build(rts_ctx* ctx, int64_t* records, int64_t* levels)
         rts_dfree(ctx, sblk, rts_bytes<uint8_t>(std::max<int64_t>(D * N, 16)));
         return rc;
     }
+    uint32_t* words = alloc_words(ctx, sw, ni);
+    for (int64_t d = 0; words && d < D; words += sw.h_nitems[d++]) sw.h_words[d] = words;
+    if ((rc = upload_words(ctx, sw, st)) != RTS_OK) {
+        rts_dfree(ctx, sblk, rts_bytes<uint8_t>(std::max<int64_t>(D * N, 16)));
+        rts_dfree(ctx, fblk, rts_bytes<double>(kFrame * 4 * N));
+        return rc;
+    }
     if (N > 0) {
         sweep_frames_kernel<<<(unsigned)std::min<int64_t>((4 * N + 255) / 256, 8192), 256, 0, st>>>(
             sw.d_vert, sw.d_normals, N, (double*)fblk);
@@ -1101,7 +1151,7 @@ extern "C" int rts_sweep_build(rts_ctx* ctx, int64_t* records, int64_t* levels)
     a.steps = sw.d_steps;
     a.nsteps = sw.d_nsteps;
     a.N = N;
-    a.words = sw.copy_words;
+    a.words = sw.d_words;
     a.flag = ctx->d_flag + 2;
     if (D > 0) {
         const int64_t per = std::max<int64_t>(1, std::min<int64_t>((2 * N + 255) / 256, 64));
@@ -1207,18 +1257,18 @@ extern "C" int rts_sweep_import_direction(rts_ctx* ctx, int64_t d, const int32_t
     // this direction's own blocks
     int rc;
     void *iblk = nullptr, *rblk = nullptr, *lblk = nullptr, *bblk = nullptr;
-    if ((rc = alloc_items(ctx, sw, &iblk, (int64_t)items.size())) != RTS_OK) return rc;
+    if ((rc = alloc_block(ctx, sw, &iblk, rts_bytes<uint32_t>(items.size()), "sweep items")) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &rblk, rts_bytes<double>(3 * items.size()), "sweep node records")) != RTS_OK)
         return rc;
     if ((rc = alloc_block(ctx, sw, &lblk, rts_bytes<int32_t>(steps.size()), "sweep steps")) != RTS_OK) return rc;
     if ((rc = alloc_block(ctx, sw, &bblk, rts_bytes<uint32_t>(bnd.size()), "sweep boundary faces")) != RTS_OK)
         return rc;
     RTS_CUDA_TRY(ctx, cudaMemcpy(iblk, items.data(), rts_bytes<uint32_t>(items.size()), cudaMemcpyHostToDevice));
-    if (sw.copy_words) {
+    uint32_t* const wblk = alloc_words(ctx, sw, (int64_t)items.size());
+    if (wblk) {
         std::vector<uint32_t> words(items.size());
         for (size_t i = 0; i < items.size(); ++i) words[i] = copy_word(pairs, st8.data(), items[i]);
-        RTS_CUDA_TRY(ctx, cudaMemcpy((uint32_t*)iblk + items.size(), words.data(), rts_bytes<uint32_t>(words.size()),
-                                     cudaMemcpyHostToDevice));
+        RTS_CUDA_TRY(ctx, cudaMemcpy(wblk, words.data(), rts_bytes<uint32_t>(words.size()), cudaMemcpyHostToDevice));
     }
     RTS_CUDA_TRY(ctx, cudaMemcpy(rblk, recs.data(), rts_bytes<double>(3 * items.size()), cudaMemcpyHostToDevice));
     RTS_CUDA_TRY(ctx, cudaMemcpy(lblk, steps.data(), rts_bytes<int32_t>(steps.size()), cudaMemcpyHostToDevice));
@@ -1228,6 +1278,7 @@ extern "C" int rts_sweep_import_direction(rts_ctx* ctx, int64_t d, const int32_t
     if (sw.have[d]) sw.records -= 3 * sw.h_nitems[d];
     sw.records += 3 * (int64_t)items.size();
     sw.h_items[d] = (uint32_t*)iblk;
+    sw.h_words[d] = wblk;
     sw.h_recs[d] = (double*)rblk;
     sw.h_steps[d] = (int32_t*)lblk;
     sw.h_bnd[d] = (uint32_t*)bblk;
@@ -1236,6 +1287,7 @@ extern "C" int rts_sweep_import_direction(rts_ctx* ctx, int64_t d, const int32_t
     sw.h_nitems[d] = (int64_t)items.size();
     sw.have[d] = 1;
     sw.max_levels = std::max<int64_t>(sw.max_levels, nsteps);
+    if ((rc = upload_words(ctx, sw, ctx->streams[RTS_STREAM_SCATTERING_1])) != RTS_OK) return rc;
     return upload_tables(ctx, sw, ctx->streams[RTS_STREAM_SCATTERING_1]);
 }
 
@@ -1347,6 +1399,7 @@ static int att_mode(rts_ctx* ctx, rts_sweep_state& sw, cudaStream_t st, int* mod
         sw.att_bytes = 0;
         const std::string keep = ctx->last_error;
         void* p = nullptr;
+        const rts_spare spare(ctx);
         if (rts_dmalloc(ctx, &p, need, "sweep attenuation factors") != RTS_OK) {
             ctx->last_error = keep;  // not an error: this sweep evaluates the factors
             return RTS_OK;
@@ -1398,7 +1451,7 @@ static int enqueue_sweep(rts_ctx* ctx, cudaStream_t st)
     a.S = ctx->d_S;
     a.illum = ctx->d_illum + ctx->out_start * sw.N * 4;
     a.N = sw.N;
-    a.words = sw.copy_words;
+    a.words = sw.d_words;
     a.md = sw.md;
     for (int i = 0; i < 4; ++i) a.bc[i] = sw.bc[i];
     exp2_table(kExpThird, a.exptab);
