@@ -323,6 +323,7 @@ scatter_list_kernel(const double* __restrict__ illum, const double* __restrict__
             atomicAdd(stats, (unsigned long long)count[0]);
         }
     }
+    if (cells == 0) return;
     if (whole) fx.list = fx.mask = nullptr;
     // whole waves of large tiles, in quarter tiles (16 out-directions); the rest in small ones
     const int per_row = 4 * dt.n_full + (dt.gy > dt.n_full ? dt.nb_last : 0), wave = 8 * num_sms;
