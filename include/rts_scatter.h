@@ -87,7 +87,9 @@ const char* rts_last_error(const rts_ctx* ctx);
 
 /* Cap on the device bytes this context may hold (default: 90% of the
  * device memory free at creation).  Allocations beyond it fail with
- * RTS_ERR_OVER_BUDGET. */
+ * RTS_ERR_OVER_BUDGET.  Scratch that calls have given back stays with the
+ * context for the next ones, within the budget; rts_hbm_used does not count it
+ * (and the driver takes it back for any other allocation that needs it). */
 int rts_set_hbm_budget(rts_ctx* ctx, int64_t bytes);
 int rts_hbm_used(const rts_ctx* ctx, int64_t* bytes);
 

@@ -9,6 +9,7 @@
 // Differences by design: a context object instead of file-scope globals,
 // status codes instead of exit(1), 64-bit sizes, an HBM budget, deadlines on
 // every host-side wait.
+#include <algorithm>
 #include <chrono>
 #include <cstdarg>
 #include <cstdio>
@@ -44,11 +45,29 @@ static bool give_way(rts_ctx* ctx)
     return rts_sweep_give_way(ctx) || digits;
 }
 
+// Gives back what the scratch pool holds unused beyond the budget, `device`
+// bytes more being allocated outside the pool and `pooled` in it.
+static void trim_pool(rts_ctx* ctx, size_t device, size_t pooled)
+{
+    // the pool holds no more than it ever had allocated (and its rounding, 32 MB pieces)
+    const int64_t room = ctx->budget_bytes - ctx->used_bytes - (int64_t)device;
+    if (!ctx->pool || ctx->pool_peak - ctx->pool_bytes + (64 << 20) <= room) return;
+    uint64_t held = 0, live = 0;
+    if (cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &live) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if ((int64_t)(held - live) > std::max<int64_t>(room, (int64_t)pooled))
+        cudaMemPoolTrimTo(ctx->pool, live + (uint64_t)std::max<int64_t>(room, (int64_t)pooled));
+}
+
 int rts_dmalloc(rts_ctx* ctx, void** p, size_t bytes, const char* what)
 {
     *p = nullptr;
     if (bytes == 0) return RTS_OK;
     if (ctx->used_bytes + (int64_t)bytes > ctx->budget_bytes) give_way(ctx);
+    trim_pool(ctx, bytes, 0);
     if (ctx->used_bytes + (int64_t)bytes > ctx->budget_bytes)
         return rts_fail(ctx, RTS_ERR_OVER_BUDGET,
                         "%s: %zu bytes would exceed the HBM budget (%lld of %lld bytes in use)",
@@ -89,6 +108,7 @@ int rts_pmalloc(rts_ctx* ctx, void** p, size_t bytes, const char* what, cudaStre
         return rts_fail(ctx, RTS_ERR_OVER_BUDGET,
                         "%s: %zu bytes would exceed the HBM budget (%lld of %lld bytes in use)",
                         what, bytes, (long long)ctx->used_bytes, (long long)ctx->budget_bytes);
+    trim_pool(ctx, 0, bytes);
     if (!ctx->pool) {
         cudaMemPoolProps props;
         memset(&props, 0, sizeof(props));
@@ -111,6 +131,8 @@ int rts_pmalloc(rts_ctx* ctx, void** p, size_t bytes, const char* what, cudaStre
                         cudaGetErrorString(e));
     }
     ctx->used_bytes += (int64_t)bytes;
+    ctx->pool_bytes += (int64_t)bytes;
+    ctx->pool_peak = std::max(ctx->pool_peak, ctx->pool_bytes);
     return RTS_OK;
 }
 
@@ -119,6 +141,7 @@ void rts_pfree(rts_ctx* ctx, void* p, size_t bytes, cudaStream_t st)
     if (!p) return;
     cudaFreeAsync(p, st);
     ctx->used_bytes -= (int64_t)bytes;
+    ctx->pool_bytes -= (int64_t)bytes;
 }
 
 static void free_grid(rts_ctx* ctx)
@@ -310,6 +333,7 @@ int rts_set_hbm_budget(rts_ctx* ctx, int64_t bytes)
                 "budget %lld below the %lld bytes already held", (long long)bytes,
                 (long long)ctx->used_bytes);
     ctx->budget_bytes = bytes;
+    trim_pool(ctx, 0, 0);
     return RTS_OK;
 }
 

@@ -172,6 +172,7 @@ struct rts_ctx {
     cudaStream_t streams[RTS_STREAM_COUNT] = {nullptr, nullptr, nullptr};
     std::string last_error;
 
+    int64_t pool_bytes = 0, pool_peak = 0;  // scratch pool: allocated, and the most that ever was
     bool spare = false;  // the allocations of the moment are optional (rts_spare)
     int64_t budget_bytes = 0;
     int64_t used_bytes = 0;

@@ -89,3 +89,21 @@ def test_digits_of_w_give_way(ctx):
     ctx.set_hbm_budget(before + geometry)
     with pytest.raises(RtsError):
         ctx.set_hbm_budget(before)
+
+
+def test_unused_scratch_is_held_within_the_budget(ctx):
+    torch = pytest.importorskip("torch")
+    M, N = 200, 100000
+    xyz, area, fa = oracle.fibonacci_directions(M)
+    il = oracle.illum(5, 0.0, 1.0, N, M, independent_faces=True)
+    ctx.init(xyz, area, fa, N)
+    S = ctx.scattering(il)  # 270 MB of digit rows
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    ctx.set_hbm_budget(ctx.hbm_used() + (40 << 20))
+    assert torch.cuda.mem_get_info()[0] - before >= 200 << 20
+    assert np.array_equal(ctx.scattering(il), S)  # in passes
+    before = torch.cuda.mem_get_info()[0]
+    rng = np.random.default_rng(1)
+    ctx.set_geometry(rng.uniform(-1, 1, (N, 4, 3)), rng.uniform(0.5, 1.0, (N, 4)), rng.uniform(0.5, 1.0, N))  # 14 MB
+    assert before - torch.cuda.mem_get_info()[0] <= 8 << 20  # out of what the pool held unused
