@@ -20,18 +20,20 @@
 // output (D_5 rounded to the total's unit), which the column exponents keep
 // below 2^64: sum_j W_jk <= 1022 2^e_k.
 //
-// Error.  The digits carry 54 bits below the row's and the column's largest
-// value and the products d >= 6 are left out: about sqrt(M) 2^-56 of
-// 2^(e_c + e_k) in all (rms), against about sqrt(M) 2^-55 of S for the FP64 FMA
-// chain of scatter_fp64_kernel (measured against 113-bit sums, lognormal
-// intensities: 1.0e-16 against 8.6e-16 rms at M = 1000, 7.5e-17 against
-// 3.8e-16 at M = 200, 7.6e-17 against 2.1e-16 at M = 64).  An output below half
-// of 2^(e_c + e_k) (a row dominated by a few directions far above the rest)
-// could be further off than the chain: it is left to that kernel, as are rows
-// with negative values, infinities, NaN or exponents out of range -- the
-// outputs are marked here and rts_launch_scatter_list computes them from the
-// Illum.  So every output is at least as accurate as the chain's, for any
-// input.
+// Error.  In units of 2^-54 of 2^(e_c + e_k): at most 1.26 a direction from the
+// products d >= 6 that are left out (five of 2^-2 at d = 6), half of Ibar / 2^e_c +
+// W / 2^e_k a direction from the operands' last digits, 0.75 per 32 directions from
+// D_5, and the rounding of S.  In ordinary rows the signs mix: measured against
+// 113-bit sums with lognormal intensities, rms 1.0e-16 against 8.6e-16 for the
+// FP64 FMA chain of scatter_fp64_kernel at M = 1000, 7.5e-17 against 3.8e-16 at
+// M = 200, 7.6e-17 against 2.1e-16 at M = 64.  That is on average: single outputs,
+// 7 to 15 % of those, are further off than the chain's, and rows of a few directions
+// (where the chain rounds a few times only) can be too, by the bound above.
+// An output below half of 2^(e_c + e_k) (a row dominated by a few directions far
+// above the rest), where that bound is large against the output, is left to the
+// chain, as are rows with negative values, infinities, NaN or exponents out of
+// range -- the outputs are marked here and rts_launch_scatter_list computes them
+// from the Illum.
 //
 // Kernel: persistent CTAs (one per SM) on tiles of 128 cells x up to 128
 // out-directions.  Warp 0 brings the digits of 32 in-directions of both

@@ -1,5 +1,7 @@
 """What the FP64 integrals' digit products report of themselves: that they ran,
 which rows they left to the FP64 cores, and contractions that gave up."""
+from fractions import Fraction
+
 import numpy as np
 import pytest
 
@@ -190,3 +192,48 @@ def test_kernel_timing_covers_the_listed_rows(ctx):
         ms[mode], launches = ctx.kernel_timing(False)
         assert launches == 3
     assert ms[1] > 0.9 * ms[0]
+
+
+@pytest.mark.parametrize("g", [None, 0.0, 0.4])
+def test_error_bound_of_the_digits(ctx, g):
+    """Rows of one direction, of equal values and of lognormal ones against exact
+    sums of the device's own W, output by output: in units of 2^-54 of the row's and
+    the column's powers of two, 1.26 a direction (the products left out), half of
+    both scaled operands a direction (their last digits), 0.75 per 32 directions
+    (D_5), and half a unit in the last place of S."""
+    M, N = 161, 200
+    xyz, area, fa = oracle.fibonacci_directions(M)
+    ctx.init(xyz, area, fa, N)
+    if g is not None:
+        ctx.set_phase(PHASE_HG, g)
+    il = np.zeros((M, N, 4))
+    il[np.arange(M), np.arange(M), 0] = 4.0  # Ibar is the unit matrix: the chain gives W itself
+    ctx.set_tuning(_native.TUNE_FP64_DIGITS, 0)
+    W = ctx.scattering(il.ravel())[:, :M].T.copy()
+    ctx.set_tuning(_native.TUNE_FP64_DIGITS, 1)
+    rng = np.random.default_rng(2)
+    ibar = rng.lognormal(0.0, 1.0, (M, N))
+    ibar[:, :8] = 0.0
+    ibar[rng.integers(0, M, 8), np.arange(8)] = rng.uniform(0.5, 1.0, 8)
+    ibar[:, 8:12] = rng.uniform(0.5, 1.0, 4)
+    il[:] = 0.0
+    il[..., 2] = 4.0 * ibar
+    S = ctx.scattering(il.ravel())
+    assert ctx.fp64_stats()[0] == 1
+    e_col = np.frexp(W.max(axis=0))[1]
+    taken = 0
+    for c in range(16):
+        e_row = int(np.frexp(ibar[:, c].max())[1])
+        used = np.flatnonzero(ibar[:, c])
+        a = {j: Fraction(float(ibar[j, c])) for j in used}
+        for k in range(M):
+            exact = sum((a[j] * Fraction(float(W[j, k])) for j in used), Fraction(0))
+            scale = Fraction(2) ** (e_row + int(e_col[k]))
+            if exact < scale / 2:
+                continue  # the chain's
+            taken += 1
+            last = float((ibar[:, c] / 2.0 ** e_row + W[:, k] / 2.0 ** int(e_col[k])).sum()) / 2
+            bound = Fraction(1.26 * M + last + 0.75 * -(-M // 32)) * scale / 2 ** 54
+            bound += Fraction(float(np.spacing(S[k, c]))) / 2
+            assert abs(Fraction(float(S[k, c])) - exact) <= bound, (c, k)
+    assert taken > 8 * M
