@@ -337,8 +337,8 @@ typedef struct rts_problem_desc {
     double g;       /* Henyey-Greenstein asymmetry, (-1, 1) */
     int precision;  /* RTS_PREC_FP16X3 or RTS_PREC_BF16X3 */
     int flush;      /* K-slices per FP32 drain (1 or 2; 0: automatic, see RTS_TUNE_FLUSH) */
-    int bn;         /* out-directions per tile, multiple of 16, <= 256 (0: balanced default;
-                       the kernel's tiles hold at most 160) */
+    int bn;         /* out-directions per tile, multiple of 16, <= 256 (0, or more than the 160 that
+                       the kernel's tiles hold: balanced default) */
 } rts_problem_desc;
 
 /* Device bytes a problem holds while resident (for admission control). */

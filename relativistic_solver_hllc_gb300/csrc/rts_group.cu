@@ -179,16 +179,18 @@ int64_t rts_group_energy_bytes(int64_t kpad, int64_t rows_pad, int n_tiles)
     return (kpad + 4) * 4 + (int64_t)n_tiles * G_SLICES * rows_pad * 8 + rows_pad * 16;
 }
 
-// Tile geometry of a problem: out-direction tiles of at most G_BN, balanced.
+// Tile geometry of a problem: out-direction tiles of at most G_BN, balanced.  A
+// width past that (a caller's, or a schedule table's of a build with wider tiles)
+// counts as none: cut to G_BN it could leave a last tile nearly empty.
 void rts_group_geometry(int64_t Min, int64_t Mout, int64_t rows, int bn_override, int* bn, int* n_tiles,
                         int64_t* kpad, int64_t* mpad, int64_t* rows_pad, int64_t* m_tiles)
 {
     int b = bn_override;
-    if (b <= 0) {
+    if (b <= 0 || b > G_BN) {
         const int64_t nt = (Mout + G_BN - 1) / G_BN;
         b = (int)round_up((Mout + nt - 1) / nt, 16);
     }
-    b = std::min(std::max(b, 16), G_BN);
+    b = std::max(b, 16);
     *bn = b;
     *n_tiles = (int)((Mout + b - 1) / b);
     *mpad = (int64_t)(*n_tiles) * b;
