@@ -313,6 +313,10 @@ group_kernel(const GroupProblem* __restrict__ probs, int nprob, int64_t total_ti
                 // no copy may still be in flight when the CTA exits
                 for (uint32_t i = (it > (uint32_t)G_STAGES ? it - G_STAGES : 0); i < it; ++i)
                     mbar_wait(full_bar(i % G_STAGES), (i / G_STAGES) & 1, flag, FLAG_WAIT_PRODUCER);
+                // nor a commit: the issuers' last arrivals on the ring (those on the accumulators' barriers,
+                // committed after them, are waited for by the drain warps, which orders the MMAs, not the arrivals)
+                for (uint32_t i = (it > (uint32_t)G_STAGES ? it - G_STAGES : 0); ok && i < it; ++i)
+                    mbar_wait(empty_bar(i % G_STAGES), (i / G_STAGES) & 1, flag, FLAG_WAIT_PRODUCER);
             }
         } else if (warp < 3) {
             // -------------------------------------------------------- MMA issuers
