@@ -147,8 +147,10 @@ int rts_copy_illum(rts_ctx* ctx, int64_t size, const double* illum_host);
  * sm_10x.  At a tensor precision the calls also hold the split Ibar rows
  * (4 bytes per cell and in-direction, 8 for RTS_PREC_TF32X3) and, where the
  * HBM budget and the device leave room, a staging of the FP64 face sums
- * (8 bytes per cell and direction) that speeds up their preparation; without
- * that room the rows are prepared directly, with the same results.
+ * (8 bytes per cell and direction), which lets directions sent in order be
+ * summed as they arrive, and speeds up the preparation of more than 14,432
+ * directions; without that room the rows are prepared directly, with the same
+ * results.
  * RTS_PREC_FP64 computes with FP64's accuracy on either the FP64 CUDA cores
  * or, for Thomson and smooth Henyey-Greenstein kernels on sm_10x, the tensor
  * cores (exact products of FP16 digits, integer sums), which hold 12 bytes per

@@ -42,11 +42,13 @@
 // accumulators in turn; warps 4..19 read each finished accumulator and add it
 // into their 64-bit totals, up to 32 a thread.
 //
-// Bound: shared memory feeds an M = 128, N = 128 MMA at about 113 cycles (64 of
-// tensor work), and the drain of a chunk -- a conversion and a 64-bit
-// multiply-add per accumulator value -- takes about as long as its MMAs; 35
-// TFLOP/s of FP64 products at 162,000 x 1000 (9.1 ms; scatter_fp64_kernel 291
-// ms), 20 at 30,011 x 302 (0.27; 5.27 ms), 10 at 10,368 x 200 (0.083; 0.94 ms).
+// Bound: the drain, a conversion and a 64-bit multiply-add per accumulator value.
+// A chunk of 32 in-directions takes 7.9k cycles at 162,000 x 1000; in copies of
+// the kernel whose drain only releases the accumulators 4.3k (42 MMAs at 103
+// cycles, fed from shared memory; 64 with resident operands), without the MMAs
+// 6.8k.  With update and residual 162,000 x 1000 takes 9.1 ms, 35 TFLOP/s of FP64
+// products (scatter_fp64_kernel 291 ms; 8.2 without them), 30,011 x 302 0.27 (5.27
+// ms), 10,368 x 200 0.083 (0.94 ms).
 #include <cuda.h>
 
 #include <algorithm>
@@ -77,7 +79,8 @@ constexpr size_t S_SMEM = (size_t)S_STAGES * S_STAGE_BYTES + 1024 + 256;
 static_assert(S_SMEM <= 227 * 1024, "shared memory per CTA");
 // Registers: 96 a thread at launch; the issuing warpgroup gives up 64 of them,
 // so that the drain warps hold their 32 totals (64 registers) and the values
-// in flight without spilling (at 96 the spills tripled the kernel's time).
+// in flight (26 bytes spilled outside their loop; at 96 the spills tripled the
+// kernel's time).
 constexpr int S_REGS = 96, S_REGS_ISSUE = 32, S_REGS_DRAIN = 112;
 static_assert(S_DRAIN_WARP0 * S_REGS_ISSUE + S_DRAIN_WARPS * S_REGS_DRAIN <=
                   (S_DRAIN_WARP0 + S_DRAIN_WARPS) * S_REGS,
@@ -313,7 +316,6 @@ sliced_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
                         break;
                     }
                     tc_fence_after();
-                    // 4 columns at a time, the next 4 on their way while these are added
                     const uint32_t ta = tmem + s0 * S_BN + lane_off, tb = tmem + s1 * S_BN + lane_off;
                     // 8 columns at a time (4 at the end), the next on their way while these are added
                     uint32_t cur[16], nxt[16];
