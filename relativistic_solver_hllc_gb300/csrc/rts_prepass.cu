@@ -544,7 +544,7 @@ int rts_pp_rows_from_faces(rts_ctx* ctx, const double* illum, int64_t N, int64_t
         ctx->launches++;
         return RTS_OK;
     }
-    // rows too long for shared memory (M > 14,000): a pass for the scales, a pass for the rows
+    // rows too long for shared memory (M > 14,432): a pass for the scales, a pass for the rows
     if (fp16 || bound) {
         rowscale_faces_kernel<<<(unsigned)((npad + 127) / 128), 128, 0, st>>>(illum, N, ld, M, B, rs, npad);
         RTS_CHECK_LAUNCH(ctx, "rowscale_faces_kernel");
