@@ -187,7 +187,7 @@ void InitDevice(const grid_directions_t& grid_dir_host, grid_t& grid_host, const
     rts_host_illum(g_ctx, &grid_host.Illum);
     rts_host_scattering(g_ctx, &grid_host.scattering);
     const int precision = env_precision();
-    if (env_fp64_chain()) report(rts_set_tuning(g_ctx, RTS_TUNE_FP64_DIGITS, 0), "InitDevice (FP64 arithmetic)");
+    report(rts_set_tuning(g_ctx, RTS_TUNE_FP64_DIGITS, env_fp64_chain() ? 0 : 1), "InitDevice (FP64 arithmetic)");
     if (report(rts_set_precision(g_ctx, precision), "InitDevice (precision)") == 0)
         tune_schedule(precision, M, grid_host.size);
     if (start == 0) {  // the first rank also receives the moments (cuda/cuda_struct.cu:158-175)
